@@ -28,7 +28,7 @@ NVCC_FLAGS = [
 LIBRARIES = {
     "libcuhe_b200.so": {
         "sources": ["cuhe_paillier.cu"],
-        "depends": ["bigint_group.cuh", "paillier_kernels.cuh", "host_bigint.h"],
+        "depends": ["bigint52.cuh", "bigint_group.cuh", "host_bigint.h", "pair52.cuh", "paillier_kernels.cuh"],
         "headers": ["cuhe_paillier.h"],
     },
     "libcuhe_bfv_b200.so": {

@@ -79,6 +79,7 @@ bool is_device_pointer(const void* p) {
 
 struct cuhe_paillier {
   int device = 0;
+  int sms = 1;  // multiprocessors of the device
   int K = 0;
   int n_words = 0;
   int tpi = 0, window = 0;
@@ -97,15 +98,25 @@ struct cuhe_paillier {
   int32_t* d_ops_sec52 = nullptr;  // the secret exponent's schedule for the FP64-pipe kernel's window
   int nops_sec52 = 0;
   uint32_t* d_crt = nullptr;  // CRT constant block, present once the factors are installed
-  double* d_crt52 = nullptr;  // per side: M and R52 mod M as 52-bit limbs (FP64-pipe CRT kernel)
+  double* d_crt52 = nullptr;  // per side: the constants mod p, q of k_pair_crt (pair_const_doubles)
+  double* d_pair = nullptr;   // the constants mod n of k_pair_modexp
+  unsigned long long pair_ninv = 0;  // -n^-1 mod 2^52
   double* d_n52 = nullptr;    // n^2 and R52 mod n^2 as 52-bit limbs, then R52 R and R52 mod n^2 in words
   unsigned long long ninv52 = 0;  // -(n^2)^-1 mod 2^52
-  int32_t* d_ops_n52 = nullptr;   // the schedule of n for k_modexp52's window
+  int32_t* d_ops_n52 = nullptr;   // the schedule of n for k_pair_modexp's window
   int nops_n52 = 0;
+  // each side's exponent in k_pair_crt: the secret's, or p - 1 and its cofactor
+  struct SideExponent {
+    int32_t* d_ops = nullptr;
+    int32_t* d_fall = nullptr;
+    int nops = 0, nfall = 0, scaled = 0;
+    cuhe::PairExponent get() const { return {d_ops, d_fall, nops, nfall, scaled}; }
+  } side_exp[2];
+  Limbs factor[2];  // p, q once installed
   cuhe::CrtScalars cs{};
   bool have_factors = false;
-  bool fp64 = true;           // decrypt / decode exponentiations on the FP64 pipe (n^2 of 4096 bits or more)
-  bool fp64_small = false;    // ... and for n^2 of 2048 bits (set_fp64(ctx, 2))
+  bool fp64 = true;           // exponentiations, server products and table encryption on the FP64 pipe
+  bool fp64_small = false;    // the latter two also for n^2 of 2048 bits (set_fp64(ctx, 2))
   uint32_t* d_gtab = nullptr;
   int message_chunks = 0;
   uint32_t* d_wide = nullptr;  // 16-bit-digit table W[j][D], built on demand (see cuhe_lookup_set_wide_table)
@@ -184,66 +195,77 @@ cudaError_t launch_modexp_crt(cuhe_paillier* ctx, const uint32_t* base, uint32_t
   return cudaGetLastError();
 }
 
-// The same with both exponentiations on the FP64 pipe (KH / 16 lanes per
-// side, ten 52-bit limbs per lane; a 3-bit window, with the secret
-// exponent's own schedule).  Independent of the integer kernels' (threads
-// per instance, window) tuning.
-constexpr int kCrt52Window = 3;
-template <int KH, int W>
-size_t modexp_crt52_smem() {
-  constexpr int TPI = KH / 16, K52 = 5 * KH / 8;
-  constexpr int IPB = cuhe::kBlockThreads / (2 * TPI);
-  return size_t(7 * 2 * KH) * 4 + size_t(K52 + IPB * 2 * (((1 << (W - 1)) + 1) * K52 + 2)) * 8;
+// Batches of at most one CTA of the five-limb kernels to an SM (items5 items a
+// CTA; one warp to a scheduler) run with five limbs per lane: at key_len 1024
+// 2,368 decodes take 1.27 ms against 2.19 with ten, as many decryptions 4.2
+// against 7.3, encryptions 13.3 against 22.7.  With two CTAs to an SM the ten-
+// limb kernel, whose one warp per scheduler then holds the same items, is as
+// fast or faster (decodes 2.15 and 2.19 ms, encryptions 25.5 and 22.7).
+bool pair_small(const cuhe_paillier* ctx, long long count, int items5) {
+  return count <= (long long)ctx->sms * items5;
 }
 
-template <int KH, int W>
-cudaError_t launch_modexp_crt52(cuhe_paillier* ctx, const uint32_t* base, uint32_t* out, long long count,
-                                int mode, int pop_words) {
-  constexpr int IPB = cuhe::kBlockThreads / (2 * (KH / 16));
-  const size_t smem = modexp_crt52_smem<KH, W>();
-  cudaError_t e = cudaFuncSetAttribute(cuhe::k_modexp_crt52<KH, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(smem));
+// The same on pairs of residues mod p and mod q (k_pair_crt).
+template <int KH, int kL>
+cudaError_t launch_pair_crt_l(cuhe_paillier* ctx, const uint32_t* base, uint32_t* out, long long count, int mode,
+                              int pop_words) {
+  using Lay = cuhe::PairLayout<5 * KH / 16, kL, 4, 2>;
+  cudaError_t e = cudaFuncSetAttribute(cuhe::k_pair_crt<KH, kL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(Lay::kBytes));
   if (e != cudaSuccess) return e;
-  const long long blocks = (count + IPB - 1) / IPB;
-  cuhe::k_modexp_crt52<KH, W><<<dim3(unsigned(blocks)), cuhe::kBlockThreads, smem, ctx->stream>>>(
-      base, out, count, ctx->d_consts, ctx->ks, ctx->d_crt, ctx->cs, ctx->d_crt52, ctx->d_ops_sec52,
-      ctx->nops_sec52, mode, pop_words, ctx->d_status);
+  const long long blocks = (count + Lay::kItems - 1) / Lay::kItems;
+  cuhe::k_pair_crt<KH, kL><<<dim3(unsigned(blocks)), cuhe52::kPairThreads, Lay::kBytes, ctx->stream>>>(
+      base, out, count, ctx->d_consts, ctx->ks, ctx->d_crt, ctx->cs, ctx->d_crt52, ctx->side_exp[0].get(),
+      ctx->side_exp[1].get(), mode, pop_words, ctx->d_status);
   return cudaGetLastError();
 }
 
-// The exponentiation mod n^2 on the FP64 pipe (no factors needed).
-template <int K, int W>
-size_t modexp52_smem() {
-  constexpr int TPI = K / 16, K52 = 5 * K / 8;
-  constexpr int IPB = cuhe::kBlockThreads / TPI;
-  return size_t(6 * K) * 4 + size_t(K52 + IPB * (((1 << (W - 1)) + 1) * K52 + 2)) * 8;
+template <int KH>
+cudaError_t launch_pair_crt(cuhe_paillier* ctx, const uint32_t* base, uint32_t* out, long long count, int mode,
+                            int pop_words) {
+  if (pair_small(ctx, count, cuhe::PairLayout<5 * KH / 16, 5, 4, 2>::kItems))
+    return launch_pair_crt_l<KH, 5>(ctx, base, out, count, mode, pop_words);
+  return launch_pair_crt_l<KH, 10>(ctx, base, out, count, mode, pop_words);
 }
 
-template <int K, int W>
-cudaError_t launch_modexp52(cuhe_paillier* ctx, const uint32_t* base, const uint32_t* aux, uint32_t* out,
-                            long long count, const int32_t* ops, int nops, int mode, int pop_words) {
-  constexpr int IPB = cuhe::kBlockThreads / (K / 16);
-  const size_t smem = modexp52_smem<K, W>();
-  cudaError_t e = cudaFuncSetAttribute(cuhe::k_modexp52<K, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(smem));
+// The exponentiation mod n^2 on pairs of residues mod n (no factors needed).
+template <int K, int kL>
+cudaError_t launch_pair_modexp_l(cuhe_paillier* ctx, const uint32_t* base, const uint32_t* aux, uint32_t* out,
+                                 long long count, const int32_t* ops, int nops, int mode, int pop_words) {
+  using Lay = cuhe::PairLayout<5 * K / 16, kL, 2, 1>;
+  cudaError_t e = cudaFuncSetAttribute(cuhe::k_pair_modexp<K, kL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(Lay::kBytes));
   if (e != cudaSuccess) return e;
-  const long long blocks = (count + IPB - 1) / IPB;
-  cuhe::k_modexp52<K, W><<<dim3(unsigned(blocks)), cuhe::kBlockThreads, smem, ctx->stream>>>(
-      base, aux, K, out, count, ctx->d_consts, ctx->ks, ctx->d_n52, ctx->ninv52, ops, nops, mode, pop_words,
+  const long long blocks = (count + Lay::kItems - 1) / Lay::kItems;
+  cuhe::k_pair_modexp<K, kL><<<dim3(unsigned(blocks)), cuhe52::kPairThreads, Lay::kBytes, ctx->stream>>>(
+      base, aux, out, count, ctx->d_consts, ctx->ks, ctx->d_pair, ctx->pair_ninv, ops, nops, mode, pop_words,
       ctx->d_status);
   return cudaGetLastError();
 }
 
-// k_modexp52 for this context's width when the FP64 pipe is selected for it
-// (n^2 of 4096 or 8192 bits; 2048 bits only with set_fp64(ctx, 2)), else null.
-using Modexp52 = cudaError_t (*)(cuhe_paillier*, const uint32_t*, const uint32_t*, uint32_t*, long long,
-                                 const int32_t*, int, int, int);
-Modexp52 direct52(const cuhe_paillier* ctx) {
-  if (!ctx->fp64 || !ctx->d_n52) return nullptr;
-  if (ctx->K == 64 && ctx->fp64_small) return &launch_modexp52<64, kCrt52Window>;
-  if (ctx->K == 128) return &launch_modexp52<128, kCrt52Window>;
-  if (ctx->K == 256) return &launch_modexp52<256, kCrt52Window>;
+template <int K>
+cudaError_t launch_pair_modexp(cuhe_paillier* ctx, const uint32_t* base, const uint32_t* aux, uint32_t* out,
+                               long long count, const int32_t* ops, int nops, int mode, int pop_words) {
+  if (pair_small(ctx, count, cuhe::PairLayout<5 * K / 16, 5, 2, 1>::kItems))
+    return launch_pair_modexp_l<K, 5>(ctx, base, aux, out, count, ops, nops, mode, pop_words);
+  return launch_pair_modexp_l<K, 10>(ctx, base, aux, out, count, ops, nops, mode, pop_words);
+}
+
+// k_pair_modexp for this context's width when the FP64 pipe is selected, else null.
+using PairModexp = cudaError_t (*)(cuhe_paillier*, const uint32_t*, const uint32_t*, uint32_t*, long long,
+                                   const int32_t*, int, int, int);
+PairModexp pair_modexp(const cuhe_paillier* ctx) {
+  if (!ctx->fp64 || !ctx->d_pair) return nullptr;
+  if (ctx->K == 64) return &launch_pair_modexp<64>;
+  if (ctx->K == 128) return &launch_pair_modexp<128>;
+  if (ctx->K == 256) return &launch_pair_modexp<256>;
   return nullptr;
+}
+
+// Whether the server's products and the lookup encryption take 52-bit limbs
+// mod n^2 (n^2 of 4096 or 8192 bits; 2048 bits only with set_fp64(ctx, 2)).
+bool limbs52(const cuhe_paillier* ctx) {
+  return ctx->fp64 && ctx->d_n52 && (ctx->K >= 128 || ctx->fp64_small);
 }
 
 // encode_hamming_server on the FP64 pipe: queries to R52 Montgomery limbs,
@@ -273,7 +295,7 @@ cudaError_t launch_outer52(cuhe_paillier* ctx, const uint32_t* query, long long 
 using Outer52 = cudaError_t (*)(cuhe_paillier*, const uint32_t*, long long, double*, const uint32_t*, long long,
                                 uint32_t*);
 Outer52 outer52(const cuhe_paillier* ctx) {
-  if (!direct52(ctx)) return nullptr;
+  if (!limbs52(ctx)) return nullptr;
   if (ctx->K == 64) return &launch_outer52<64>;
   if (ctx->K == 128) return &launch_outer52<128>;
   if (ctx->K == 256) return &launch_outer52<256>;
@@ -323,7 +345,7 @@ struct Lookup52 {
                         uint32_t*);
 };
 bool lookup52(const cuhe_paillier* ctx, Lookup52* l) {
-  if (!direct52(ctx)) return false;
+  if (!limbs52(ctx)) return false;
   if (ctx->K == 64) *l = {&build_wide52<64>, &launch_lookup52<64>};
   else if (ctx->K == 128) *l = {&build_wide52<128>, &launch_lookup52<128>};
   else if (ctx->K == 256) *l = {&build_wide52<256>, &launch_lookup52<256>};
@@ -332,14 +354,13 @@ bool lookup52(const cuhe_paillier* ctx, Lookup52* l) {
 }
 
 template <int K>
-cudaError_t prepare_tasks52(int device, int* grid) {
-  const size_t smem = modexp52_smem<K, kCrt52Window>();
-  cudaError_t e = cudaFuncSetAttribute(cuhe::k_modexp52_tasks<K, kCrt52Window>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+cudaError_t prepare_pair_tasks(int device, int* grid) {
+  constexpr size_t smem = cuhe::PairLayout<5 * K / 16, 10, 2, 1>::kBytes;
+  cudaError_t e = cudaFuncSetAttribute(cuhe::k_pair_modexp_tasks<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(smem));
   if (e != cudaSuccess) return e;
   int per_sm = 0, sms = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cuhe::k_modexp52_tasks<K, kCrt52Window>,
-                                                    cuhe::kBlockThreads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cuhe::k_pair_modexp_tasks<K>, cuhe52::kPairThreads, smem);
   if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return e;
@@ -348,9 +369,9 @@ cudaError_t prepare_tasks52(int device, int* grid) {
 }
 
 template <int K>
-cudaError_t launch_tasks52(const cuhe::ModexpTask* tasks, int ntasks, long long units, unsigned long long* counter,
-                           int* status, int grid, cudaStream_t stream) {
-  cuhe::k_modexp52_tasks<K, kCrt52Window><<<grid, cuhe::kBlockThreads, modexp52_smem<K, kCrt52Window>(), stream>>>(
+cudaError_t launch_pair_tasks(const cuhe::ModexpTask* tasks, int ntasks, long long units, unsigned long long* counter,
+                              int* status, int grid, cudaStream_t stream) {
+  cuhe::k_pair_modexp_tasks<K><<<grid, cuhe52::kPairThreads, cuhe::PairLayout<5 * K / 16, 10, 2, 1>::kBytes, stream>>>(
       tasks, ntasks, units, counter, status);
   return cudaGetLastError();
 }
@@ -517,14 +538,13 @@ bool find_dispatch(int K, int TPI, int W, Dispatch* d) {
 cudaError_t secret_modexp(cuhe_paillier* ctx, const Dispatch& d, const uint32_t* base, uint32_t* out,
                           long long count, int mode, int pop_words) {
   if (ctx->have_factors && ctx->fp64) {
-    // n^2 of 2048 bits (1024-bit sides) stays on the integer pipe: measured faster there
-    if (ctx->K == 64 && ctx->fp64_small) return launch_modexp_crt52<32, kCrt52Window>(ctx, base, out, count, mode, pop_words);
-    if (ctx->K == 128) return launch_modexp_crt52<64, kCrt52Window>(ctx, base, out, count, mode, pop_words);
-    if (ctx->K == 256) return launch_modexp_crt52<128, kCrt52Window>(ctx, base, out, count, mode, pop_words);
+    if (ctx->K == 64) return launch_pair_crt<32>(ctx, base, out, count, mode, pop_words);
+    if (ctx->K == 128) return launch_pair_crt<64>(ctx, base, out, count, mode, pop_words);
+    if (ctx->K == 256) return launch_pair_crt<128>(ctx, base, out, count, mode, pop_words);
   }
   if (ctx->have_factors) return d.modexp_crt(ctx, base, out, count, mode, pop_words);
-  if (Modexp52 f = direct52(ctx)) return f(ctx, base, nullptr, out, count, ctx->d_ops_sec52, ctx->nops_sec52, mode,
-                                           pop_words);
+  if (PairModexp f = pair_modexp(ctx)) return f(ctx, base, nullptr, out, count, ctx->d_ops_sec52, ctx->nops_sec52,
+                                                mode, pop_words);
   return d.modexp(ctx, base, nullptr, out, count, ctx->d_ops_sec, ctx->nops_sec, mode, pop_words);
 }
 
@@ -680,7 +700,7 @@ int upload_schedule(cuhe_paillier* ctx, const Limbs& e, int32_t** dptr, int* nop
   return CUHE_OK;
 }
 
-// k_modexp52's constants: n^2 and R52 mod n^2 as K52 = 5K/8 limbs of 52 bits
+// The 52-bit constants mod n^2: n^2 and R52 mod n^2 as K52 = 5K/8 limbs of 52 bits
 // (doubles), then R52 R mod n^2 as K words; R52 = 2^(52 K52), R = 2^(32K).
 int setup_direct52(cuhe_paillier* ctx) {
   const size_t k = size_t(ctx->K), k52 = 5 * k / 8;
@@ -710,6 +730,101 @@ int setup_direct52(cuhe_paillier* ctx) {
   CUHE_CUDA(ctx, cudaMalloc(&ctx->d_n52, block.size() * 8), "constants allocation");
   CUHE_CUDA(ctx, cudaMemcpy(ctx->d_n52, block.data(), block.size() * 8, cudaMemcpyHostToDevice), "constants upload");
   return CUHE_OK;
+}
+
+// v as k limbs of 52 bits, balanced (each but the top one in [-2^51, 2^51))
+void balanced52(const Limbs& v, size_t k, double* out, size_t stride) {
+  int64_t carry = 0;
+  for (size_t i = 0; i < k; ++i) {
+    int64_t limb = carry;
+    for (int b = 0; b < 52; ++b) {
+      const size_t bit = 52 * i + size_t(b);
+      if (bit / 32 < v.size() && ((v[bit / 32] >> (bit % 32)) & 1u)) limb += int64_t(1) << b;
+    }
+    carry = i + 1 < k && limb >= (int64_t(1) << 51) ? 1 : 0;
+    if (carry) limb -= int64_t(1) << 52;
+    out[i * stride] = double(limb);
+  }
+}
+
+// The constants of one modulus m (pair_const_doubles) for pair_power: k limbs
+// per component, `entry` chunks of a value; scale: null, or the cofactor u of
+// an exponent u (m - 1).  m in its natural limb count w; m^2 in 2w limbs.
+std::vector<double> pair_constants(const Limbs& m_in, size_t k, int entry, const Limbs* scale) {
+  Limbs m = m_in;
+  while (m.size() > 1 && m.back() == 0) m.pop_back();
+  const size_t w = m.size(), bits = 52 * k;
+  const Limbs mm = cuhe::host::mul(m, m, 2 * w);
+  std::vector<double> block(size_t(cuhe::pair_const_doubles(int(k), entry)), 0.0);
+  balanced52(m, k, block.data(), 1);
+  double* rows = block.data() + k;
+  auto put = [&](int row, const Limbs& v) {  // the pair (v mod m, floor(v / m))
+    Limbs quotient;
+    const Limbs rem = cuhe::host::mod_reduce(v, m, &quotient);
+    balanced52(rem, k, rows + size_t(row) * 2 * k, 2);
+    balanced52(quotient, k, rows + size_t(row) * 2 * k + 1, 2);
+  };
+  Limbs x(2 * w, 0u);
+  x[0] = 1u;  // m >= 3
+  rows[size_t(entry) * 2 * k] = 1.0;
+  x = cuhe::host::shift_mod(x, bits, mm);
+  put(entry + 2, x);
+  for (int j = 0; j < entry; ++j) {
+    x = cuhe::host::shift_mod(x, bits, mm);
+    put(j, x);  // R^(j+2)
+  }
+  if (scale) {
+    const Limbs u = cuhe::host::mod_reduce(*scale, m);
+    balanced52(cuhe::host::shift_mod(u, bits, m), k, rows + size_t(entry + 1) * 2 * k, 2);
+  }
+  return block;
+}
+
+// -m^-1 mod 2^52 for odd m (Newton's iteration on the low 64 bits)
+unsigned long long negative_inverse52(const Limbs& m) {
+  const uint64_t m0 = (uint64_t(m.size() > 1 ? m[1] : 0u) << 32) | m[0];
+  uint64_t inv = m0;
+  for (int it = 0; it < 6; ++it) inv *= 2 - m0 * inv;
+  return (0 - inv) & ((1ull << 52) - 1);
+}
+
+int upload_constants(cuhe_paillier* ctx, const std::vector<double>& block, double** dptr) {
+  if (!*dptr) CUHE_CUDA(ctx, cudaMalloc(dptr, block.size() * 8), "constants allocation");
+  CUHE_CUDA(ctx, cudaMemcpy(*dptr, block.data(), block.size() * 8, cudaMemcpyHostToDevice), "constants upload");
+  return CUHE_OK;
+}
+
+// k_pair_crt's constants and schedules, from the factors and the secret
+// exponent (whichever came last).  A multiple u (p - 1) of p - 1 with u > 1
+// (a textbook key's phi) is raised as p - 1, half the exponent's length.
+int setup_pair_crt(cuhe_paillier* ctx) {
+  if (!ctx->have_factors) return CUHE_OK;
+  const size_t k = 5 * size_t(ctx->K) / 32;
+  std::vector<double> block;
+  for (int s = 0; s < 2; ++s) {
+    auto& side = ctx->side_exp[s];
+    const Limbs& p = ctx->factor[s];
+    ctx->cs.ninv52[s] = negative_inverse52(p);
+    side.scaled = 0;
+    Limbs cofactor, main = ctx->secret_exp;
+    if (ctx->have_secret && !cuhe::host::is_zero(ctx->secret_exp)) {
+      Limbs pm1 = p;
+      pm1[0] -= 1u;  // p is odd
+      while (pm1.size() > 1 && pm1.back() == 0) pm1.pop_back();
+      if (cuhe::host::is_zero(cuhe::host::mod_reduce(ctx->secret_exp, pm1, &cofactor)) &&
+          cuhe::host::bit_length(cofactor) > 1) {
+        side.scaled = 1;
+        main = pm1;
+      }
+    }
+    const std::vector<double> one = pair_constants(p, k, 4, side.scaled ? &cofactor : nullptr);
+    block.insert(block.end(), one.begin(), one.end());
+    if (!ctx->have_secret) continue;
+    if (int rc = upload_schedule(ctx, main, &side.d_ops, &side.nops, cuhe::kPairWindow)) return rc;
+    if (side.scaled)
+      if (int rc = upload_schedule(ctx, cofactor, &side.d_fall, &side.nfall, cuhe::kPairWindow)) return rc;
+  }
+  return upload_constants(ctx, block, &ctx->d_crt52);
 }
 
 struct DeviceGuard {
@@ -766,6 +881,7 @@ int cuhe_paillier_create(const uint32_t* n_in, int n_words, int device, cuhe_pai
   auto* ctx = new (std::nothrow) cuhe_paillier();
   if (!ctx) return fail(nullptr, CUHE_OUT_OF_MEMORY, "context allocation");
   ctx->device = device;
+  if (cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) ctx->sms = 148;
   ctx->K = K;
   ctx->n_words = K / 2;
   default_tuning(K, &ctx->tpi, &ctx->window);
@@ -814,9 +930,11 @@ int cuhe_paillier_create(const uint32_t* n_in, int n_words, int device, cuhe_pai
     return rc;
   }
   ctx->stream = ctx->own_stream;
+  ctx->pair_ninv = negative_inverse52(nk);
   if (upload_schedule(ctx, nk, &ctx->d_ops_n, &ctx->nops_n) != CUHE_OK ||
-      upload_schedule(ctx, nk, &ctx->d_ops_n52, &ctx->nops_n52, kCrt52Window) != CUHE_OK ||
-      setup_direct52(ctx) != CUHE_OK) {
+      upload_schedule(ctx, nk, &ctx->d_ops_n52, &ctx->nops_n52, cuhe::kPairWindow) != CUHE_OK ||
+      setup_direct52(ctx) != CUHE_OK ||
+      upload_constants(ctx, pair_constants(nk, 5 * k / 16, 2, nullptr), &ctx->d_pair) != CUHE_OK) {
     g_create_error = ctx->error;
     cuhe_paillier_destroy(ctx);
     return CUHE_CUDA_ERROR;
@@ -837,7 +955,12 @@ void cuhe_paillier_destroy(cuhe_paillier* ctx) {
   cudaFree(ctx->d_ops_sec52);
   cudaFree(ctx->d_crt);
   cudaFree(ctx->d_crt52);
+  cudaFree(ctx->d_pair);
   cudaFree(ctx->d_n52);
+  for (auto& side : ctx->side_exp) {
+    cudaFree(side.d_ops);
+    cudaFree(side.d_fall);
+  }
   cudaFree(ctx->d_ops_n52);
   cudaFree(ctx->d_gtab);
   cudaFree(ctx->d_wide);
@@ -926,7 +1049,8 @@ int cuhe_paillier_set_secret(cuhe_paillier* ctx, const uint32_t* exponent, int e
   ctx->ks.mult_is_zero = cuhe::host::is_zero(mult) ? 1u : 0u;
   ctx->secret_exp = e;
   ctx->have_secret = true;
-  if (int rc = upload_schedule(ctx, e, &ctx->d_ops_sec52, &ctx->nops_sec52, kCrt52Window)) return rc;
+  if (int rc = upload_schedule(ctx, e, &ctx->d_ops_sec52, &ctx->nops_sec52, cuhe::kPairWindow)) return rc;
+  if (int rc = setup_pair_crt(ctx)) return rc;
   return upload_schedule(ctx, e, &ctx->d_ops_sec, &ctx->nops_sec);
 }
 
@@ -960,33 +1084,13 @@ int cuhe_paillier_set_factors(cuhe_paillier* ctx, const uint32_t* p_in, int p_wo
   auto put_half = [&](int row, int s, const Limbs& v) {
     std::memcpy(block.data() + size_t(row) * k + size_t(s) * kh, v.data(), 4 * kh);
   };
-  // FP64-pipe kernel: K52 = 5 KH / 8 limbs of 52 bits per side, R52 = 2^(52 K52)
-  const size_t k52 = 5 * kh / 8;
-  std::vector<double> block52(2 * 2 * k52, 0.0);
-  auto put52 = [&](int s, int row, const Limbs& v) {
-    for (size_t i = 0; i < k52; ++i) {
-      uint64_t limb = 0;
-      for (int b = 0; b < 52; ++b) {
-        const size_t bit = 52 * i + size_t(b);
-        if (bit / 32 < v.size() && ((v[bit / 32] >> (bit % 32)) & 1u)) limb |= 1ull << b;
-      }
-      block52[(size_t(s) * 2 + size_t(row)) * k52 + i] = double(limb);
-    }
-  };
   for (int s = 0; s < 2; ++s) {
     Limbs rm = cuhe::host::shift_mod(one, 32 * kh, side[s]);
     put_half(cuhe::CR_M, s, side[s]);
     put_half(cuhe::CR_RM, s, rm);
     put_half(cuhe::CR_R3, s, cuhe::host::shift_mod(rm, 64 * kh, side[s]));
-    put_half(cuhe::CR_R52, s, cuhe::host::shift_mod(one, 52 * k52 + 64 * kh, side[s]));
+    put_half(cuhe::CR_PR, s, cuhe::host::shift_mod(cuhe::host::resized((s ? q : p).data(), kh, kh), 32 * kh, side[s]));
     ctx->cs.ninv[s] = 0u - cuhe::host::inv32(side[s][0]);
-    // -(M^-1) mod 2^52 by Newton's iteration on the low 64 bits of M
-    const uint64_t m0 = (uint64_t(side[s][1]) << 32) | side[s][0];
-    uint64_t inv = m0;
-    for (int it = 0; it < 6; ++it) inv *= 2 - m0 * inv;
-    ctx->cs.ninv52[s] = (0 - inv) & ((1ull << 52) - 1);
-    put52(s, 0, side[s]);
-    put52(s, 1, cuhe::host::shift_mod(one, 52 * k52, side[s]));
   }
   put_half(cuhe::CR_H, 0, cuhe::host::shift_mod(qinv, 32 * kh, side[0]));
   Limbs cq = cuhe::host::shift_mod(cuhe::host::resized(side[1].data(), kh, k), 32 * k, ctx->n2);
@@ -995,11 +1099,10 @@ int cuhe_paillier_set_factors(cuhe_paillier* ctx, const uint32_t* p_in, int p_wo
   CUHE_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronize before CRT constants upload");
   if (!ctx->d_crt) CUHE_CUDA(ctx, cudaMalloc(&ctx->d_crt, block.size() * 4), "CRT constants allocation");
   CUHE_CUDA(ctx, cudaMemcpy(ctx->d_crt, block.data(), block.size() * 4, cudaMemcpyHostToDevice), "CRT constants upload");
-  if (!ctx->d_crt52) CUHE_CUDA(ctx, cudaMalloc(&ctx->d_crt52, block52.size() * 8), "CRT constants allocation");
-  CUHE_CUDA(ctx, cudaMemcpy(ctx->d_crt52, block52.data(), block52.size() * 8, cudaMemcpyHostToDevice),
-            "CRT constants upload");
+  ctx->factor[0] = p;
+  ctx->factor[1] = q;
   ctx->have_factors = true;
-  return CUHE_OK;
+  return setup_pair_crt(ctx);
 }
 
 int cuhe_paillier_has_factors(const cuhe_paillier* ctx) { return ctx && ctx->have_factors ? 1 : 0; }
@@ -1028,7 +1131,7 @@ int cuhe_paillier_encrypt(cuhe_paillier* ctx, const uint32_t* m, const uint32_t*
   st.add(r, bytes, true, false);
   st.add(c, bytes, false, true);
   if (int rc = st.bind()) return rc;
-  if (Modexp52 f = direct52(ctx)) {
+  if (PairModexp f = pair_modexp(ctx)) {
     CUHE_CUDA(ctx, f(ctx, (const uint32_t*)st.dev(1), (const uint32_t*)st.dev(0), (uint32_t*)st.dev(2), count,
                      ctx->d_ops_n52, ctx->nops_n52, cuhe::EXP_ENCRYPT, 0),
               "encrypt launch");
@@ -1272,8 +1375,8 @@ int cuhe_paillier_modexp(cuhe_paillier* ctx, const uint32_t* base, const uint32_
   // exponent of any width: build its schedule
   Limbs e(exponent, exponent + exponent_words);
   while (e.size() > 1 && e.back() == 0) e.pop_back();
-  const Modexp52 f52 = direct52(ctx);
-  std::vector<int32_t> ops = cuhe::host::window_schedule(e, f52 ? kCrt52Window : ctx->window);
+  const PairModexp f52 = pair_modexp(ctx);
+  std::vector<int32_t> ops = cuhe::host::window_schedule(e, f52 ? cuhe::kPairWindow : ctx->window);
   if (!ops.empty()) {
     if (cudaError_t ce = ctx->tmp_ops.reserve(ops.size() * 4)) return cuda_fail(ctx, ce, "schedule allocation");
     CUHE_CUDA(ctx, cudaMemcpyAsync(ctx->tmp_ops.ptr, ops.data(), ops.size() * 4, cudaMemcpyHostToDevice, ctx->stream),
@@ -1722,7 +1825,7 @@ struct cuhe_mix {
     cuhe::ModexpTask* d_tasks = nullptr;
     std::vector<int32_t*> d_ops;
     Dispatch d;
-    bool fp52 = false;  // k_modexp52_tasks: every context of the width selects the FP64 pipe
+    bool fp52 = false;  // k_pair_modexp_tasks: every context of the width selects the FP64 pipe
     cudaError_t (*prepare)(int, int*) = nullptr;
     cudaError_t (*launch)(const cuhe::ModexpTask*, int, long long, unsigned long long*, int*, int,
                           cudaStream_t) = nullptr;
@@ -1847,15 +1950,15 @@ int cuhe_mix_plan(cuhe_mix* mix) {
     if (!find_dispatch(w.K, w.tpi, w.window, &w.d)) return mix_fail(mix, CUHE_INVALID_ARGUMENT, "no compiled variant");
     // the pipe follows the contexts, as their one-launch-per-batch calls do
     w.fp52 = true;
-    for (size_t i : kv.second) w.fp52 = w.fp52 && direct52(mix->entries[i].ctx) != nullptr;
+    for (size_t i : kv.second) w.fp52 = w.fp52 && pair_modexp(mix->entries[i].ctx) != nullptr;
     w.prepare = w.d.prepare_tasks;
     w.launch = w.d.launch_tasks;
     if (w.fp52) {
-      w.window = kCrt52Window;
-      w.tpi = w.K / 16;
-      if (w.K == 64) { w.prepare = &prepare_tasks52<64>; w.launch = &launch_tasks52<64>; }
-      if (w.K == 128) { w.prepare = &prepare_tasks52<128>; w.launch = &launch_tasks52<128>; }
-      if (w.K == 256) { w.prepare = &prepare_tasks52<256>; w.launch = &launch_tasks52<256>; }
+      w.window = cuhe::kPairWindow;
+      w.tpi = w.K / 32;
+      if (w.K == 64) { w.prepare = &prepare_pair_tasks<64>; w.launch = &launch_pair_tasks<64>; }
+      if (w.K == 128) { w.prepare = &prepare_pair_tasks<128>; w.launch = &launch_pair_tasks<128>; }
+      if (w.K == 256) { w.prepare = &prepare_pair_tasks<256>; w.launch = &launch_pair_tasks<256>; }
     }
     const long long ipb = cuhe::kBlockThreads / w.tpi;
     std::vector<cuhe::ModexpTask> tasks;
@@ -1882,8 +1985,8 @@ int cuhe_mix_plan(cuhe_mix* mix) {
       t.ks = e.ctx->ks;
       t.nops = int(ops.size());
       t.mode = cuhe::EXP_POW;
-      t.n52 = e.ctx->d_n52;
-      t.ninv52 = e.ctx->ninv52;
+      t.n52 = e.ctx->d_pair;
+      t.ninv52 = e.ctx->pair_ninv;
       tasks.push_back(t);
       w.units += (e.count + ipb - 1) / ipb;
     }

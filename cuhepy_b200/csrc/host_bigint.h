@@ -126,14 +126,19 @@ inline void sub_mod(Limbs& x, const Limbs& y, const Limbs& m) {
   if (sub_in_place(x, y)) add_in_place(x, m);
 }
 
-// x mod m (bitwise long division; m nonzero).  Result has m's limb count.
-inline Limbs mod_reduce(const Limbs& x, const Limbs& m) {
+// x mod m (bitwise long division; m nonzero).  Result has m's limb count, the
+// quotient (when asked for) x's.
+inline Limbs mod_reduce(const Limbs& x, const Limbs& m, Limbs* quotient = nullptr) {
   Limbs r(m.size(), 0u);
+  if (quotient) quotient->assign(x.size(), 0u);
   for (size_t i = bit_length(x); i-- > 0;) {
     const uint32_t top = r.back() >> 31;
     for (size_t k = r.size(); k-- > 1;) r[k] = (r[k] << 1) | (r[k - 1] >> 31);
     r[0] = (r[0] << 1) | ((x[i / 32] >> (i % 32)) & 1u);
-    if (top || cmp(r, m) >= 0) sub_in_place(r, m);
+    if (top || cmp(r, m) >= 0) {
+      sub_in_place(r, m);
+      if (quotient) (*quotient)[i / 32] |= 1u << (i % 32);
+    }
   }
   return r;
 }

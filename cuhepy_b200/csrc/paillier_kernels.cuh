@@ -8,6 +8,7 @@
 #include <cstdint>
 #include "bigint52.cuh"
 #include "bigint_group.cuh"
+#include "pair52.cuh"
 
 namespace cuhe {
 
@@ -33,13 +34,13 @@ enum CrtRow : int {
   CR_R3 = 2,   // R_h^3 mod p^2 | R_h^3 mod q^2
   CR_H = 3,    // (q^2)^-1 R_h mod p^2 | 0
   CR_CQ = 4,   // q^2 R mod n^2 (full row)
-  CR_R52 = 5,  // R52 R_h^2 mod p^2 | R52 R_h^2 mod q^2, R52 = 2^(52 K52) (FP64-pipe kernel)
+  CR_PR = 5,   // p R_h mod p^2 | q R_h mod q^2
   CR_ROWS = 6
 };
 
 struct CrtScalars {
   uint32_t ninv[2];   // -(p^2)^-1, -(q^2)^-1 mod 2^32
-  unsigned long long ninv52[2];  // -(p^2)^-1, -(q^2)^-1 mod 2^52
+  unsigned long long ninv52[2];  // -p^-1, -q^-1 mod 2^52
 };
 
 struct KeyScalars {
@@ -353,8 +354,8 @@ struct ModexpTask {
   KeyScalars ks;
   int nops;
   int mode;
-  const double* n52;            // k_modexp52_tasks: the key's 52-bit constants
-  unsigned long long ninv52;
+  const double* n52;            // k_pair_modexp_tasks: the key's constants mod n (pair_const_doubles)
+  unsigned long long ninv52;    // -n^-1 mod 2^52
 };
 
 // Persistent mixed launch: CTAs take units (IPB instances of one task) from
@@ -518,24 +519,6 @@ k_modexp_crt(const uint32_t* __restrict__ base, uint32_t* __restrict__ out, long
   decrypt_epilogue<K, 2 * TPI>(g, x, out, inst, consts, ks, s_one, s_r2n, s_multr, mode, pop_words);
 }
 
-// ---------------------------------------------------------------------------
-// The same CRT decrypt / decode with both exponentiations on the FP64 pipe.
-//
-// Per side the value mod M (p^2 or q^2, KH 32-bit words) is carried as
-// K52 = 5 KH / 8 limbs of 52 bits on TPI = KH / 16 lanes (ten limbs per
-// lane, sixteen 32-bit words), in the Montgomery domain of R52 = 2^(52 K52)
-// (cuhe52::Group52).  Ten limbs per lane give each lane twenty independent
-// products per step to cover the latency of the step's m; a 3-bit window
-// keeps the table small enough for four CTAs per SM.  Entry and
-// exit stay in 32-bit words: c R_h^-1 by the 32-bit reduction as in
-// k_modexp_crt, then * (R52 R_h^2 mod M) gives c R52 mod M, which is
-// re-cut into 52-bit limbs through shared memory; the odd-power table and
-// the window schedule run as 52-bit Montgomery products; the result mod M
-// is re-cut into 32-bit words and the Garner recombination and epilogue of
-// k_modexp_crt follow unchanged, so the output equals k_modexp_crt's (and
-// the direct kernel's) for every c < n^2.
-// ---------------------------------------------------------------------------
-
 // limb i (52 bits at 52 i) of a little-endian array of nwords 32-bit words
 __device__ __forceinline__ uint64_t limb52_from_words(const uint32_t* w, int nwords, int i) {
   const int bit = 52 * i, j = bit >> 5, off = bit & 31;
@@ -557,370 +540,447 @@ __device__ __forceinline__ uint32_t word_from_limbs52(const uint64_t* l, int nli
   return uint32_t(v);
 }
 
-template <int KH, int W>
-__global__ void __launch_bounds__(kBlockThreads, 3)
-k_modexp_crt52(const uint32_t* __restrict__ base, uint32_t* __restrict__ out, long long count,
-               const uint32_t* __restrict__ consts, KeyScalars ks, const uint32_t* __restrict__ crt, CrtScalars cs,
-               const double* __restrict__ crt52, const int32_t* __restrict__ ops, int nops, int mode,
-               int pop_words, int* status) {
-  constexpr int K = 2 * KH;
-  constexpr int TPI = KH / 16;     // lanes per side
-  constexpr int L = 16;            // 32-bit words per lane and side
-  constexpr int K52 = 5 * KH / 8;  // 52-bit limbs per side
-  constexpr int L52 = K52 / TPI;   // ten
-  static_assert(L52 == 10, "ten limbs per lane");
-  static_assert(52 * K52 > 32 * KH + 1, "R52 must exceed 2 M");
-  constexpr int T = 1 << (W - 1);
-  constexpr int IPB = kBlockThreads / (2 * TPI);
-  constexpr int SIDE = (T + 1) * K52 + 2;  // doubles per side: x, then T odd powers; +2 moves the banks
-  extern __shared__ __align__(16) uint32_t smem[];
-  // block rows: ONE, R2N, MULTR (K words each), RM, R52, H (two halves), CQ; then 1 as K52 doubles
-  uint32_t* s_one = smem;
-  uint32_t* s_r2n = smem + K;
-  uint32_t* s_multr = smem + 2 * K;
-  uint32_t* s_rm = smem + 3 * K;
-  uint32_t* s_r52 = smem + 4 * K;
-  uint32_t* s_h = smem + 5 * K;
-  uint32_t* s_cq = smem + 6 * K;
-  double* s_one52 = reinterpret_cast<double*>(smem + 7 * K);
-  double* s_items = s_one52 + K52;
-  {
-    const int rows[3] = {C_ONE, C_R2N, C_MULTR};
-    copy_rows_to_smem<K, TPI>(smem, consts, rows, 3);
-    const int crows[4] = {CR_RM, CR_R52, CR_H, CR_CQ};
-    copy_rows_to_smem<K, TPI>(smem + 3 * K, crt, crows, 4);
-    for (int i = threadIdx.x; i < K52; i += blockDim.x) s_one52[i] = i == 0 ? 1.0 : 0.0;
-  }
-  __syncthreads();
+// ---------------------------------------------------------------------------
+// Exponentiation mod m^2 on pairs of residues mod m (pair52.cuh): the
+// decrypt / decode kernel by the Chinese remainder theorem (m = p and q), and
+// the kernel mod n^2 (m = n) for encryption's r^n, public powers and
+// decryption without the factors.  K limbs of 52 bits a component on TPI
+// lanes, 128 threads.  kL = 10 limbs per lane with two CTAs per SM (about 250
+// registers a thread, which let the compiler interleave the accumulations;
+// 168 registers and three CTAs: 1,530 against 2,045 M squarings a second at
+// 2,048-bit m^2) is the best rate; kL = 5 spreads a value over twice the lanes
+// for batches that leave SMs idle: 1,960 M a second when the GPU is full, but
+// 2.7 us a squaring against 4.7 for a warp alone (the host's rule:
+// pair_small).
+//
+// A value of 32-bit words enters as kEntry chunks u_j of 52 K bits,
+// x R = sum_j u_j (R^(j+2) R^-1), one product with a constant pair each, and
+// leaves by a product with the pair (1, 0), its components re-cut to 32-bit
+// words in [0, m]; the recombination, the Paillier factor 1 + a n (the pair
+// (1, a): it takes the place of (1, 0)) and the L() epilogue follow on words.
+// ---------------------------------------------------------------------------
+constexpr int kPairWindow = 3;                       // odd powers x, x^3, x^5, x^7
+constexpr int kPairTable = 1 << (kPairWindow - 1);
 
-  Group<K, 2 * TPI> g;            // the whole ciphertext, 32-bit words
-  Group<KH, TPI> h;               // this side's half, 32-bit words
-  cuhe52::Group52<K52, TPI> f;    // this side's half, 52-bit limbs
-  const int side = (threadIdx.x / TPI) & 1;
-  const int slot = threadIdx.x / (2 * TPI);
-  const long long inst = (long long)blockIdx.x * IPB + slot;
-  if (inst >= count) return;  // both halves leave together
-  double* s_x = s_items + (slot * 2 + side) * SIDE;
-  double* s_tab = s_x + K52;
+// Constants of one modulus m as doubles: m as K limbs, then rows of K pairs:
+// the entry chunks' R^(j+2) mod m^2, (1, 0), (u R mod m, 0) and R mod m^2.
+__host__ __device__ constexpr int pair_const_doubles(int K, int entry) { return K + 2 * K * (entry + 3); }
 
-  {
-    uint32_t c[L], n2[L];
-    g.load_ro(n2, consts + C_N2 * K);
-    g.load(c, base + inst * K);
-    if (!g.less_than(c, n2)) {
-      if (g.gl == 0) atomicOr(status, ST_RANGE);
-      return;
-    }
-  }
-  const uint32_t ninv = cs.ninv[side];
-  uint32_t* s_w = reinterpret_cast<uint32_t*>(s_x);  // KH words fit in the K52 doubles of x
-  {
-    // c = lo + hi R_h:  (lo + hi * (R_h mod M)) R_h^-1 = c R_h^-1, then * R52 R_h^2 R_h^-1 = c R52
-    uint32_t m[L], lo[L], hi[L], acc[L];
-    h.load_ro(m, crt + CR_M * K + side * KH);
-    h.load(lo, base + inst * K);
-    h.load(hi, base + inst * K + KH);
-    h.mont_mul_acc(acc, lo, hi, s_rm + side * KH, m, ninv);
-    h.mont_mul(acc, acc, s_r52 + side * KH, m, ninv);
-    h.publish(s_w, acc);
-  }
-  double x52[L52], m52[L52], acc52[L52];
-  const double* cm = crt52 + side * 2 * K52;  // M, then R52 mod M
+// An exponent's window schedule, or x^e by way of x^(m-1) (PairExponent::scaled).
+struct PairExponent {
+  const int32_t* ops;
+  const int32_t* fall;
+  int nops, nfall;
+  // e = u (p - 1): the schedule is that of p - 1.  When x^(p-1) = 1 + p z1
+  // (always, for x prime to a prime p), x^e = 1 + p (z1 u mod p); any other
+  // value in a warp sends the warp through the schedule `fall` of u, which
+  // holds for every x and every p.
+  int scaled;
+};
+
+template <int K, int TPI>
+__device__ __forceinline__ void pair_publish(const cuhe52::Pair52<K, TPI>& f, double2* s, const double (&x)[K / TPI],
+                                             const double (&y)[K / TPI]) {
+  __syncwarp();
 #pragma unroll
-  for (int k = 0; k < L52; ++k) {
-    x52[k] = cuhe52::to_f64(limb52_from_words(s_w, KH, f.gl * L52 + k));
-    m52[k] = __ldg(cm + f.gl * L52 + k);
-  }
-  const uint64_t ninv52 = cs.ninv52[side];
-  f.publish(s_tab, x52);
-#pragma unroll
-  for (int k = 0; k < L52; ++k) acc52[k] = x52[k];
-  // Every Montgomery product of the exponentiation goes through the one
-  // call site below: the unrolled product is large, and a single copy of it
-  // stays in the instruction cache.  Phases: the odd-power table (x^2 to
-  // s_x, then x^3 .. x^(2T-1)), the window schedule (squarings of s_x and
-  // products with table entries), the final product with 1.
-  enum { kTable = 0, kSchedule = 1, kFinal = 2, kDone = 3 };
-  int phase = T > 1 ? kTable : kSchedule, pc = 0, o = 1, sq_left = 0, idx = 0;
-  if (phase == kSchedule) pc = T;  // no table products: go straight to the schedule set-up
-  double xs52[L52];
-  while (phase != kDone) {
-    if (phase == kTable || pc == T) {
-      // (after the table) the schedule starts from its first table entry
-      if (phase == kSchedule && pc == T) {
-        pc = 0;
-        if (nops == 0) {
-#pragma unroll
-          for (int k = 0; k < L52; ++k) acc52[k] = __ldg(cm + K52 + f.gl * L52 + k);  // e = 0: R52 mod M
-        } else {
-          const int first = __ldg(ops) & 0xffff;
-          __syncwarp(f.mask);
-#pragma unroll
-          for (int k = 0; k < L52; ++k) acc52[k] = s_tab[(first - 1) * K52 + f.gl * L52 + k];
-        }
-        f.publish(s_x, acc52);
-        while (sq_left == 0 && idx == 0) {
-          if (o >= nops) {
-            phase = kFinal;
-            break;
-          }
-          const int op = __ldg(ops + o++);
-          sq_left = op >> 16;
-          idx = op & 0xffff;
-        }
-      }
-    }
-    const double* bsrc = phase == kTable   ? (pc == 0 ? s_tab : s_x)
-                         : phase == kFinal ? s_one52
-                         : sq_left > 0     ? s_x
-                                           : s_tab + (idx - 1) * K52;
-    f.mont_mul(xs52, acc52, bsrc, m52, ninv52);
-    if (phase == kFinal) break;  // xs52 = x_side, canonical
-    if (phase == kTable && pc == 0) {
-      f.publish(s_x, xs52);  // x^2 R52; acc52 stays x
-    } else {
-#pragma unroll
-      for (int k = 0; k < L52; ++k) acc52[k] = xs52[k];
-      f.publish(phase == kTable ? s_tab + pc * K52 : s_x, acc52);
-    }
-    if (phase == kTable) {
-      if (++pc == T) phase = kSchedule;  // pc == T: set-up at the top of the next pass
-      continue;
-    }
-    if (sq_left > 0) --sq_left;
-    else idx = 0;
-    while (sq_left == 0 && idx == 0) {
-      if (o >= nops) {
-        phase = kFinal;
-        break;
-      }
-      const int op = __ldg(ops + o++);
-      sq_left = op >> 16;
-      idx = op & 0xffff;
-    }
-  }
-  uint64_t* s_l = reinterpret_cast<uint64_t*>(s_x);
-  __syncwarp(f.mask);
-#pragma unroll
-  for (int k = 0; k < L52; ++k) s_l[f.gl * L52 + k] = cuhe52::to_u64(xs52[k]);
-  __syncwarp(f.mask);
-  uint32_t xs[L];
-#pragma unroll
-  for (int j = 0; j < L; ++j) xs[j] = word_from_limbs52(s_l, K52, h.gl * L + j);
-  __syncwarp(g.mask);
-  uint32_t* s_xp = reinterpret_cast<uint32_t*>(s_items + (slot * 2) * SIDE);
-  uint32_t* s_xq = reinterpret_cast<uint32_t*>(s_items + (slot * 2 + 1) * SIDE);
-  h.store(side == 0 ? s_xp : s_xq, xs);
-  __syncwarp(g.mask);
-  if (side == 0) {
-    // h = x_p (q^2)^-1 - x_q (q^2)^-1 mod p^2   (x_q may exceed p^2; x_q < R_h)
-    uint32_t m[L], xq[L], v[L], u[L];
-    h.load_ro(m, crt + CR_M * K);
-    h.load(xq, s_xq);
-    h.mont_mul(v, xs, s_h, m, ninv);
-    h.mont_mul(u, xq, s_h, m, ninv);
-    sub_mod<KH, TPI>(h, v, u, m);
-    __syncwarp(h.mask);
-    h.store(s_xp, v);
-  }
-  __syncwarp(g.mask);
-  // x = x_q + q^2 h over the whole group: side 0 lanes hold the low words
-  uint32_t hv[L], xq[L], x[L];
-  if (side == 0) {
-    h.load(hv, s_xp);
-    h.load(xq, s_xq);
-  } else {
-#pragma unroll
-    for (int j = 0; j < L; ++j) hv[j] = xq[j] = 0u;
-  }
-  uint32_t n2[L];
-  g.load_ro(n2, consts + C_N2 * K);
-  g.mont_mul(x, hv, s_cq, n2, ks.ninv2);  // h q^2 mod n^2 = h q^2
-  (void)add_group<K, 2 * TPI>(g, x, xq);
-  decrypt_epilogue<K, 2 * TPI>(g, x, out, inst, consts, ks, s_one, s_r2n, s_multr, mode, pop_words);
+  for (int k = 0; k < K / TPI; ++k) s[f.gl * (K / TPI) + k] = make_double2(x[k], y[k]);
+  __syncwarp();
 }
 
-// ---------------------------------------------------------------------------
-// The exponentiation mod n^2 itself on the FP64 pipe, for the exponents that
-// need no factors (encryption's r^n, any fixed public exponent) and for
-// decryption when the factors are not installed.  The value is carried as
-// K52 = 5K/8 limbs of 52 bits on K/16 lanes (ten limbs per lane) in the
-// Montgomery domain of R52 = 2^(52 K52), with k_modexp_crt52's product and
-// schedule; entry: x R52 mod n^2 by one 32-bit Montgomery product with
-// R52 R mod n^2, exit: the product with 1, re-cut into 32-bit words; then
-// k_modexp's modes on 32-bit words (the factor 1 + m n of an encryption,
-// the L() / popcount epilogue), so every output equals k_modexp's.
-// n52: n^2 and R52 mod n^2 as K52 doubles each, then R52 R mod n^2 as K words.
-// ---------------------------------------------------------------------------
-template <int K, int W>
-__device__ __forceinline__ void modexp52_unit(const uint32_t* __restrict__ base, const uint32_t* __restrict__ aux,
-                                              int aux_words, uint32_t* __restrict__ out, long long count,
-                                              const uint32_t* __restrict__ consts, const KeyScalars& ks,
-                                              const double* __restrict__ n52, unsigned long long ninv52,
-                                              const int32_t* __restrict__ ops, int nops, int mode, int pop_words,
-                                              int* status, long long block) {
-  constexpr int TPI = K / 16;      // lanes per value
-  constexpr int L = 16;            // 32-bit words per lane
-  constexpr int K52 = 5 * K / 8;   // 52-bit limbs
-  constexpr int L52 = K52 / TPI;   // ten
-  static_assert(L52 == 10, "ten limbs per lane");
-  static_assert(52 * K52 > 32 * K + 1, "R52 must exceed 2 n^2");
-  constexpr int T = 1 << (W - 1);
-  constexpr int IPB = kBlockThreads / TPI;
-  constexpr int SLOT = (T + 1) * K52 + 2;  // doubles per value: x, then T odd powers; +2 moves the banks
+// x^e for this group's value (all lanes of the warp call it): words = the
+// value, nwords of them; rows = the modulus' constant pairs in shared memory
+// (kEntry entry rows, (1, 0), the scale row); one = R mod m^2 in global
+// memory; s = this group's K pairs, tab = this thread's table column (stride
+// kPairThreads).  aux: null, or the words a of the factor (1, a).  Leaves the
+// canonical limbs (z0, z1), each in [0, m], as pairs of 64-bit integers in s.
+template <int K, int TPI, int kEntry>
+__device__ __forceinline__ void pair_power(const cuhe52::Pair52<K, TPI>& f, const uint32_t* __restrict__ words,
+                                           int nwords, const double2* rows, const double2* __restrict__ one,
+                                           double2* s, double2* tab, const double (&m)[K / TPI], uint64_t ninv,
+                                           const PairExponent& ex, const uint32_t* __restrict__ aux) {
+  constexpr int L = K / TPI;
+  constexpr int kStride = cuhe52::kPairThreads;
+  const int32_t* ops = ex.ops;
+  int nops = ex.nops;
+  bool scaled = ex.scaled != 0;
+  double z0[L], z1[L], a0[L], a1[L];
+  uint64_t A0[L], A1[L];
+  const int at = f.gl * L;
+  auto bits = [](double d) { return static_cast<uint64_t>(__double_as_longlong(d)); };
+  auto raw = [](uint64_t v) { return __longlong_as_double(static_cast<long long>(v)); };
+
+  int j = 0;  // entry chunks, then the square of x; again from there with the schedule ex.fall
+  while (true) {
+#pragma unroll 1
+    for (; j <= kEntry; ++j) {
+      if (j < kEntry) {
+#pragma unroll
+        for (int k = 0; k < L; ++k) a0[k] = f.to_f64(limb52_from_words(words, nwords, j * K + at + k));
+      } else {
+        if (nops == 0) break;
+#pragma unroll
+        for (int k = 0; k < L; ++k) {
+          tab[k * kStride] = make_double2(z0[k], z1[k]);
+          a0[k] = z0[k];
+        }
+        f.twice_limbs(a1, z1);
+        pair_publish<K, TPI>(f, s, z0, a1);
+      }
+      f.template product<false>(A0, A1, a0, a0, j < kEntry ? rows + j * K : s, m, ninv);
+      if (j == kEntry) {  // x^2 stays in s for the odd powers, x in z
+        f.template limbs<2>(a0, A0);
+        f.template limbs<2>(a1, A1);
+        pair_publish<K, TPI>(f, s, a0, a1);
+        break;
+      }
+      // the chunks are summed as columns, kept in s between them
+      f.template columns<2>(A0);
+      f.template columns<2>(A1);
+#pragma unroll
+      for (int k = 0; k < L; ++k) {
+        if (j > 0) {
+          A0[k] += bits(s[at + k].x);
+          A1[k] += bits(s[at + k].y);
+        }
+        s[at + k] = make_double2(raw(A0[k]), raw(A1[k]));
+      }
+      if (j == kEntry - 1) {
+        f.from_columns(z0, A0);
+        f.from_columns(z1, A1);
+      }
+    }
+    if (nops == 0) {  // e = 0
+#pragma unroll
+      for (int k = 0; k < L; ++k) {
+        const double2 t = __ldg(one + at + k);
+        z0[k] = t.x;
+        z1[k] = t.y;
+      }
+    } else {
+#pragma unroll 1
+      for (int t = 1; t < kPairTable; ++t) {  // x^(2t+1) = x^(2t-1) x^2
+        f.template product<true>(A0, A1, z0, z1, s, m, ninv);
+        f.template limbs<2>(z0, A0);
+        f.template limbs<3>(z1, A1);
+#pragma unroll
+        for (int k = 0; k < L; ++k) tab[(t * L + k) * kStride] = make_double2(z0[k], z1[k]);
+      }
+      const int first = (__ldg(ops) & 0xffff) - 1;
+#pragma unroll
+      for (int k = 0; k < L; ++k) {
+        const double2 t = tab[(first * L + k) * kStride];
+        z0[k] = t.x;
+        z1[k] = t.y;
+      }
+    }
+    // Each op squares at least once and then multiplies by a table entry; the
+    // last pass is the way out, the product with (1, 0) or (1, aux).
+    f.twice_limbs(a1, z1);
+    int op = nops > 1 ? __ldg(ops + 1) : 0;
+#pragma unroll 1
+    for (int o = 1;; ++o) {
+      const bool out = o >= nops;
+      const int sq = out ? 0 : op >> 16, idx = op & 0xffff;
+      if (o + 1 < nops) op = __ldg(ops + o + 1);
+#pragma unroll 1
+      for (int i = 1; i <= sq; ++i) {
+        pair_publish<K, TPI>(f, s, z0, a1);  // (z0, 2 z1)
+        f.template product<false>(A0, A1, z0, z0, s, m, ninv);
+        f.template limbs<2>(z0, A0);
+        if (i < sq) f.template twice<2>(a1, A1);
+        else f.template limbs<2>(z1, A1);
+      }
+      const double2* b = s;
+      if (out) {
+        if (aux) {
+          double one0[L];
+#pragma unroll
+          for (int k = 0; k < L; ++k) {
+            A1[k] = limb52_from_words(aux, nwords, at + k);
+            one0[k] = at + k == 0 ? 1.0 : 0.0;
+          }
+          f.from_columns(a1, A1);
+          pair_publish<K, TPI>(f, s, one0, a1);
+        } else {
+          b = rows + kEntry * K;
+        }
+#pragma unroll
+        for (int k = 0; k < L; ++k) {
+          a0[k] = z0[k];
+          a1[k] = z1[k];
+        }
+      } else {
+        if (idx == 0) continue;  // the schedule's last squarings
+        pair_publish<K, TPI>(f, s, z0, z1);
+#pragma unroll
+        for (int k = 0; k < L; ++k) {
+          const double2 t = tab[((idx - 1) * L + k) * kStride];
+          a0[k] = t.x;
+          a1[k] = t.y;
+        }
+      }
+      f.template product<true>(A0, A1, a0, a1, b, m, ninv);
+      if (out) break;
+      f.template limbs<2>(z0, A0);
+      f.template limbs<3>(z1, A1);
+      f.template twice<3>(a1, A1);
+    }
+    f.template columns<2>(A0);
+    f.template columns<3>(A1);
+    f.canonical(A0);
+    f.canonical(A1);
+    bool isone = true;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+      s[at + k] = make_double2(raw(A0[k]), raw(A1[k]));
+      isone = isone && A0[k] == (at + k == 0 ? 1ull : 0ull);
+    }
+    __syncwarp();
+    if (!scaled) return;
+    if (__all_sync(0xffffffffu, isone)) break;
+    // x^(p-1) is not 1 mod p somewhere: raise it (still in z) to u instead
+    scaled = false;
+    ops = ex.fall;
+    nops = ex.nfall;
+    j = kEntry;
+  }
+  // (1, z1) -> (1, z1 u mod p)
+#pragma unroll
+  for (int k = 0; k < L; ++k) a0[k] = f.to_f64(A1[k]);
+  f.template product<false>(A0, A1, a0, a0, rows + (kEntry + 1) * K, m, ninv);
+  f.template columns<2>(A0);
+  f.canonical(A0);
+#pragma unroll
+  for (int k = 0; k < L; ++k) s[at + k].y = raw(A0[k]);
+  __syncwarp();
+}
+
+// word i (32 bits at 32 i) of component `second` of K pairs of 64-bit limbs
+template <int K>
+__device__ __forceinline__ uint32_t word_from_pairs(const double2* s, bool second, int i) {
+  const int bit = 32 * i, j = bit / 52, off = bit - 52 * j;
+  auto limb = [&](int k) -> uint64_t {
+    if (k >= K) return 0;
+    return static_cast<uint64_t>(__double_as_longlong(second ? s[k].y : s[k].x));
+  };
+  uint64_t v = limb(j) >> off;
+  if (off > 20) v |= limb(j + 1) << (52 - off);
+  return uint32_t(v);
+}
+
+// x = z1 m + z0 mod m^2 (canonical) over a group, from the pairs in s: mr =
+// m R mod m^2 (R = 2^(32K)), mm = m^2.
+template <int KL, int K, int TPI>
+__device__ __forceinline__ void pair_words(const Group<K, TPI>& g, uint32_t (&x)[K / TPI], const double2* s,
+                                           const uint32_t* mr, const uint32_t (&mm)[K / TPI], uint32_t ninv) {
+  constexpr int L = K / TPI;
+  uint32_t z[L];
+#pragma unroll
+  for (int j = 0; j < L; ++j) z[j] = word_from_pairs<KL>(s, true, g.gl * L + j);
+  g.mont_mul(x, z, mr, mm, ninv);  // z1 m, at most m^2 - m
+#pragma unroll
+  for (int j = 0; j < L; ++j) z[j] = word_from_pairs<KL>(s, false, g.gl * L + j);
+  (void)add_group<K, TPI>(g, x, z);  // at most m^2
+  if (!g.less_than(x, mm)) sub_group<K, TPI>(g, x, mm);
+}
+
+template <int K, int kL, int kEntry, int kSides>
+struct PairLayout {  // K limbs per component (kL per lane), kSides moduli per item
+  static constexpr int TPI = K / kL;
+  static constexpr int kGroups = cuhe52::kPairThreads / TPI;   // values of a CTA
+  static constexpr int kItems = kGroups / kSides;
+  static constexpr int kRows = (kEntry + 2) * K;               // constant pairs per modulus
+  static constexpr int kSlot = K + 1;                          // pairs per value; +1 moves the banks
+  static constexpr size_t kTab = size_t(kPairTable) * kL * cuhe52::kPairThreads;
+  static constexpr size_t kBytes = (size_t(kSides) * kRows + size_t(kGroups) * kSlot + kTab) * 16;
+};
+
+// Decrypt / decode with the factors installed: c^e mod p^2 and mod q^2 in the
+// two halves of the CTA (whole warps per side, so each side follows its own
+// schedule), then Garner's recombination and the epilogue of k_modexp_crt on
+// words, 2 KH / 16 lanes per ciphertext.
+template <int KH, int kL>
+__global__ void __launch_bounds__(cuhe52::kPairThreads, 2)
+k_pair_crt(const uint32_t* __restrict__ base, uint32_t* __restrict__ out, long long count,
+           const uint32_t* __restrict__ consts, KeyScalars ks, const uint32_t* __restrict__ crt, CrtScalars cs,
+           const double* __restrict__ crt52, PairExponent e0, PairExponent e1, int mode, int pop_words, int* status) {
+  constexpr int K = 2 * KH, KL = 5 * KH / 16, kEntry = 4;
+  using Lay = PairLayout<KL, kL, kEntry, 2>;
+  constexpr int IPB = Lay::kItems, TPI = Lay::TPI;
   extern __shared__ __align__(16) uint32_t smem[];
-  // block rows: ONE, R2, NR, R2N, MULTR, R52 R (K words each); then 1 as K52 doubles
-  uint32_t* s_one = smem;
-  uint32_t* s_r2 = smem + K;
-  uint32_t* s_nr = smem + 2 * K;
-  uint32_t* s_r2n = smem + 3 * K;
-  uint32_t* s_multr = smem + 4 * K;
-  uint32_t* s_r52r = smem + 5 * K;
-  double* s_one52 = reinterpret_cast<double*>(smem + 6 * K);
-  double* s_items = s_one52 + K52;
-  {
-    const int rows[5] = {C_ONE, C_R2, C_NR, C_R2N, C_MULTR};
-    copy_rows_to_smem<K, TPI>(smem, consts, rows, 5);
-    const uint32_t* r52r = reinterpret_cast<const uint32_t*>(n52 + 2 * K52);
-    for (int i = threadIdx.x; i < K; i += blockDim.x) s_r52r[i] = r52r[i];
-    for (int i = threadIdx.x; i < K52; i += blockDim.x) s_one52[i] = i == 0 ? 1.0 : 0.0;
+  double2* s_rows = reinterpret_cast<double2*>(smem);
+  double2* s_vals = s_rows + 2 * Lay::kRows;
+  double2* s_tab = s_vals + Lay::kGroups * Lay::kSlot;
+  constexpr int kConst = pair_const_doubles(KL, kEntry);
+  for (int i = threadIdx.x; i < 2 * Lay::kRows; i += blockDim.x) {
+    const int sd = i / Lay::kRows;
+    s_rows[i] = reinterpret_cast<const double2*>(crt52 + sd * kConst + KL)[i - sd * Lay::kRows];
   }
   __syncthreads();
-
-  Group<K, TPI> g;                // the value, 32-bit words
-  cuhe52::Group52<K52, TPI> f;    // the value, 52-bit limbs (same lanes)
-  const int slot = threadIdx.x / TPI;
-  const long long inst = block * IPB + slot;
-  if (inst >= count) return;  // whole groups leave together
-  double* s_x = s_items + slot * SLOT;
-  double* s_tab = s_x + K52;
-  uint32_t* s_w = reinterpret_cast<uint32_t*>(s_x);  // K words fit in the K52 doubles of x
-  uint32_t n2[L];
-  g.load_ro(n2, consts + C_N2 * K);
+  const long long first = (long long)blockIdx.x * IPB;
   {
-    uint32_t x[L], xr[L];
+    const int side = threadIdx.x / (cuhe52::kPairThreads / 2);
+    const int group = threadIdx.x / TPI;  // side * IPB + item
+    const long long inst = min(first + group - side * IPB, count - 1);  // idle groups repeat the last item
+    cuhe52::Pair52<KL, TPI> f;
+    const double* cm = crt52 + side * kConst;
+    double m[kL];
+#pragma unroll
+    for (int k = 0; k < kL; ++k) m[k] = __ldg(cm + f.gl * kL + k);
+    pair_power<KL, TPI, kEntry>(f, base + inst * K, K, s_rows + side * Lay::kRows,
+                                reinterpret_cast<const double2*>(cm + KL) + (kEntry + 2) * KL,
+                                s_vals + group * Lay::kSlot, s_tab + threadIdx.x, m,
+                                f.gl == 0 ? cs.ninv52[side] : 0ull, side ? e1 : e0, nullptr);
+  }
+  __syncthreads();
+  // words: ONE, R2N, MULTR (K words each), p R_h, H (two halves), CQ, then
+  // per item of a pass x_p and x_q (KH words each), over the powers' table
+  constexpr int LT = KH / 16, L = 16;  // lanes per side
+  constexpr int PER = cuhe52::kPairThreads / (2 * LT);
+  uint32_t* s_one = reinterpret_cast<uint32_t*>(s_tab);
+  uint32_t* s_r2n = s_one + K;
+  uint32_t* s_multr = s_one + 2 * K;
+  uint32_t* s_pr = s_one + 3 * K;
+  uint32_t* s_h = s_one + 4 * K;
+  uint32_t* s_cq = s_one + 5 * K;
+  {
+    const int rows[3] = {C_ONE, C_R2N, C_MULTR};
+    copy_rows_to_smem<K, LT>(s_one, consts, rows, 3);
+    const int crows[3] = {CR_PR, CR_H, CR_CQ};
+    copy_rows_to_smem<K, LT>(s_pr, crt, crows, 3);
+  }
+  __syncthreads();
+  Group<K, 2 * LT> g;  // the whole ciphertext
+  Group<KH, LT> h;     // this side's half
+  const int side = (threadIdx.x / LT) & 1;
+  const int slot = threadIdx.x / (2 * LT);
+  uint32_t* s_xp = s_one + 6 * K + slot * (K + 4);
+  uint32_t* s_xq = s_xp + KH;
+#pragma unroll 1
+  for (int item = slot; item < IPB; item += PER) {
+    const long long inst = first + item;
+    if (inst >= count) break;
+    uint32_t n2[L], x[L], m[L], hv[L], xq[L];
+    g.load_ro(n2, consts + C_N2 * K);
     g.load(x, base + inst * K);
     if (!g.less_than(x, n2)) {
       if (g.gl == 0) atomicOr(status, ST_RANGE);
-      return;
-    }
-    g.mont_mul(xr, x, s_r52r, n2, ks.ninv2);  // x R52 mod n^2
-    g.publish(s_w, xr);
-  }
-  double x52[L52], m52[L52], acc52[L52];
-#pragma unroll
-  for (int k = 0; k < L52; ++k) {
-    x52[k] = cuhe52::to_f64(limb52_from_words(s_w, K, f.gl * L52 + k));
-    m52[k] = __ldg(n52 + f.gl * L52 + k);
-  }
-  f.publish(s_tab, x52);
-#pragma unroll
-  for (int k = 0; k < L52; ++k) acc52[k] = x52[k];
-  // One call site for every product (k_modexp_crt52): the odd-power table,
-  // the window schedule, the final product with 1.
-  enum { kTable = 0, kSchedule = 1, kFinal = 2 };
-  int phase = T > 1 ? kTable : kSchedule, pc = 0, o = 1, sq_left = 0, idx = 0;
-  if (phase == kSchedule) pc = T;
-  double xs52[L52];
-  while (true) {
-    if (phase == kSchedule && pc == T) {
-      pc = 0;
-      if (nops == 0) {
-#pragma unroll
-        for (int k = 0; k < L52; ++k) acc52[k] = __ldg(n52 + K52 + f.gl * L52 + k);  // e = 0: R52 mod n^2
-      } else {
-        const int first = __ldg(ops) & 0xffff;
-        __syncwarp(f.mask);
-#pragma unroll
-        for (int k = 0; k < L52; ++k) acc52[k] = s_tab[(first - 1) * K52 + f.gl * L52 + k];
-      }
-      f.publish(s_x, acc52);
-      while (sq_left == 0 && idx == 0) {
-        if (o >= nops) {
-          phase = kFinal;
-          break;
-        }
-        const int op = __ldg(ops + o++);
-        sq_left = op >> 16;
-        idx = op & 0xffff;
-      }
-    }
-    const double* bsrc = phase == kTable   ? (pc == 0 ? s_tab : s_x)
-                         : phase == kFinal ? s_one52
-                         : sq_left > 0     ? s_x
-                                           : s_tab + (idx - 1) * K52;
-    f.mont_mul(xs52, acc52, bsrc, m52, ninv52);
-    if (phase == kFinal) break;  // xs52 = x^e, canonical
-    if (phase == kTable && pc == 0) {
-      f.publish(s_x, xs52);  // x^2 R52; acc52 stays x
-    } else {
-#pragma unroll
-      for (int k = 0; k < L52; ++k) acc52[k] = xs52[k];
-      f.publish(phase == kTable ? s_tab + pc * K52 : s_x, acc52);
-    }
-    if (phase == kTable) {
-      if (++pc == T) phase = kSchedule;  // pc == T: set-up at the top of the next pass
       continue;
     }
-    if (sq_left > 0) --sq_left;
-    else idx = 0;
-    while (sq_left == 0 && idx == 0) {
-      if (o >= nops) {
-        phase = kFinal;
-        break;
-      }
-      const int op = __ldg(ops + o++);
-      sq_left = op >> 16;
-      idx = op & 0xffff;
+    h.load_ro(m, crt + CR_M * K + side * KH);
+    pair_words<KL, KH, LT>(h, x, s_vals + (side * IPB + item) * Lay::kSlot, s_pr + side * KH, m, cs.ninv[side]);
+    __syncwarp(g.mask);
+    h.store(side == 0 ? s_xp : s_xq, x);
+    __syncwarp(g.mask);
+    if (side == 0) {
+      // h = x_p (q^2)^-1 - x_q (q^2)^-1 mod p^2   (x_q may exceed p^2; x_q < R_h)
+      h.load(xq, s_xq);
+      h.mont_mul(hv, x, s_h, m, cs.ninv[0]);
+      h.mont_mul(x, xq, s_h, m, cs.ninv[0]);
+      sub_mod<KH, LT>(h, hv, x, m);
+      __syncwarp(h.mask);
+      h.store(s_xp, hv);
     }
-  }
-  uint64_t* s_l = reinterpret_cast<uint64_t*>(s_x);
-  __syncwarp(f.mask);
+    __syncwarp(g.mask);
+    // x = x_q + q^2 h over the whole group: side 0 lanes hold the low words
+    if (side == 0) {
+      h.load(hv, s_xp);
+      h.load(xq, s_xq);
+    } else {
 #pragma unroll
-  for (int k = 0; k < L52; ++k) s_l[f.gl * L52 + k] = cuhe52::to_u64(xs52[k]);
-  __syncwarp(f.mask);
-  uint32_t x[L];
-#pragma unroll
-  for (int j = 0; j < L; ++j) x[j] = word_from_limbs52(s_l, K52, g.gl * L + j);
-  if (mode == EXP_POW) {
-    g.store(out + inst * K, x);
-    return;
+      for (int j = 0; j < L; ++j) hv[j] = xq[j] = 0u;
+    }
+    g.mont_mul(x, hv, s_cq, n2, ks.ninv2);  // h q^2 mod n^2 = h q^2
+    (void)add_group<K, 2 * LT>(g, x, xq);
+    decrypt_epilogue<K, 2 * LT>(g, x, out, inst, consts, ks, s_one, s_r2n, s_multr, mode, pop_words);
+    __syncwarp(g.mask);
   }
-  if (mode == EXP_ENCRYPT) {
-    uint32_t m[L], nn[L], gm[L], xr[L];
-    g.load(m, aux + inst * aux_words);  // aux_words == K (zero-padded m < n)
-    g.load_ro(nn, consts + C_N * K);
-    if (!g.less_than(m, nn)) {
+}
+
+// The exponentiation mod n^2 (k_modexp's modes): items [block * kItems, ...)
+// of a batch.
+template <int K, int kL>
+__device__ __forceinline__ void pair_modexp_unit(const uint32_t* __restrict__ base, const uint32_t* __restrict__ aux,
+                                                 uint32_t* __restrict__ out, long long count,
+                                                 const uint32_t* __restrict__ consts, const KeyScalars& ks,
+                                                 const double* __restrict__ n52, unsigned long long ninv52,
+                                                 const int32_t* __restrict__ ops, int nops, int mode, int pop_words,
+                                                 int* status, long long block) {
+  constexpr int KL = 5 * K / 16, kEntry = 2;
+  using Lay = PairLayout<KL, kL, kEntry, 1>;
+  constexpr int IPB = Lay::kItems, TPI = Lay::TPI;
+  extern __shared__ __align__(16) uint32_t smem[];
+  double2* s_rows = reinterpret_cast<double2*>(smem);
+  double2* s_vals = s_rows + Lay::kRows;
+  double2* s_tab = s_vals + Lay::kGroups * Lay::kSlot;
+  for (int i = threadIdx.x; i < Lay::kRows; i += blockDim.x)
+    s_rows[i] = reinterpret_cast<const double2*>(n52 + KL)[i];
+  __syncthreads();
+  const long long first = block * IPB;
+  {
+    const int group = threadIdx.x / TPI;
+    const long long inst = min(first + group, count - 1);  // idle groups repeat the last item
+    cuhe52::Pair52<KL, TPI> f;
+    double m[kL];
+#pragma unroll
+    for (int k = 0; k < kL; ++k) m[k] = __ldg(n52 + f.gl * kL + k);
+    const PairExponent ex{ops, nullptr, nops, 0, 0};
+    pair_power<KL, TPI, kEntry>(f, base + inst * K, K, s_rows,
+                                reinterpret_cast<const double2*>(n52 + KL) + (kEntry + 2) * KL,
+                                s_vals + group * Lay::kSlot, s_tab + threadIdx.x, m, f.gl == 0 ? ninv52 : 0ull, ex,
+                                mode == EXP_ENCRYPT ? aux + inst * K : nullptr);
+  }
+  __syncthreads();
+  constexpr int LT = K / 16, L = 16, PER = cuhe52::kPairThreads / LT;
+  uint32_t* s_one = reinterpret_cast<uint32_t*>(s_tab);
+  uint32_t* s_nr = s_one + K;
+  uint32_t* s_r2n = s_one + 2 * K;
+  uint32_t* s_multr = s_one + 3 * K;
+  {
+    const int rows[4] = {C_ONE, C_NR, C_R2N, C_MULTR};
+    copy_rows_to_smem<K, LT>(s_one, consts, rows, 4);
+  }
+  __syncthreads();
+  Group<K, LT> g;
+  uint32_t n2[L], x[L], y[L];
+  g.load_ro(n2, consts + C_N2 * K);
+#pragma unroll 1
+  for (int item = threadIdx.x / LT; item < IPB; item += PER) {
+    const long long inst = first + item;
+    if (inst >= count) break;
+    g.load(x, base + inst * K);
+    bool valid = g.less_than(x, n2);
+    if (mode == EXP_ENCRYPT) {
+      g.load(x, aux + inst * K);
+      g.load_ro(y, consts + C_N * K);
+      valid = g.less_than(x, y) && valid;
+    }
+    if (!valid) {
       if (g.gl == 0) atomicOr(status, ST_RANGE);
-      return;
+      continue;
     }
-    g.mont_mul(gm, m, s_nr, n2, ks.ninv2);  // m*n (exact, < n^2)
-    add_small<K, TPI>(g, gm, 1u);           // 1 + m*n = g^m mod n^2
-    g.publish(s_w, gm);
-    g.mont_mul(xr, x, s_r2, n2, ks.ninv2);  // r^n R
-    g.mont_mul(x, xr, s_w, n2, ks.ninv2);   // r^n * g^m
-    g.store(out + inst * K, x);
-    return;
+    pair_words<KL, K, LT>(g, x, s_vals + item * Lay::kSlot, s_nr, n2, ks.ninv2);
+    if (mode == EXP_POW || mode == EXP_ENCRYPT) g.store(out + inst * K, x);
+    else decrypt_epilogue<K, LT>(g, x, out, inst, consts, ks, s_one, s_r2n, s_multr, mode, pop_words);
   }
-  decrypt_epilogue<K, TPI>(g, x, out, inst, consts, ks, s_one, s_r2n, s_multr, mode, pop_words);
 }
 
-template <int K, int W>
-__global__ void __launch_bounds__(kBlockThreads, 3)
-k_modexp52(const uint32_t* __restrict__ base, const uint32_t* __restrict__ aux, int aux_words,
-           uint32_t* __restrict__ out, long long count, const uint32_t* __restrict__ consts, KeyScalars ks,
-           const double* __restrict__ n52, unsigned long long ninv52, const int32_t* __restrict__ ops, int nops,
-           int mode, int pop_words, int* status) {
-  modexp52_unit<K, W>(base, aux, aux_words, out, count, consts, ks, n52, ninv52, ops, nops, mode, pop_words, status,
-                      blockIdx.x);
+template <int K, int kL>
+__global__ void __launch_bounds__(cuhe52::kPairThreads, 2)
+k_pair_modexp(const uint32_t* __restrict__ base, const uint32_t* __restrict__ aux, uint32_t* __restrict__ out,
+              long long count, const uint32_t* __restrict__ consts, KeyScalars ks, const double* __restrict__ n52,
+              unsigned long long ninv52, const int32_t* __restrict__ ops, int nops, int mode, int pop_words,
+              int* status) {
+  pair_modexp_unit<K, kL>(base, aux, out, count, consts, ks, n52, ninv52, ops, nops, mode, pop_words, status, blockIdx.x);
 }
 
-// The persistent mixed launch (k_modexp_tasks) on the FP64 pipe: units of
-// IPB = 128 / (K/16) instances of one task.
-template <int K, int W>
-__global__ void __launch_bounds__(kBlockThreads, 3)
-k_modexp52_tasks(const ModexpTask* __restrict__ tasks, int ntasks, long long total_units,
-                 unsigned long long* __restrict__ counter, int* status) {
+// The persistent mixed launch (k_modexp_tasks): units of PairLayout::kItems
+// instances of one task.
+template <int K>
+__global__ void __launch_bounds__(cuhe52::kPairThreads, 2)
+k_pair_modexp_tasks(const ModexpTask* __restrict__ tasks, int ntasks, long long total_units,
+                    unsigned long long* __restrict__ counter, int* status) {
   __shared__ long long s_unit;
   while (true) {
     if (threadIdx.x == 0) s_unit = (long long)atomicAdd(counter, 1ull);
@@ -933,8 +993,8 @@ k_modexp52_tasks(const ModexpTask* __restrict__ tasks, int ntasks, long long tot
       if (tasks[mid].first_unit <= unit) lo = mid; else hi = mid - 1;
     }
     const ModexpTask& t = tasks[lo];
-    modexp52_unit<K, W>(t.base, nullptr, K, t.out, t.count, t.consts, t.ks, t.n52, t.ninv52, t.ops, t.nops, t.mode,
-                        0, status, unit - t.first_unit);
+    pair_modexp_unit<K, 10>(t.base, nullptr, t.out, t.count, t.consts, t.ks, t.n52, t.ninv52, t.ops, t.nops, t.mode, 0,
+                        status, unit - t.first_unit);
     __syncthreads();  // shared rows and tables are restaged by the next unit
   }
 }
