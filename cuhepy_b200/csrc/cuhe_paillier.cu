@@ -101,7 +101,7 @@ struct cuhe_paillier {
   double* d_crt52 = nullptr;  // per side: the constants mod p, q of k_pair_crt (pair_const_doubles)
   double* d_pair = nullptr;   // the constants mod n of k_pair_modexp
   unsigned long long pair_ninv = 0;  // -n^-1 mod 2^52
-  double* d_n52 = nullptr;    // n^2 and R52 mod n^2 as 52-bit limbs, then R52 R and R52 mod n^2 in words
+  double* d_n52 = nullptr;    // n^2 and R52 mod n^2 as 52-bit limbs, then R52 R mod n^2 in words
   unsigned long long ninv52 = 0;  // -(n^2)^-1 mod 2^52
   int32_t* d_ops_n52 = nullptr;   // the schedule of n for k_pair_modexp's window
   int nops_n52 = 0;
@@ -116,12 +116,36 @@ struct cuhe_paillier {
   cuhe::CrtScalars cs{};
   bool have_factors = false;
   bool fp64 = true;           // exponentiations, server products and table encryption on the FP64 pipe
-  bool fp64_small = false;    // the latter two also for n^2 of 2048 bits (set_fp64(ctx, 2))
+  bool fp64_small = false;    // server products also for n^2 of 2048 bits (set_fp64(ctx, 2))
   uint32_t* d_gtab = nullptr;
   int message_chunks = 0;
   uint32_t* d_wide = nullptr;  // 16-bit-digit table W[j][D], built on demand (see cuhe_lookup_set_wide_table)
-  double* d_wide52 = nullptr;  // ... as 52-bit limbs in the R52 domain (FP64-pipe encryption), with
-  double* d_noise52 = nullptr; // the noise table likewise
+  // The tables as rows of limb pairs mod n (FP64-pipe encryption), built from
+  // the installed ones when a call first needs them and dropped with them.
+  struct PairTables {
+    double2* digits = nullptr;  // [message_chunks][256]: the 8-bit table
+    double2* embed = nullptr;   // [ceil(message_chunks / 2)][256]: 8 embedding bits (16 plaintext bits)
+    double2* noise = nullptr;   // [noise_entries]
+    double2* noise2 = nullptr;  // [noise_entries][noise_entries]: products of two
+    double2* wide_digits = nullptr;  // [ceil(message_chunks / 2)][65536]: 16-bit digits
+    double2* wide_embed = nullptr;   // [wide_rows][65536]: 16 embedding bits
+    int wide_rows = 0;
+    void release() {
+      for (double2** p : {&digits, &embed, &noise, &noise2, &wide_digits, &wide_embed}) {
+        cudaFree(*p);
+        *p = nullptr;
+      }
+      wide_rows = 0;
+    }
+    void release_wide() {
+      cudaFree(wide_digits);
+      cudaFree(wide_embed);
+      wide_digits = wide_embed = nullptr;
+      wide_rows = 0;
+    }
+    bool wide() const { return wide_digits || wide_embed; }
+  } pt;
+  double2* d_entry = nullptr;  // k_pair_rows' constants
   int wide_mode = 1;           // 0 never, 1 for large batches when it fits, 2 always
   uint32_t* d_noise = nullptr;
   int noise_entries = 0;
@@ -262,8 +286,8 @@ PairModexp pair_modexp(const cuhe_paillier* ctx) {
   return nullptr;
 }
 
-// Whether the server's products and the lookup encryption take 52-bit limbs
-// mod n^2 (n^2 of 4096 or 8192 bits; 2048 bits only with set_fp64(ctx, 2)).
+// Whether the server's products take 52-bit limbs mod n^2 (n^2 of 4096 or
+// 8192 bits; 2048 bits only with set_fp64(ctx, 2)).
 bool limbs52(const cuhe_paillier* ctx) {
   return ctx->fp64 && ctx->d_n52 && (ctx->K >= 128 || ctx->fp64_small);
 }
@@ -302,53 +326,62 @@ Outer52 outer52(const cuhe_paillier* ctx) {
   return nullptr;
 }
 
-// The 16-bit-digit table and the noise table as 52-bit limbs in the R52
-// domain (k_wide_table52 row by row, k_to_mont52 from the 32-bit Montgomery
-// form), and encryption from them.
+// Rows of limb pairs for the lookup encryption (k_pair_rows, k_pair_products)
+// and encryption from them (k_pair_lookup).
 template <int K>
-cudaError_t build_wide52(cuhe_paillier* ctx, double* wide52, double* noise52) {
-  constexpr int TPI = K / 16, K52 = 5 * K / 8, IPB = cuhe::kBlockThreads / TPI;
-  const uint32_t* r52w = reinterpret_cast<const uint32_t*>(ctx->d_n52 + 2 * K52) + K;
-  const size_t smem = size_t(K + IPB * K) * 4;
-  for (int j = 0; j < (ctx->message_chunks + 1) / 2; ++j) {
-    cuhe::k_wide_table52<K><<<dim3(65536 / IPB), cuhe::kBlockThreads, smem, ctx->stream>>>(
-        ctx->d_gtab, ctx->message_chunks, j, wide52, ctx->d_consts, ctx->ks, r52w);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  // no noise table: encryption reports every noise index as out of range
-  if (ctx->noise_entries == 0) return cudaSuccess;
-  cuhe::k_to_mont52<K><<<dim3(unsigned((ctx->noise_entries + IPB - 1) / IPB)), cuhe::kBlockThreads, smem,
-                         ctx->stream>>>(ctx->d_noise, ctx->noise_entries, noise52, ctx->d_consts, ctx->ks, r52w,
-                                        ctx->d_status);
+cudaError_t launch_pair_rows(cuhe_paillier* ctx, const uint32_t* in, long long count, double2* out) {
+  constexpr int KL = 5 * K / 16, IPB = cuhe52::kPairThreads / (KL / 10);
+  const size_t smem = size_t(2 * KL + 1) * 16;
+  cuhe::k_pair_rows<K><<<dim3(unsigned((count + IPB - 1) / IPB)), cuhe52::kPairThreads, smem, ctx->stream>>>(
+      in, count, out, ctx->d_entry, ctx->d_pair, ctx->pair_ninv);
   return cudaGetLastError();
 }
 
 template <int K>
-cudaError_t launch_lookup52(cuhe_paillier* ctx, const uint8_t* bits, int embed_len, int chunk_len, int chunk_num,
-                            const uint32_t* plain, long long count, const uint8_t* idx, uint32_t* out) {
-  constexpr int TPI = K / 16, K52 = 5 * K / 8, IPB = cuhe::kBlockThreads / TPI;
-  const size_t rows_bytes = size_t(IPB) * cuhe::lookup_rows_stride(ctx->message_chunks) * 2;
-  const size_t smem = size_t(K52 + IPB * (K52 + 2)) * 8 + ((rows_bytes + 15) & ~size_t(15));
-  cudaError_t e = cudaFuncSetAttribute(cuhe::k_lookup_encrypt52<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+cudaError_t launch_pair_products(cuhe_paillier* ctx, const double2* src, int rows, int kind, long long first,
+                                 long long count, double2* out) {
+  constexpr int KL = 5 * K / 16, IPB = cuhe52::kPairThreads / (KL / 10);
+  const size_t smem = size_t(IPB) * (KL + 1) * 16;
+  cuhe::k_pair_products<K><<<dim3(unsigned((count + IPB - 1) / IPB)), cuhe52::kPairThreads, smem, ctx->stream>>>(
+      src, rows, kind, first, count, out, ctx->d_pair, ctx->pair_ninv);
+  return cudaGetLastError();
+}
+
+template <int K, int kL>
+cudaError_t launch_pair_lookup_l(cuhe_paillier* ctx, const cuhe::LookupDigits& dg, long long count,
+                                 const double2* table, const double2* noise, bool pairs, const uint8_t* idx,
+                                 uint32_t* out) {
+  using Lay = cuhe::LookupLayout<K, kL>;
+  const size_t smem = Lay::bytes(dg.rows);
+  cudaError_t e = cudaFuncSetAttribute(cuhe::k_pair_lookup<K, kL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        int(smem));
   if (e != cudaSuccess) return e;
-  cuhe::k_lookup_encrypt52<K><<<dim3(unsigned((count + IPB - 1) / IPB)), cuhe::kBlockThreads, smem, ctx->stream>>>(
-      bits, embed_len, chunk_len, chunk_num, plain, K, count, ctx->message_chunks, ctx->d_wide52, ctx->d_noise52,
-      ctx->noise_entries, idx, out, ctx->d_n52, ctx->ninv52, ctx->d_status);
+  const long long blocks = (count + Lay::kGroups - 1) / Lay::kGroups;
+  cuhe::k_pair_lookup<K, kL><<<dim3(unsigned(blocks)), cuhe52::kPairThreads, smem, ctx->stream>>>(
+      dg, count, table, noise, ctx->noise_entries, pairs ? 1 : 0, idx, out, ctx->d_consts, ctx->ks, ctx->d_pair,
+      ctx->pair_ninv, ctx->d_status);
   return cudaGetLastError();
 }
 
-struct Lookup52 {
-  cudaError_t (*build)(cuhe_paillier*, double*, double*);
-  cudaError_t (*launch)(cuhe_paillier*, const uint8_t*, int, int, int, const uint32_t*, long long, const uint8_t*,
-                        uint32_t*);
+template <int K>
+cudaError_t launch_pair_lookup(cuhe_paillier* ctx, const cuhe::LookupDigits& dg, long long count, const double2* table,
+                               const double2* noise, bool pairs, const uint8_t* idx, uint32_t* out) {
+  if (pair_small(ctx, count, cuhe::LookupLayout<K, 5>::kGroups))
+    return launch_pair_lookup_l<K, 5>(ctx, dg, count, table, noise, pairs, idx, out);
+  return launch_pair_lookup_l<K, 10>(ctx, dg, count, table, noise, pairs, idx, out);
+}
+
+struct PairLookup {
+  cudaError_t (*rows)(cuhe_paillier*, const uint32_t*, long long, double2*);
+  cudaError_t (*products)(cuhe_paillier*, const double2*, int, int, long long, long long, double2*);
+  cudaError_t (*launch)(cuhe_paillier*, const cuhe::LookupDigits&, long long, const double2*, const double2*, bool,
+                        const uint8_t*, uint32_t*);
 };
-bool lookup52(const cuhe_paillier* ctx, Lookup52* l) {
-  if (!limbs52(ctx)) return false;
-  if (ctx->K == 64) *l = {&build_wide52<64>, &launch_lookup52<64>};
-  else if (ctx->K == 128) *l = {&build_wide52<128>, &launch_lookup52<128>};
-  else if (ctx->K == 256) *l = {&build_wide52<256>, &launch_lookup52<256>};
+bool pair_lookup(const cuhe_paillier* ctx, PairLookup* l) {
+  if (!ctx->fp64 || !ctx->d_pair) return false;
+  if (ctx->K == 64) *l = {&launch_pair_rows<64>, &launch_pair_products<64>, &launch_pair_lookup<64>};
+  else if (ctx->K == 128) *l = {&launch_pair_rows<128>, &launch_pair_products<128>, &launch_pair_lookup<128>};
+  else if (ctx->K == 256) *l = {&launch_pair_rows<256>, &launch_pair_products<256>, &launch_pair_lookup<256>};
   else return false;
   return true;
 }
@@ -671,8 +704,6 @@ cudaError_t stream_after(cudaStream_t waiter, cudaStream_t from) {
 constexpr long long kWideMinItems = 1 << 16;
 constexpr size_t kWideMaxBytes = size_t(8) << 30;
 
-int ensure_wide_table(cuhe_paillier* ctx, const Dispatch& d, long long items);
-
 int check_status(cuhe_paillier* ctx, bool synchronous) {
   // Range errors are reported by the kernels through d_status; reading it
   // needs a synchronisation, done only for calls that already synchronise.
@@ -706,7 +737,7 @@ int setup_direct52(cuhe_paillier* ctx) {
   const size_t k = size_t(ctx->K), k52 = 5 * k / 8;
   Limbs one(k, 0u);
   one[0] = 1u;
-  std::vector<double> block(2 * k52 + k, 0.0);
+  std::vector<double> block(2 * k52 + k / 2, 0.0);
   auto put52 = [&](size_t row, const Limbs& v) {
     for (size_t i = 0; i < k52; ++i) {
       uint64_t limb = 0;
@@ -721,8 +752,6 @@ int setup_direct52(cuhe_paillier* ctx) {
   put52(1, cuhe::host::shift_mod(one, 52 * k52, ctx->n2));
   const Limbs r52r = cuhe::host::shift_mod(one, 52 * k52 + 32 * k, ctx->n2);
   std::memcpy(block.data() + 2 * k52, r52r.data(), 4 * k);
-  const Limbs r52 = cuhe::host::shift_mod(one, 52 * k52, ctx->n2);
-  std::memcpy(block.data() + 2 * k52 + k / 2, r52.data(), 4 * k);
   const uint64_t m0 = (uint64_t(ctx->n2[1]) << 32) | ctx->n2[0];
   uint64_t inv = m0;
   for (int it = 0; it < 6; ++it) inv *= 2 - m0 * inv;
@@ -964,8 +993,8 @@ void cuhe_paillier_destroy(cuhe_paillier* ctx) {
   cudaFree(ctx->d_ops_n52);
   cudaFree(ctx->d_gtab);
   cudaFree(ctx->d_wide);
-  cudaFree(ctx->d_wide52);
-  cudaFree(ctx->d_noise52);
+  ctx->pt.release();
+  cudaFree(ctx->d_entry);
   cudaFree(ctx->d_noise);
   for (cudaStream_t st : {ctx->copy, ctx->side})
     if (st) cudaStreamSynchronize(st);
@@ -1559,6 +1588,79 @@ int cuhe_paillier_mulmod_outer(cuhe_paillier* ctx, const uint32_t* query, int64_
   return check_status(ctx, true);
 }
 
+}  // extern "C"
+
+namespace {
+
+bool capturing(const cuhe_paillier* ctx) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+}
+
+// One table of rows: allocate, then build on the context's stream and wait (a
+// later call may use another stream).  A table that does not fit, or is first
+// wanted under stream capture, leaves *out null (CUHE_OK: another one serves
+// the call).
+template <class Build>
+int pair_table(cuhe_paillier* ctx, double2** out, long long rows, Build build) {
+  if (*out || capturing(ctx)) return CUHE_OK;
+  double2* t = nullptr;
+  if (cudaMalloc(&t, size_t(rows) * size_t(5 * ctx->K / 16) * 16) != cudaSuccess) {
+    cudaGetLastError();
+    return CUHE_OK;
+  }
+  cudaError_t e = build(t);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) {
+    cudaFree(t);
+    return cuda_fail(ctx, e, "lookup table build");
+  }
+  *out = t;
+  return CUHE_OK;
+}
+
+// The 8-bit digit, embedding and noise rows (65,536 + 32,768 + 256 rows at
+// key_len 1024, 63 MB): made when tables are installed, or by the first call
+// after the pipe was changed.
+int pair_tables(cuhe_paillier* ctx, const PairLookup& pl) {
+  auto& pt = ctx->pt;
+  const int chunks = ctx->message_chunks, entries = ctx->noise_entries, rows8 = (chunks + 1) / 2;
+  if (chunks == 0 || entries == 0 || (pt.digits && pt.noise && pt.embed)) return CUHE_OK;
+  if (capturing(ctx)) return CUHE_OK;
+  if (!ctx->d_entry) {  // R^(j+2) 2^(-32K) mod n^2 as pairs
+    const size_t k = size_t(ctx->K), kl = 5 * k / 16;
+    Limbs n = ctx->n;
+    while (n.size() > 1 && n.back() == 0) n.pop_back();
+    Limbs x(k, 0u);
+    x[0] = 1u;
+    x = cuhe::host::shift_mod(x, 52 * kl, ctx->n2);
+    for (size_t i = 0; i < 32 * k; ++i) cuhe::host::half_mod(x, ctx->n2);
+    std::vector<double> block(4 * kl, 0.0);
+    for (int j = 0; j < 2; ++j) {
+      x = cuhe::host::shift_mod(x, 52 * kl, ctx->n2);
+      Limbs quotient;
+      const Limbs rem = cuhe::host::mod_reduce(x, n, &quotient);
+      balanced52(rem, kl, block.data() + size_t(j) * 2 * kl, 2);
+      balanced52(quotient, kl, block.data() + size_t(j) * 2 * kl + 1, 2);
+    }
+    if (int rc = upload_constants(ctx, block, reinterpret_cast<double**>(&ctx->d_entry))) return rc;
+  }
+  if (int rc = pair_table(ctx, &pt.digits, (long long)chunks * 256, [&](double2* t) {
+        return pl.rows(ctx, ctx->d_gtab, (long long)chunks * 256, t);
+      }))
+    return rc;
+  if (int rc = pair_table(ctx, &pt.noise, entries, [&](double2* t) { return pl.rows(ctx, ctx->d_noise, entries, t); }))
+    return rc;
+  if (!pt.digits) return CUHE_OK;
+  return pair_table(ctx, &pt.embed, (long long)rows8 * 256, [&](double2* t) {
+    return pl.products(ctx, pt.digits, chunks, cuhe::kEmbed, 0, (long long)rows8 * 256, t);
+  });
+}
+
+}  // namespace
+
+extern "C" {
+
 int cuhe_lookup_set_tables(cuhe_paillier* ctx, const uint32_t* g_table, int message_chunks, const uint32_t* noise,
                            int noise_entries) {
   if (!ctx || !g_table || !noise || message_chunks <= 0 || noise_entries <= 0 || noise_entries > 256)
@@ -1573,13 +1675,10 @@ int cuhe_lookup_set_tables(cuhe_paillier* ctx, const uint32_t* g_table, int mess
   cudaFree(ctx->d_gtab);
   cudaFree(ctx->d_noise);
   cudaFree(ctx->d_wide);
-  cudaFree(ctx->d_wide52);
-  cudaFree(ctx->d_noise52);
+  ctx->pt.release();
   ctx->d_gtab = nullptr;
   ctx->d_noise = nullptr;
   ctx->d_wide = nullptr;
-  ctx->d_wide52 = nullptr;
-  ctx->d_noise52 = nullptr;
   ctx->message_chunks = 0;
   ctx->noise_entries = 0;
   CUHE_CUDA(ctx, cudaMalloc(&ctx->d_gtab, gbytes), "table allocation");
@@ -1595,7 +1694,8 @@ int cuhe_lookup_set_tables(cuhe_paillier* ctx, const uint32_t* g_table, int mess
   if (int rc = check_status(ctx, true)) return rc;
   ctx->message_chunks = message_chunks;
   ctx->noise_entries = noise_entries;
-  return CUHE_OK;
+  PairLookup pl{};
+  return pair_lookup(ctx, &pl) ? pair_tables(ctx, pl) : CUHE_OK;
 }
 
 int cuhe_lookup_build_tables(cuhe_paillier* ctx, const uint32_t* g, int message_chunks, const uint32_t* noise,
@@ -1636,12 +1736,9 @@ int cuhe_lookup_build_tables(cuhe_paillier* ctx, const uint32_t* g, int message_
   CUHE_CUDA(ctx, d.convert(ctx, b, (uint32_t*)bm.ptr, message_chunks, 1), "row conversion");
   cudaFree(ctx->d_gtab);
   cudaFree(ctx->d_wide);
-  cudaFree(ctx->d_wide52);
-  cudaFree(ctx->d_noise52);
+  ctx->pt.release();
   ctx->d_gtab = nullptr;
   ctx->d_wide = nullptr;
-  ctx->d_wide52 = nullptr;
-  ctx->d_noise52 = nullptr;
   ctx->message_chunks = 0;
   CUHE_CUDA(ctx, cudaMalloc(&ctx->d_gtab, size_t(message_chunks) * 256 * kb), "table allocation");
   CUHE_CUDA(ctx, d.table_rows(ctx, (const uint32_t*)bm.ptr, message_chunks, ctx->d_gtab), "table rows");
@@ -1663,7 +1760,8 @@ int cuhe_lookup_build_tables(cuhe_paillier* ctx, const uint32_t* g, int message_
   if (int rc = check_status(ctx, true)) return rc;
   ctx->message_chunks = message_chunks;
   if (noise) ctx->noise_entries = noise_entries;
-  return CUHE_OK;
+  PairLookup pl{};
+  return pair_lookup(ctx, &pl) ? pair_tables(ctx, pl) : CUHE_OK;
 }
 
 int cuhe_lookup_get_g_table(cuhe_paillier* ctx, uint32_t* out) {
@@ -1687,44 +1785,119 @@ int cuhe_lookup_get_g_table(cuhe_paillier* ctx, uint32_t* out) {
 
 namespace {
 
+// The wide table's share of device memory under the default policy.
+int wide_allowed(cuhe_paillier* ctx, long long items, size_t bytes, bool* allowed) {
+  *allowed = ctx->wide_mode == 2;
+  if (ctx->wide_mode != 1 || items < kWideMinItems || bytes > kWideMaxBytes) return CUHE_OK;
+  size_t free_bytes = 0, total_bytes = 0;
+  CUHE_CUDA(ctx, cudaMemGetInfo(&free_bytes, &total_bytes), "free memory");
+  *allowed = bytes <= free_bytes / 4;
+  return CUHE_OK;
+}
+
 int ensure_wide_table(cuhe_paillier* ctx, const Dispatch& d, long long items) {
-  if (ctx->d_wide || ctx->d_wide52 || ctx->wide_mode == 0 || !ctx->d_gtab) return CUHE_OK;
-  if (ctx->wide_mode == 1 && items < kWideMinItems) return CUHE_OK;
-  // the table as the selected pipe takes it: 52-bit limbs (doubles, K52 =
-  // 5K/8 a row) for the FP64 pipe, else 32-bit words
-  Lookup52 l52{};
-  const bool fp52 = lookup52(ctx, &l52);
-  const size_t entry = fp52 ? size_t(5 * ctx->K / 8) * 8 : size_t(ctx->K) * 4;
-  const size_t bytes = size_t((ctx->message_chunks + 1) / 2) * 65536 * entry;
-  if (ctx->wide_mode == 1) {
-    size_t free_bytes = 0, total_bytes = 0;
-    CUHE_CUDA(ctx, cudaMemGetInfo(&free_bytes, &total_bytes), "free memory");
-    if (bytes > kWideMaxBytes || bytes > free_bytes / 4) return CUHE_OK;
-  }
+  if (ctx->d_wide || !ctx->d_gtab) return CUHE_OK;
+  const size_t bytes = size_t((ctx->message_chunks + 1) / 2) * 65536 * size_t(ctx->K) * 4;
+  bool allowed = false;
+  if (int rc = wide_allowed(ctx, items, bytes, &allowed)) return rc;
+  if (!allowed) return CUHE_OK;
   void* wide = nullptr;
-  void* noise52 = nullptr;
-  cudaError_t e = cudaMalloc(&wide, bytes);
-  if (e == cudaSuccess && fp52 && ctx->noise_entries > 0)
-    e = cudaMalloc(&noise52, size_t(ctx->noise_entries) * entry);
-  if (e != cudaSuccess) {
+  if (cudaMalloc(&wide, bytes) != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(wide);
     if (ctx->wide_mode == 2) return fail(ctx, CUHE_OUT_OF_MEMORY, "wide table allocation");
     return CUHE_OK;
   }
-  e = fp52 ? l52.build(ctx, static_cast<double*>(wide), static_cast<double*>(noise52))
-           : d.wide_table(ctx, static_cast<uint32_t*>(wide));
-  if (e != cudaSuccess) {
+  if (cudaError_t e = d.wide_table(ctx, static_cast<uint32_t*>(wide))) {
     cudaFree(wide);
-    cudaFree(noise52);
     return cuda_fail(ctx, e, "wide table build");
   }
-  if (fp52) {
-    ctx->d_wide52 = static_cast<double*>(wide);
-    ctx->d_noise52 = static_cast<double*>(noise52);
+  ctx->d_wide = static_cast<uint32_t*>(wide);
+  return CUHE_OK;
+}
+
+// Noise products of two repay their table (noise_entries^2 products, seven
+// saved by a ciphertext) from this many ciphertexts in one call.
+constexpr long long kNoisePairItems = 8192;
+
+// Encryption from the limb-pair tables, building those the call needs; *done
+// is false (nothing launched) when they do not fit in device memory.
+int pair_lookup_encrypt(cuhe_paillier* ctx, const PairLookup& pl, cuhe::LookupDigits dg, long long count,
+                        const uint8_t* idx, uint32_t* out, bool* done) {
+  *done = false;
+  auto& pt = ctx->pt;
+  const int chunks = ctx->message_chunks, entries = ctx->noise_entries;
+  if (int rc = pair_tables(ctx, pl)) return rc;
+  if (!pt.digits || !pt.noise) return CUHE_OK;
+  if (count >= kNoisePairItems)
+    if (int rc = pair_table(ctx, &pt.noise2, (long long)entries * entries, [&](double2* t) {
+          return pl.products(ctx, pt.noise, entries, cuhe::kNoise, 0, (long long)entries * entries, t);
+        }))
+      return rc;
+  const double2* table = pt.digits;
+  dg.message_chunks = chunks;
+  dg.rows = chunks;
+  dg.wide = dg.embed_bits = 0;
+  const size_t row_bytes = size_t(5 * ctx->K / 16) * 16;
+  bool allowed = false;
+  if (dg.bits && dg.chunk_len % 2 == 0 && pt.embed) {
+    const int rows8 = (chunks + 1) / 2;
+    // rows that this call's chunks reach (32 plaintext bits each)
+    const int reach = std::min(2 * dg.embed_len, dg.chunk_len);
+    const int need8 = std::min(rows8, (reach + 15) / 16), need = (need8 + 1) / 2;
+    if (pt.wide_rows < need && !capturing(ctx)) {
+      if (int rc = wide_allowed(ctx, count, size_t(need) * 65536 * row_bytes, &allowed)) return rc;
+      if (allowed) {
+        double2* wide = nullptr;
+        const int before = pt.wide_rows;
+        if (cudaMalloc(&wide, size_t(need) * 65536 * row_bytes) != cudaSuccess) {
+          cudaGetLastError();
+          if (ctx->wide_mode == 2) return fail(ctx, CUHE_OUT_OF_MEMORY, "wide table allocation");
+        } else {
+          cudaError_t e = before ? cudaMemcpyAsync(wide, pt.wide_embed, size_t(before) * 65536 * row_bytes,
+                                                   cudaMemcpyDeviceToDevice, ctx->stream)
+                                 : cudaSuccess;
+          if (e == cudaSuccess)
+            e = pl.products(ctx, pt.embed, rows8, cuhe::kWide, (long long)before * 65536,
+                            (long long)(need - before) * 65536, wide);
+          if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+          if (e != cudaSuccess) {
+            cudaFree(wide);
+            return cuda_fail(ctx, e, "wide table build");
+          }
+          cudaFree(pt.wide_embed);
+          pt.wide_embed = wide;
+          pt.wide_rows = need;
+        }
+      }
+    }
+    const bool wide = pt.wide_rows >= need && pt.wide_embed;
+    dg.embed_bits = wide ? 16 : 8;
+    dg.rows = wide ? need : need8;
+    table = wide ? pt.wide_embed : pt.embed;
   } else {
-    ctx->d_wide = static_cast<uint32_t*>(wide);
+    const int rows = (chunks + 1) / 2;
+    if (!pt.wide_digits && !capturing(ctx)) {
+      if (int rc = wide_allowed(ctx, count, size_t(rows) * 65536 * row_bytes, &allowed)) return rc;
+      if (allowed) {
+        if (int rc = pair_table(ctx, &pt.wide_digits, (long long)rows * 65536, [&](double2* t) {
+              return pl.products(ctx, pt.digits, chunks, cuhe::kWide, 0, (long long)rows * 65536, t);
+            }))
+          return rc;
+        if (!pt.wide_digits && ctx->wide_mode == 2) return fail(ctx, CUHE_OUT_OF_MEMORY, "wide table allocation");
+      }
+    }
+    if (pt.wide_digits) {
+      dg.wide = 1;
+      dg.rows = rows;
+      table = pt.wide_digits;
+    }
   }
+  // a short table's pairs are complete for every valid index; with any other
+  // the call reports the range error
+  const bool pairs = pt.noise2 != nullptr;
+  cudaError_t e = pl.launch(ctx, dg, count, table, pairs ? pt.noise2 : pt.noise, pairs, idx, out);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "lookup encrypt launch");
+  *done = true;
   return CUHE_OK;
 }
 
@@ -1737,19 +1910,16 @@ int cuhe_lookup_set_wide_table(cuhe_paillier* ctx, int mode) {
   DeviceGuard guard(ctx->device);
   std::lock_guard<std::mutex> lock(ctx->mu);
   ctx->wide_mode = mode;
-  if (mode == 0 && (ctx->d_wide || ctx->d_wide52)) {
+  if (mode == 0 && (ctx->d_wide || ctx->pt.wide())) {
     CUHE_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "wide table release");
     cudaFree(ctx->d_wide);
-    cudaFree(ctx->d_wide52);
-    cudaFree(ctx->d_noise52);
     ctx->d_wide = nullptr;
-    ctx->d_wide52 = nullptr;
-    ctx->d_noise52 = nullptr;
+    ctx->pt.release_wide();
   }
   return CUHE_OK;
 }
 
-int cuhe_lookup_wide_table_ready(const cuhe_paillier* ctx) { return ctx && (ctx->d_wide || ctx->d_wide52) ? 1 : 0; }
+int cuhe_lookup_wide_table_ready(const cuhe_paillier* ctx) { return ctx && (ctx->d_wide || ctx->pt.wide()) ? 1 : 0; }
 
 int cuhe_lookup_encrypt_bits(cuhe_paillier* ctx, const uint8_t* bits, int64_t vectors, int embed_len, int chunk_len,
                              int chunk_num, const uint8_t* noise_index, uint32_t* out) {
@@ -1765,17 +1935,29 @@ int cuhe_lookup_encrypt_bits(cuhe_paillier* ctx, const uint8_t* bits, int64_t ve
   Dispatch d;
   find_dispatch(ctx->K, ctx->tpi, ctx->window, &d);
   const int64_t total = vectors * chunk_num;
-  if (int rc = ensure_wide_table(ctx, d, total)) return rc;
+  PairLookup pl{};
+  const bool pairs = pair_lookup(ctx, &pl);
   Stager st(ctx);
   st.add(bits, size_t(vectors) * embed_len, true, false);
   st.add(noise_index, size_t(total) * cuhe::kNoiseMultiples, true, false);
   st.add(out, size_t(total) * ctx->K * 4, false, true);
   if (int rc = st.bind()) return rc;
-  Lookup52 l52{};
-  const bool fp52 = ctx->d_wide52 && lookup52(ctx, &l52);
-  CUHE_CUDA(ctx, (fp52 ? l52.launch : d.lookup)(ctx, (const uint8_t*)st.dev(0), embed_len, chunk_len, chunk_num, nullptr,
-                                               total, (const uint8_t*)st.dev(1), (uint32_t*)st.dev(2)),
-            "lookup encrypt launch");
+  bool done = false;
+  if (pairs) {
+    cuhe::LookupDigits dg{};
+    dg.bits = (const uint8_t*)st.dev(0);
+    dg.embed_len = embed_len;
+    dg.chunk_len = chunk_len;
+    dg.chunk_num = chunk_num;
+    if (int rc = pair_lookup_encrypt(ctx, pl, dg, total, (const uint8_t*)st.dev(1), (uint32_t*)st.dev(2), &done))
+      return rc;
+  }
+  if (!done) {
+    if (int rc = ensure_wide_table(ctx, d, total)) return rc;
+    CUHE_CUDA(ctx, d.lookup(ctx, (const uint8_t*)st.dev(0), embed_len, chunk_len, chunk_num, nullptr, total,
+                            (const uint8_t*)st.dev(1), (uint32_t*)st.dev(2)),
+              "lookup encrypt launch");
+  }
   if (int rc = st.finish()) return rc;
   return check_status(ctx, st.staged());
 }
@@ -1790,17 +1972,28 @@ int cuhe_lookup_encrypt_ints(cuhe_paillier* ctx, const uint32_t* m, int64_t coun
   std::lock_guard<std::mutex> lock(ctx->mu);
   Dispatch d;
   find_dispatch(ctx->K, ctx->tpi, ctx->window, &d);
-  if (int rc = ensure_wide_table(ctx, d, count)) return rc;
+  PairLookup pl{};
+  const bool pairs = pair_lookup(ctx, &pl);
   Stager st(ctx);
   st.add(m, size_t(count) * ctx->K * 4, true, false);
   st.add(noise_index, size_t(count) * cuhe::kNoiseMultiples, true, false);
   st.add(out, size_t(count) * ctx->K * 4, false, true);
   if (int rc = st.bind()) return rc;
-  Lookup52 l52{};
-  const bool fp52 = ctx->d_wide52 && lookup52(ctx, &l52);
-  CUHE_CUDA(ctx, (fp52 ? l52.launch : d.lookup)(ctx, nullptr, 0, 0, 1, (const uint32_t*)st.dev(0), count,
-                                               (const uint8_t*)st.dev(1), (uint32_t*)st.dev(2)),
-            "lookup encrypt launch");
+  bool done = false;
+  if (pairs) {
+    cuhe::LookupDigits dg{};
+    dg.plain = (const uint32_t*)st.dev(0);
+    dg.plain_words = ctx->K;
+    dg.chunk_num = 1;
+    if (int rc = pair_lookup_encrypt(ctx, pl, dg, count, (const uint8_t*)st.dev(1), (uint32_t*)st.dev(2), &done))
+      return rc;
+  }
+  if (!done) {
+    if (int rc = ensure_wide_table(ctx, d, count)) return rc;
+    CUHE_CUDA(ctx, d.lookup(ctx, nullptr, 0, 0, 1, (const uint32_t*)st.dev(0), count, (const uint8_t*)st.dev(1),
+                            (uint32_t*)st.dev(2)),
+              "lookup encrypt launch");
+  }
   if (int rc = st.finish()) return rc;
   return check_status(ctx, st.staged());
 }

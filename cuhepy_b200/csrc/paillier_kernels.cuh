@@ -1008,8 +1008,7 @@ k_pair_modexp_tasks(const ModexpTask* __restrict__ tasks, int ntasks, long long 
 // shuffling, so each output costs one product: mont52(index, query R52) =
 // index * query mod n^2, canonical, as k_mulmod_outer's.
 // ---------------------------------------------------------------------------
-// row: R52 R mod n^2 for plain inputs, R52 mod n^2 for inputs already in
-// the 32-bit Montgomery form (x R): either way out = x R52 mod n^2.
+// row: R52 R mod n^2; out = x R52 mod n^2.
 template <int K>
 __global__ void __launch_bounds__(kBlockThreads)
 k_to_mont52(const uint32_t* __restrict__ in, long long count, double* __restrict__ out,
@@ -1571,121 +1570,296 @@ k_wide_table(const uint32_t* __restrict__ gtab, int message_chunks, uint32_t* __
   g.store(wide + inst * K, r);
 }
 
-// The 16-bit-digit table in 52-bit limbs, R52 domain, one row j at a time:
-// W[j][D] = G[2j][D mod 256] G[2j+1][D / 256] R52 mod n^2 from the 8-bit
-// table (32-bit Montgomery form): one 32-bit product for the pair, one with
-// R52 mod n^2 (r52w) into the R52 domain.
-template <int K>
-__global__ void __launch_bounds__(kBlockThreads)
-k_wide_table52(const uint32_t* __restrict__ gtab, int message_chunks, int j, double* __restrict__ wide52,
-               const uint32_t* __restrict__ consts, KeyScalars ks, const uint32_t* __restrict__ r52w) {
-  constexpr int TPI = K / 16, L = 16, K52 = 5 * K / 8, L52 = K52 / TPI;
-  constexpr int IPB = kBlockThreads / TPI;
-  extern __shared__ __align__(16) uint32_t smem[];
-  uint32_t* s_r52 = smem;
-  for (int i = threadIdx.x; i < K; i += blockDim.x) s_r52[i] = r52w[i];
-  __syncthreads();
-  Group<K, TPI> g;
-  const int slot = threadIdx.x / TPI;
-  const int D = blockIdx.x * IPB + slot;
-  if (D >= 65536) return;
-  uint32_t* s_b = smem + K + slot * K;
-  uint32_t n2[L], lo[L], hi[L], p[L];
-  g.load_ro(n2, consts + C_N2 * K);
-  g.load_ro(lo, gtab + ((long long)(2 * j) * 256 + (D & 255)) * K);
-  if (2 * j + 1 < message_chunks) g.load_ro(hi, gtab + ((long long)(2 * j + 1) * 256 + (D >> 8)) * K);
-  else g.load_ro(hi, consts + C_RM * K);
-  g.publish(s_b, hi);
-  g.mont_mul(p, lo, s_b, n2, ks.ninv2);      // the pair, 32-bit Montgomery form
-  g.mont_mul(lo, p, s_r52, n2, ks.ninv2);    // x R52 mod n^2
-  g.publish(s_b, lo);
-  double* o = wide52 + ((long long)j * 65536 + D) * K52;
-#pragma unroll
-  for (int k = 0; k < L52; ++k) o[g.gl * L52 + k] = cuhe52::to_f64(limb52_from_words(s_b, K, g.gl * L52 + k));
+// ---------------------------------------------------------------------------
+// Paillier-Lookup encryption on pairs of residues mod n (pair52.cuh): tables
+// and noise entries are rows of KL limb pairs in the R domain, a product is
+// five n-wide limb products, and the ciphertext leaves as in k_pair_modexp.
+//
+// Digits.  Plaintext words are read as 8-bit digits (or 16-bit, with the wide
+// table).  A binary embedding sets every second plaintext bit only, so the
+// table of its digits is indexed by embedding bits: 8 of them (16 plaintext
+// bits) by 256 rows, or 16 (32 plaintext bits) by 65,536, which halves the
+// rows per ciphertext again and the wide table with them.  Noise entries
+// come one by one or, for large calls, two at a time from a table of all
+// their products.  At key_len 1024 an embedding of 512 bits takes 64 + 14,
+// or wide 32 + 7, products instead of 120 + 14 and 64 + 14.
+// ---------------------------------------------------------------------------
+
+// A row's limb pairs stand in the order of the ten-limb kernels' loads: limb
+// 10 g + k at k (KL / 10) + g, so that a group's lanes read neighbours.
+template <int KL, int kL>
+__device__ __forceinline__ int pair_row_slot(int gl, int k) {
+  constexpr int T = KL / 10;
+  if (kL == 10) return k * T + gl;
+  return ((gl & 1) * 5 + k) * T + (gl >> 1);
 }
 
-// Paillier-Lookup encryption with the 16-bit-digit table on the FP64 pipe
-// (n^2 of 4096 / 8192 bits): the table and the noise entries as 52-bit limbs
-// in the R52 domain, the product accumulated as in k_modexp52 (the next row
-// loaded during each product), the result re-cut into words: the
-// ciphertexts of k_lookup_encrypt.
+// out[i] = in[i] as a row: in = K words in the 32-bit Montgomery form x 2^(32K)
+// mod n^2, entry = R^(j+2) 2^(-32K) mod n^2 as pairs for the two chunks.
 template <int K>
-__global__ void __launch_bounds__(kBlockThreads, 3)
-k_lookup_encrypt52(const uint8_t* __restrict__ bits, int embed_len, int chunk_len, int chunk_num,
-                   const uint32_t* __restrict__ plain, int plain_words, long long count, int message_chunks,
-                   const double* __restrict__ wide52, const double* __restrict__ noise52, int noise_entries,
-                   const uint8_t* __restrict__ noise_idx, uint32_t* __restrict__ out,
-                   const double* __restrict__ n52, unsigned long long ninv52, int* status) {
-  constexpr int TPI = K / 16, L = 16, K52 = 5 * K / 8, L52 = K52 / TPI;
-  constexpr int IPB = kBlockThreads / TPI;
-  extern __shared__ __align__(16) double smd[];
-  double* s_one52 = smd;         // 1
-  double* s_accs = smd + K52;    // per instance: the accumulator (b operand), K52 + 2 doubles
-  __shared__ int s_count[IPB];
-  for (int i = threadIdx.x; i < K52; i += blockDim.x) s_one52[i] = i == 0 ? 1.0 : 0.0;
+__global__ void __launch_bounds__(cuhe52::kPairThreads, 2)
+k_pair_rows(const uint32_t* __restrict__ in, long long count, double2* __restrict__ out,
+            const double2* __restrict__ entry, const double* __restrict__ n52, unsigned long long ninv52) {
+  constexpr int KL = 5 * K / 16, TPI = KL / 10, L = 10;
+  extern __shared__ __align__(16) uint32_t smem[];
+  double2* s_rows = reinterpret_cast<double2*>(smem);
+  for (int i = threadIdx.x; i < 2 * KL + 1; i += blockDim.x) s_rows[i] = i < 2 * KL ? entry[i] : make_double2(0.0, 0.0);
   __syncthreads();
-  Group<K, TPI> g;
-  cuhe52::Group52<K52, TPI> f;
-  const int slot = threadIdx.x / TPI;
-  const long long inst = (long long)blockIdx.x * IPB + slot;
-  if (inst >= count) return;
-  uint16_t* s_rows16 =
-      reinterpret_cast<uint16_t*>(s_accs + IPB * (K52 + 2)) + slot * lookup_rows_stride(message_chunks);
-  const uint32_t* s_rows32 = reinterpret_cast<const uint32_t*>(s_rows16);
-  if (g.gl == 0)
-    s_count[slot] = lookup_digit_rows<true>(bits, embed_len, chunk_len, chunk_num, plain, plain_words, inst,
-                                            message_chunks, s_rows16);
-  __syncwarp(f.mask);
-  const int cnt = s_count[slot];
-  double* s_b = s_accs + slot * (K52 + 2);
-  double acc[L52], a[L52], nx[L52], m52[L52];
-  auto load_row = [&](double (&v)[L52], const double* row) {
-    const double2* r2 = reinterpret_cast<const double2*>(row + f.gl * L52);
+  cuhe52::Pair52<KL, TPI> f;
+  const long long item = (long long)blockIdx.x * (cuhe52::kPairThreads / TPI) + threadIdx.x / TPI;
+  const long long inst = min(item, count - 1);
+  const uint64_t ninv = f.gl == 0 ? ninv52 : 0ull;
+  double m[L], a[L], r[L];
+  uint64_t A0[L], A1[L], S0[L], S1[L];
 #pragma unroll
-    for (int k = 0; k < L52 / 2; ++k) {
-      const double2 t = __ldg(r2 + k);
-      v[2 * k] = t.x;
-      v[2 * k + 1] = t.y;
+  for (int k = 0; k < L; ++k) m[k] = __ldg(n52 + f.gl * L + k);
+#pragma unroll 1
+  for (int j = 0; j < 2; ++j) {
+#pragma unroll
+    for (int k = 0; k < L; ++k) a[k] = f.to_f64(limb52_from_words(in + inst * K, K, j * KL + f.gl * L + k));
+    f.template product<false>(A0, A1, a, a, s_rows + j * KL, m, ninv);
+    f.template columns<2>(A0);
+    f.template columns<2>(A1);
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+      S0[k] = j ? S0[k] + A0[k] : A0[k];
+      S1[k] = j ? S1[k] + A1[k] : A1[k];
     }
-  };
-#pragma unroll
-  for (int k = 0; k < L52; ++k) {
-    m52[k] = __ldg(n52 + f.gl * L52 + k);
-    acc[k] = __ldg(n52 + K52 + f.gl * L52 + k);  // R52 mod n^2: one in the R52 domain
   }
-  f.publish(s_b, acc);
-  if (cnt > 0) load_row(a, wide52 + (long long)s_rows32[0] * K52);
-#pragma unroll 1
-  for (int j = 0; j < cnt; ++j) {
-    if (j + 1 < cnt) load_row(nx, wide52 + (long long)s_rows32[j + 1] * K52);
-    f.mont_mul(acc, a, s_b, m52, ninv52);
-    f.publish(s_b, acc);
+  f.from_columns(a, S0);
+  f.from_columns(r, S1);
+  if (item >= count) return;
 #pragma unroll
-    for (int k = 0; k < L52; ++k) a[k] = nx[k];
+  for (int k = 0; k < L; ++k) out[item * KL + pair_row_slot<KL, L>(f.gl, k)] = make_double2(a[k], r[k]);
+}
+
+// Table of products of two rows of one source: entry i = x y, with
+//   kEmbed  row j = i / 256 of 8 embedding bits b: digits 2j and 2j + 1 of the
+//           8-bit table at the bits of b spread to the even places
+//   kWide   row j = i / 65536 of 16 bits D: rows 2j and 2j + 1 at D's bytes
+//   kNoise  i = a entries + b: noise entries a and b
+// A factor past the source's last row is one.
+enum PairProducts : int { kEmbed = 0, kWide = 1, kNoise = 2 };
+
+__device__ __forceinline__ int spread4(int b) { return (b & 1) | (b & 2) << 1 | (b & 4) << 2 | (b & 8) << 3; }
+
+template <int K>
+__global__ void __launch_bounds__(cuhe52::kPairThreads, 2)
+k_pair_products(const double2* __restrict__ src, int rows, int kind, long long first, long long count,
+                double2* __restrict__ out, const double* __restrict__ n52, unsigned long long ninv52) {
+  constexpr int KL = 5 * K / 16, TPI = KL / 10, L = 10, kSlot = KL + 1;
+  extern __shared__ __align__(16) uint32_t smem[];
+  double2* s = reinterpret_cast<double2*>(smem) + (threadIdx.x / TPI) * kSlot;
+  cuhe52::Pair52<KL, TPI> f;
+  const long long item = first + (long long)blockIdx.x * (cuhe52::kPairThreads / TPI) + threadIdx.x / TPI;
+  const long long i = min(item, first + count - 1);
+  long long ia, ib;
+  if (kind == kNoise) {
+    ia = i / rows;
+    ib = i % rows;
+  } else {
+    const int bits = kind == kWide ? 16 : 8;
+    const int j = int(i >> bits), d = int(i & ((1 << bits) - 1));
+    const int lo = kind == kWide ? d & 255 : spread4(d & 15), hi = kind == kWide ? d >> 8 : spread4(d >> 4);
+    ia = (2ll * j) * 256 + lo;
+    ib = 2 * j + 1 < rows ? (2ll * j + 1) * 256 + hi : -1;
   }
-  const uint8_t* idx = noise_idx + inst * kNoiseMultiples;
+  // R mod n^2 stands in limb order, rows in their own
+  const double2* one = reinterpret_cast<const double2*>(n52 + KL) + 4 * KL;
+  double m[L], a0[L], a1[L], y0[L], y1[L];
+  uint64_t A0[L], A1[L];
+#pragma unroll
+  for (int k = 0; k < L; ++k) {
+    m[k] = __ldg(n52 + f.gl * L + k);
+    const int slot = pair_row_slot<KL, L>(f.gl, k);
+    const double2 x = __ldg(src + ia * KL + slot);
+    const double2 y = ib >= 0 ? __ldg(src + ib * KL + slot) : __ldg(one + f.gl * L + k);
+    a0[k] = x.x;
+    a1[k] = x.y;
+    y0[k] = y.x;
+    y1[k] = y.y;
+  }
+  pair_publish<KL, TPI>(f, s, y0, y1);
+  f.template product<true>(A0, A1, a0, a1, s, m, f.gl == 0 ? ninv52 : 0ull);
+  f.template limbs<2>(a0, A0);
+  f.template limbs<3>(a1, A1);
+  if (item >= first + count) return;
+#pragma unroll
+  for (int k = 0; k < L; ++k) out[item * KL + pair_row_slot<KL, L>(f.gl, k)] = make_double2(a0[k], a1[k]);
+}
+
+// How a ciphertext's rows are found.
+struct LookupDigits {
+  const uint8_t* bits;    // embeddings, or null for plaintext words
+  const uint32_t* plain;
+  int embed_len, chunk_len, chunk_num, plain_words;
+  int embed_bits;         // 8 or 16: digits of embedding bits; 0: of plaintext bits
+  int wide;               // 16-bit digits
+  int rows;               // rows of the table
+  int message_chunks;     // 8-bit plaintext digits the tables cover
+};
+
+__device__ __forceinline__ int lookup_digit(const LookupDigits& d, long long inst, int r) {
+  int v = 0;
+  if (d.bits) {
+    const long long vec = inst / d.chunk_num;
+    const int cbase = int(inst % d.chunk_num) * d.chunk_len;
+    const int avail = min(max(2 * d.embed_len - cbase, 0), d.chunk_len);
+    const uint8_t* vb = d.bits + vec * d.embed_len;
+    if (d.embed_bits) {  // chunk_len is even: plaintext bit 2 i is embedding bit last - i
+      const int last = (cbase + avail) / 2 - 1, n = d.embed_bits;
 #pragma unroll 1
-  for (int k = 0; k < kNoiseMultiples; ++k) {
-    const int r = idx[k];
-    if (r >= noise_entries) {
+      for (int b = 0; b < n; ++b) {
+        const int i = r * n + b;
+        if (2 * i < avail) v |= (vb[last - i] & 1) << b;
+      }
+      return v;
+    }
+    const int n = d.wide ? 16 : 8;
+#pragma unroll 1
+    for (int b = 0; b < n; ++b) {
+      const int e = n * r + b;  // exponent within the chunk value
+      if (e >= avail || e >= 8 * d.message_chunks) break;
+      const int p = cbase + (avail - 1 - e);  // padded MSB-first position
+      if (p & 1) v |= (vb[p >> 1] & 1) << b;
+    }
+    return v;
+  }
+  const uint8_t* mb = reinterpret_cast<const uint8_t*>(d.plain + inst * d.plain_words);
+  const int bytes = min(d.plain_words * 4, d.message_chunks);
+  if (!d.wide) return r < bytes ? int(mb[r]) : 0;
+  if (2 * r < bytes) v = mb[2 * r];
+  if (2 * r + 1 < bytes) v |= int(mb[2 * r + 1]) << 8;
+  return v;
+}
+
+template <int K, int kL>
+struct LookupLayout {
+  static constexpr int KL = 5 * K / 16, TPI = KL / kL;
+  static constexpr int kGroups = cuhe52::kPairThreads / TPI, kSlot = KL + 1;
+  static size_t bytes(int rows) {  // (1, 0), the values, n R in words, the digits
+    return size_t(kSlot + kGroups * kSlot) * 16 + size_t(K) * 4 + size_t(kGroups) * ((rows + 1) & ~1) * 2;
+  }
+};
+
+template <int K, int kL>
+__global__ void __launch_bounds__(cuhe52::kPairThreads, 2)
+k_pair_lookup(LookupDigits dg, long long count, const double2* __restrict__ table, const double2* __restrict__ noise,
+              int noise_entries, int noise_pairs, const uint8_t* __restrict__ noise_idx, uint32_t* __restrict__ out,
+              const uint32_t* __restrict__ consts, KeyScalars ks, const double* __restrict__ n52,
+              unsigned long long ninv52, int* status) {
+  using Lay = LookupLayout<K, kL>;
+  constexpr int KL = Lay::KL, TPI = Lay::TPI, L = kL, IPB = Lay::kGroups;
+  extern __shared__ __align__(16) uint32_t smem[];
+  double2* s_unit = reinterpret_cast<double2*>(smem);
+  double2* s_vals = s_unit + Lay::kSlot;
+  uint32_t* s_nr = reinterpret_cast<uint32_t*>(s_vals + IPB * Lay::kSlot);
+  uint16_t* s_digits = reinterpret_cast<uint16_t*>(s_nr + K);
+  for (int i = threadIdx.x; i < Lay::kSlot; i += blockDim.x) s_unit[i] = make_double2(i == 0 ? 1.0 : 0.0, 0.0);
+  for (int i = threadIdx.x; i < K; i += blockDim.x) s_nr[i] = consts[C_NR * K + i];
+  __syncthreads();
+  const long long first = (long long)blockIdx.x * IPB;
+  bool valid = true;
+  {
+    cuhe52::Pair52<KL, TPI> f;
+    const int group = threadIdx.x / TPI;
+    const long long inst = min(first + group, count - 1);  // idle groups repeat the last item
+    double2* s = s_vals + group * Lay::kSlot;
+    uint16_t* digits = s_digits + group * ((dg.rows + 1) & ~1);
+    for (int r = f.gl; r < dg.rows; r += TPI) digits[r] = uint16_t(lookup_digit(dg, inst, r));
+    __syncwarp();
+    const uint8_t* idx = noise_idx + inst * kNoiseMultiples;
+    for (int k = 0; k < kNoiseMultiples; ++k) valid = valid && idx[k] < noise_entries;
+    const int digit_bits = dg.embed_bits == 16 || dg.wide ? 16 : 8;
+    const int noises = noise_pairs ? kNoiseMultiples / 2 : kNoiseMultiples;
+    double m[L], a0[L], a1[L], z0[L], z1[L];
+    uint64_t A0[L], A1[L];
+#pragma unroll
+    for (int k = 0; k < L; ++k) m[k] = __ldg(n52 + f.gl * L + k);
+    const uint64_t ninv = f.gl == 0 ? ninv52 : 0ull;
+    // the rows in order: digits that are not zero for every group of the
+    // warp (a zero digit's row is one), then the noise
+    auto next = [&](int t) {
+      while (t < dg.rows && !__any_sync(0xffffffffu, digits[t] != 0)) ++t;
+      return t;
+    };
+    auto row = [&](int t) -> const double2* {
+      if (t < dg.rows) return table + ((static_cast<long long>(t) << digit_bits) + digits[t]) * KL;
+      const int k = t - dg.rows;
+      if (!valid) return noise;
+      if (noise_pairs) return noise + (static_cast<long long>(idx[2 * k]) * noise_entries + idx[2 * k + 1]) * KL;
+      return noise + static_cast<long long>(idx[k]) * KL;
+    };
+    int t = next(0);
+    const int end = dg.rows + noises;
+    bool begun = false;
+#pragma unroll 1
+    while (true) {
+      const bool out_now = t >= end;
+      if (!out_now) {
+        const double2* r = row(t);
+#pragma unroll
+        for (int k = 0; k < L; ++k) {
+          const double2 v = __ldg(r + pair_row_slot<KL, L>(f.gl, k));
+          a0[k] = v.x;
+          a1[k] = v.y;
+        }
+        t = t < dg.rows ? next(t + 1) : t + 1;
+        if (t < end) {  // bring the next row closer while this product runs
+          const double2* ahead = row(t);
+          for (int k = f.gl; k * 8 < KL; k += TPI) asm volatile("prefetch.global.L1 [%0];" ::"l"(ahead + k * 8));
+        }
+        if (!begun) {  // the first row is the value
+          begun = true;
+#pragma unroll
+          for (int k = 0; k < L; ++k) {
+            z0[k] = a0[k];
+            z1[k] = a1[k];
+          }
+          continue;
+        }
+        pair_publish<KL, TPI>(f, s, z0, z1);
+      } else {
+#pragma unroll
+        for (int k = 0; k < L; ++k) {
+          a0[k] = z0[k];
+          a1[k] = z1[k];
+        }
+      }
+      f.template product<true>(A0, A1, a0, a1, out_now ? s_unit : s, m, ninv);
+      if (out_now) break;
+      f.template limbs<2>(z0, A0);
+      f.template limbs<3>(z1, A1);
+    }
+    f.template columns<2>(A0);
+    f.template columns<3>(A1);
+    f.canonical(A0);
+    f.canonical(A1);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < L; ++k)
+      s[f.gl * L + k] = make_double2(__longlong_as_double(static_cast<long long>(A0[k])),
+                                     __longlong_as_double(static_cast<long long>(A1[k])));
+    // the validity of a group's noise indexes, for the lanes that store it
+    if (f.gl == 0) s[KL].x = valid ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  constexpr int LT = K / 16, LW = 16, PER = cuhe52::kPairThreads / LT;
+  Group<K, LT> g;
+  uint32_t n2[LW], x[LW];
+  g.load_ro(n2, consts + C_N2 * K);
+#pragma unroll 1
+  for (int item = threadIdx.x / LT; item < IPB; item += PER) {
+    const long long inst = first + item;
+    if (inst >= count) break;
+    const double2* s = s_vals + item * Lay::kSlot;
+    if (s[KL].x == 0.0) {
       if (g.gl == 0) atomicOr(status, ST_RANGE);
-      return;
+      continue;
     }
-    load_row(a, noise52 + (long long)r * K52);
-    f.mont_mul(acc, a, s_b, m52, ninv52);
-    f.publish(s_b, acc);
+    pair_words<KL, K, LT>(g, x, s, s_nr, n2, ks.ninv2);
+    g.store(out + inst * K, x);
   }
-  double res[L52];
-  f.mont_mul(res, acc, s_one52, m52, ninv52);  // canonical
-  uint64_t* s_l = reinterpret_cast<uint64_t*>(s_b);
-  __syncwarp(f.mask);
-#pragma unroll
-  for (int k = 0; k < L52; ++k) s_l[f.gl * L52 + k] = cuhe52::to_u64(res[k]);
-  __syncwarp(f.mask);
-  uint32_t w[L];
-#pragma unroll
-  for (int t = 0; t < L; ++t) w[t] = word_from_limbs52(s_l, K52, g.gl * L + t);
-  g.store(out + inst * K, w);
 }
 
 // ---------------------------------------------------------------------------

@@ -77,3 +77,68 @@ def test_halved_exponent_with_factors_that_are_not_prime(bits):
         assert ctx.decrypt(values) == [_decrypt(c, e, mult, n) for c in values], e.bit_length()
         units = [1 + n * rng.randrange(n) for _ in range(20)]  # 1 mod p and q: the shortcut holds
         assert ctx.decrypt(units) == [_decrypt(c, e, mult, n) for c in units]
+
+
+@pytest.mark.parametrize("chunk_len,embed", [(1024, 700), (1024, 1), (96, 200), (33, 31)])
+def test_lookup_digits_of_embeddings_and_words(chunk_len, embed):
+    """Embedding digits (even chunk lengths: 8 and 16 bits of the embedding a
+    row, part rows, chunks past the table's digits) and plain digits (odd chunk
+    lengths, sparse words) against the integer kernel's 8-bit digits."""
+    from cuhepy_b200.paillier.gpu import PaillierDevice
+
+    rng = random.Random(chunk_len)
+    n = _odd(rng, 1000)
+    ctx = PaillierDevice(n)
+    message_chunks = 125 if chunk_len == 1024 else 7
+    ctx.build_tables(n + 1 + rng.randrange(n * n - n - 2), message_chunks, [rng.randrange(n * n) for _ in range(19)])
+    gen = np.random.default_rng(chunk_len)
+    chunk_num = -(-2 * embed // chunk_len)
+    count = 70
+    bits = gen.integers(0, 2, size=(count, embed), dtype=np.uint8)
+    bits[0], bits[1], bits[2, : embed // 2] = 0, 1, 0
+    noise = gen.integers(0, 19, size=(count * chunk_num, 14), dtype=np.uint8)
+    words = [0, 1, 1 << (8 * message_chunks - 1), 255 << 8] + [rng.getrandbits(8 * message_chunks) % n for _ in range(40)]
+    idx = gen.integers(0, 19, size=(len(words), 14), dtype=np.uint8)
+    results = []
+    for fp64, wide in ((0, 0), (1, 0), (1, 2)):
+        ctx.set_fp64(fp64)
+        ctx.set_wide_table(wide)
+        results.append((ctx.lookup_encrypt_bits(bits, chunk_len, chunk_num, noise), ctx.lookup_encrypt_ints(words, idx)))
+    assert results[0] == results[1]
+    assert results[0] == results[2]
+
+
+def test_lookup_encrypt_large_call_and_capture():
+    """A call large enough for the table of noise products equals small calls;
+    a call captured in a graph before any table was made for its pipe uses
+    what is there."""
+    import torch
+
+    from cuhepy_b200.paillier.gpu import PaillierDevice
+
+    rng = random.Random(5)
+    n = _odd(rng, 1023)
+    ctx = PaillierDevice(n)
+    ctx.build_tables(n + 2, 16, [rng.randrange(n * n) for _ in range(256)])
+    gen = np.random.default_rng(5)
+    count, embed = 8192 + 3, 60
+    bits = torch.from_numpy(gen.integers(0, 2, size=(count, embed), dtype=np.uint8)).cuda()
+    noise = torch.from_numpy(gen.integers(0, 256, size=(count, 14), dtype=np.uint8)).cuda()
+    large = torch.zeros((count, ctx.words), dtype=torch.int32, device="cuda")
+    small = torch.zeros_like(large)
+    part = torch.zeros_like(large)
+    torch.cuda.synchronize()
+    for lo in range(0, count, 4096):
+        rows = min(4096, count - lo)
+        ctx.lookup_encrypt_bits_array(bits[lo:lo + rows], rows, embed, 1024, 1, noise[lo:lo + rows], small[lo:lo + rows])
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="global"):
+        ctx.lookup_encrypt_bits_array(bits, count, embed, 1024, 1, noise, part)
+    graph.replay()
+    torch.cuda.synchronize()
+    ctx.set_stream(None)
+    ctx.lookup_encrypt_bits_array(bits, count, embed, 1024, 1, noise, large)
+    ctx.synchronize()
+    assert torch.equal(large, small) and torch.equal(part, small)
