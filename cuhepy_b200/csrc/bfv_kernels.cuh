@@ -1118,6 +1118,355 @@ k_keyswitch_tm(const SwitchOp* __restrict__ ops, const RingDev* __restrict__ rin
   if (warp == 0) tmem_dealloc(s_tmem, kCols);
 }
 
+// ---- rotations of ciphertexts in the NTT domain ---------------------------------
+// A chain of rotations keeps its ciphertexts in the NTT domain, where the
+// automorphism X -> X^g is a permutation of the evaluation points and sums
+// are pointwise, and transforms only what the gadget digits need:
+//
+//   out = base + (sigma(x0), 0) + KS(sigma(x1))
+//
+// with base, x0, x1 and out in the NTT domain, the digits of sigma(x1) from
+// its composed words, and out_1's coefficients (for the next composition)
+// from one inverse transform.  Digit 0 needs no transform either: the digits
+// sum to sigma(x1) mod p, so
+//
+//   sum_d digit_d key_d = sigma(x1) key_0 + sum_{d >= 1} digit_d (key_d - 2^(bits d) key_0)
+//
+// (keys lifted once, k_lift_key).  A rotation with six digits takes five
+// forward transforms and one inverse per prime, where k_keyswitch_tm's
+// coefficient-domain switch takes six and two.
+struct RotateOp {
+  const u64* base;   // [2][L][N] NTT domain, or null
+  const u64* x0;     // [L][N] NTT domain, gathered through g, or null
+  const u64* x1;     // [L][N] NTT domain, gathered through g
+  const u64* words;  // composed sigma_g(x1): [N][W]
+  const u64* key;    // lifted key [D][2][L][N] NTT domain
+  const u64* key_q;  // its Shoup quotients
+  u64* out;          // [2][L][N] NTT domain; may be base, and x0, x1 then are its components
+  u64* coef;         // [L][N] coefficients of out_1, or null
+  const u64* mask;   // [L][N] NTT-domain plaintext that multiplies out, or null
+  unsigned g;
+  unsigned pad;
+};
+
+// the evaluation point that sigma_g moves to index i: index i of the
+// bit-reversed order holds the value at psi^(2 bitrev(i) + 1)
+__device__ __forceinline__ int sigma_index(int i, unsigned g, int logn) {
+  const unsigned e = 2u * (__brev(unsigned(i)) >> (32 - logn)) + 1u;
+  const unsigned ge = (g * e) & ((2u << logn) - 1u);
+  return int(__brev((ge - 1u) >> 1) >> (32 - logn));
+}
+
+// lifted[d] = key[d] - 2^(bits d) key[0] (d >= 1), planes [d][component][prime];
+// power[d * L + j] = 2^(bits d) mod p_j
+__global__ void k_lift_key(const u64* __restrict__ key, const u64* __restrict__ power, int digits, int L,
+                           u64* __restrict__ lifted, const RingDev* __restrict__ ring) {
+  const RingDev& R = *ring;
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long per = 2LL * L * R.n;
+  if (idx >= digits * per) return;
+  const int d = int(idx / per), j = int((idx / R.n) % L);
+  const Prime& m = R.prime[j];
+  lifted[idx] = d ? submod(key[idx], mulmod(key[idx % per], power[d * L + j], m), m.p) : key[idx];
+}
+
+// CTA per (op, prime), two per SM at N <= 8192, accumulators in tensor memory
+// as in k_keyswitch_tm (thread t's coefficients and columns as there, pairs
+// where log2 N = 1 mod MAXP).  Every read of base, x0 and x1 is in the first
+// pass over the coefficients, before the first barrier; out is written after
+// the last digit, so out may be base and hold x0 and x1.  At least two
+// digits.  Bound as k_keyswitch_tm: the integer multiplies of the transforms.
+template <int MAXP, int kCoef = 16>
+__global__ void __launch_bounds__(512, kCoef == 16 ? 2 : 1)
+k_rotate_tm(const RotateOp* __restrict__ ops, const RingDev* __restrict__ ring) {
+  constexpr int kThreads = 512, kChunks = kCoef / 4, kCols = 16 * kCoef;
+  extern __shared__ __align__(16) u64 s_plane[];
+  __shared__ uint32_t s_tmem;
+  const RingDev& R = *ring;
+  const RotateOp op = ops[blockIdx.x];
+  const int j = blockIdx.y;
+  const int n = R.n, L = R.residue, W = R.words, logn = R.logn;
+  const u64 p = R.prime[j].p, two_p = 2 * p;
+  const int warp = int(threadIdx.x >> 5);
+  if (warp == 0) {
+    tmem_alloc(&s_tmem, kCols);
+    tmem_relinquish();
+  }
+  tmem_fence_before_sync();
+  __syncthreads();
+  tmem_fence_after_sync();
+  const uint32_t tbase = s_tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t((warp >> 2) * 4 * kCoef);
+  const bool pairs = logn % MAXP == 1 && logn > 1;
+  // column group kk of chunk c holds coefficient coef(c, kk)
+  auto coef = [&](int c, int kk) {
+    return pairs ? 2 * (int(threadIdx.x) + (c * 2 + (kk >> 1)) * kThreads) + (kk & 1)
+                 : int(threadIdx.x) + (c * 4 + kk) * kThreads;
+  };
+  const ulonglong2* w2 = R.fwd2[j];
+  const int half_n = n >> 1;
+  const long long plane = (long long)j * n, comp = (long long)L * n;
+  // a sum starts below 2p and each digit adds less than 2p: up to seven
+  // digits are summed unreduced (below 16p)
+  const bool lazy_sum = R.digits <= 7;
+  // digit 0: sigma(x1) itself, with the addends
+#pragma unroll 1
+  for (int c = 0; c < kChunks; ++c) {
+    uint32_t acc[16];
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const int i = coef(c, kk);
+      u64 a0 = 0, a1 = 0;
+      if (i < n) {
+        const int from = sigma_index(i, op.g, logn);
+        const u64 v = op.x1[plane + from];
+        a0 = shoup_lazy(v, __ldg(op.key + plane + i), __ldg(op.key_q + plane + i), p);
+        a1 = shoup_lazy(v, __ldg(op.key + comp + plane + i), __ldg(op.key_q + comp + plane + i), p);
+        if (op.base) {
+          a0 += op.base[plane + i];
+          a1 += op.base[comp + plane + i];
+        }
+        if (op.x0) a0 += op.x0[plane + from];
+        if (!lazy_sum) {
+          a0 = a0 >= two_p ? a0 - two_p : a0;
+          a1 = a1 >= two_p ? a1 - two_p : a1;
+        }
+      }
+      acc[4 * kk] = uint32_t(a0);
+      acc[4 * kk + 1] = uint32_t(a0 >> 32);
+      acc[4 * kk + 2] = uint32_t(a1);
+      acc[4 * kk + 3] = uint32_t(a1 >> 32);
+    }
+    tmem_st16(tbase + uint32_t(c * 16), acc);
+  }
+  tmem_wait_st();
+  for (int d = 1; d < R.digits; ++d) {
+    const int start = d * R.digit_bits, limb = start / 64, off = start % 64;
+    if (R.digit_bits <= 63) {
+      // digits below 2^63 < 16p enter the lazy transform unreduced; the
+      // words of four coefficients are loaded before any is used
+      const u64 dmask = (u64(1) << R.digit_bits) - 1;
+      const bool two = off && off + R.digit_bits > 64 && limb + 1 < W;
+      for (int i0 = int(threadIdx.x); i0 < n; i0 += 4 * kThreads) {
+        u64 w0[4], w1[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * kThreads;
+          const u64* w = op.words + (long long)i * W;
+          w0[u] = i < n && limb < W ? w[limb] : 0;
+          w1[u] = i < n && two ? w[limb + 1] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * kThreads;
+          u64 v = w0[u] >> off;
+          if (two) v |= w1[u] << (64 - off);
+          if (i < n) s_plane[sp(i)] = v & dmask;
+        }
+      }
+    } else {
+      for (int i = threadIdx.x; i < n; i += kThreads)
+        s_plane[sp(i)] = gadget_digit(op.words + (long long)i * W, W, d, R, j);
+    }
+    __syncthreads();
+    // the digit transforms feed only the Shoup key products: no canonical pass
+    if (pairs) ntt_forward_stages(s_plane, R, j, MAXP, logn - 1);
+    else ntt_forward_fast(s_plane, R, j, MAXP, 0, false);
+    const long long k0o = (2LL * d) * comp + plane, k1o = k0o + comp;
+#pragma unroll 1
+    for (int c = 0; c < kChunks; ++c) {
+      uint32_t acc[16];
+      tmem_ld16(tbase + uint32_t(c * 16), acc);
+      if (pairs) {
+#pragma unroll
+        for (int kp = 0; kp < 2; ++kp) {
+          const int b = int(threadIdx.x) + (c * 2 + kp) * kThreads;
+          if (b < half_n) {
+            // the last forward stage: gap 1, twiddle (N/2 + b)
+            u64 u = s_plane[sp(2 * b)];
+            const u64 x1 = s_plane[sp(2 * b + 1)];
+            const ulonglong2 tw = __ldg(w2 + half_n + b);
+            if (u >= 8 * p) u -= 8 * p;
+            const u64 v = shoup_lazy(x1, tw.x, tw.y, p);
+            const u64 y[2] = {u + v, u + two_p - v};
+#pragma unroll
+            for (int comp_i = 0; comp_i < 2; ++comp_i) {
+              const long long ko = comp_i ? k1o : k0o;
+              const ulonglong2 kv = __ldg(reinterpret_cast<const ulonglong2*>(op.key + ko) + b);
+              const ulonglong2 kq = __ldg(reinterpret_cast<const ulonglong2*>(op.key_q + ko) + b);
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const int col = 4 * (2 * kp + e) + 2 * comp_i;
+                u64 a = shoup_lazy(y[e], e ? kv.y : kv.x, e ? kq.y : kq.x, p);
+                a += u64(acc[col]) | (u64(acc[col + 1]) << 32);
+                if (!lazy_sum) a = a >= two_p ? a - two_p : a;
+                acc[col] = uint32_t(a);
+                acc[col + 1] = uint32_t(a >> 32);
+              }
+            }
+          }
+        }
+      } else {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const int i = coef(c, kk);
+          if (i < n) {
+            const u64 v = s_plane[sp(i)];
+            u64 a0 = shoup_lazy(v, __ldg(op.key + k0o + i), __ldg(op.key_q + k0o + i), p);
+            u64 a1 = shoup_lazy(v, __ldg(op.key + k1o + i), __ldg(op.key_q + k1o + i), p);
+            a0 += u64(acc[4 * kk]) | (u64(acc[4 * kk + 1]) << 32);
+            a1 += u64(acc[4 * kk + 2]) | (u64(acc[4 * kk + 3]) << 32);
+            if (!lazy_sum) {
+              a0 = a0 >= two_p ? a0 - two_p : a0;
+              a1 = a1 >= two_p ? a1 - two_p : a1;
+            }
+            acc[4 * kk] = uint32_t(a0);
+            acc[4 * kk + 1] = uint32_t(a0 >> 32);
+            acc[4 * kk + 2] = uint32_t(a1);
+            acc[4 * kk + 3] = uint32_t(a1 >> 32);
+          }
+        }
+      }
+      tmem_st16(tbase + uint32_t(c * 16), acc);
+    }
+    tmem_wait_st();
+    if (d + 1 < R.digits) __syncthreads();  // the next digit overwrites the plane
+  }
+  // the sums reduced, masked and written; out_1 also into the plane (each
+  // thread's own coefficients, whose last reader it was) for its inverse
+#pragma unroll 1
+  for (int c = 0; c < kChunks; ++c) {
+    uint32_t acc[16];
+    tmem_ld16(tbase + uint32_t(c * 16), acc);
+    u64 r1[4];
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const int i = coef(c, kk);
+      r1[kk] = 0;
+      if (i < n) {
+        u64 a0 = u64(acc[4 * kk]) | (u64(acc[4 * kk + 1]) << 32);
+        u64 a1 = u64(acc[4 * kk + 2]) | (u64(acc[4 * kk + 3]) << 32);
+        a0 = reduce_below_16p(a0, p);
+        a1 = reduce_below_16p(a1, p);
+        if (op.mask) {
+          const u64 m = op.mask[plane + i];
+          a0 = reduce128(u128(a0) * m, R.prime[j]);
+          a1 = reduce128(u128(a1) * m, R.prime[j]);
+        }
+        op.out[plane + i] = a0;
+        op.out[comp + plane + i] = a1;
+        r1[kk] = a1;
+      }
+    }
+    if (op.coef) {
+      if (pairs) {
+#pragma unroll
+        for (int kp = 0; kp < 2; ++kp) {
+          const int b = int(threadIdx.x) + (c * 2 + kp) * kThreads;
+          if (b < half_n) {
+            inverse_stage0(r1[2 * kp], r1[2 * kp + 1], R.inv2[j], half_n, b, p);
+            s_plane[sp(2 * b)] = r1[2 * kp];
+            s_plane[sp(2 * b + 1)] = r1[2 * kp + 1];
+          }
+        }
+      } else {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const int i = coef(c, kk);
+          if (i < n) s_plane[sp(i)] = r1[kk];
+        }
+      }
+    }
+  }
+  if (op.coef) {
+    __syncthreads();
+    if (pairs) ntt_inverse_from(s_plane, R, j, MAXP, 1);
+    else ntt_inverse_fast(s_plane, R, j, MAXP);
+    u64* o = op.coef + plane;
+    for (int i = threadIdx.x; i < n; i += kThreads) o[i] = s_plane[sp(i)];
+  }
+  tmem_fence_before_sync();
+  __syncthreads();
+  tmem_fence_after_sync();
+  if (warp == 0) tmem_dealloc(s_tmem, kCols);
+}
+
+// The same unfused, for few ops (one CTA per (op, prime) would leave most SMs
+// idle): digits 1 .. D - 1 as planes [op][prime][d - 1] and, behind them, the
+// gathered addends [op][prime][base_0 + sigma(x0), sigma(x1)] (gathered before
+// anything is written: out may be base and hold x0 and x1); then the digits'
+// transforms, this sum, and the inverse transforms of out_1 (k_inverse_ops).
+__global__ void k_rotate_digits(const RotateOp* __restrict__ ops, int count, int L, u64* __restrict__ digits,
+                                const RingDev* __restrict__ ring) {
+  const RingDev& R = *ring;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= R.n) return;
+  const int D = R.digits, d = blockIdx.y % D, pair = blockIdx.y / D;  // pair = op * L + j
+  const int j = pair % L;
+  const RotateOp& o = ops[pair / L];
+  if (d > 0) {
+    digits[((long long)pair * (D - 1) + d - 1) * R.n + i] =
+        gadget_digit(o.words + (long long)i * R.words, R.words, d, R, j);
+    return;
+  }
+  const u64 p = R.prime[j].p;
+  const int from = sigma_index(i, o.g, R.logn);
+  u64 v = o.base ? o.base[(long long)j * R.n + i] : 0;
+  if (o.x0) v = addmod(v, o.x0[(long long)j * R.n + from], p);
+  u64* g = digits + ((long long)count * L * (D - 1) + 2LL * pair) * R.n + i;
+  g[0] = v;
+  g[R.n] = o.x1[(long long)j * R.n + from];
+}
+
+// thread per (op, prime, coefficient)
+__global__ void k_rotate_mac(const RotateOp* __restrict__ ops, int count, int L, const u64* __restrict__ digits,
+                             const RingDev* __restrict__ ring) {
+  const RingDev& R = *ring;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= R.n) return;
+  const int D = R.digits, pair = blockIdx.y, j = pair % L;
+  const RotateOp o = ops[pair / L];
+  const u64 p = R.prime[j].p;
+  const long long comp = (long long)L * R.n, at = (long long)j * R.n + i;
+  const u64* g = digits + ((long long)count * L * (D - 1) + 2LL * pair) * R.n + i;
+  const u64 v = g[R.n];
+  u64 a0 = addmod(shoup(v, __ldg(o.key + at), __ldg(o.key_q + at), p), g[0], p);
+  u64 a1 = shoup(v, __ldg(o.key + comp + at), __ldg(o.key_q + comp + at), p);
+  if (o.base) a1 = addmod(a1, o.base[comp + at], p);
+  for (int d = 1; d < D; ++d) {
+    const u64 y = digits[((long long)pair * (D - 1) + d - 1) * R.n + i];
+    const long long ko = 2LL * d * comp + at;
+    a0 = addmod(a0, shoup(y, __ldg(o.key + ko), __ldg(o.key_q + ko), p), p);
+    a1 = addmod(a1, shoup(y, __ldg(o.key + ko + comp), __ldg(o.key_q + ko + comp), p), p);
+  }
+  if (o.mask) {
+    a0 = mulmod(a0, o.mask[at], R.prime[j]);
+    a1 = mulmod(a1, o.mask[at], R.prime[j]);
+  }
+  o.out[at] = a0;
+  o.out[comp + at] = a1;
+}
+
+// dst = inverse transform of src ([L][N] each; dst may be src), CTA per
+// (op, prime); ops without a destination are skipped
+struct InverseOp {
+  const u64* src;
+  u64* dst;
+};
+__global__ void __launch_bounds__(1024, 1)
+k_inverse_ops(const InverseOp* __restrict__ ops, const RingDev* __restrict__ ring) {
+  extern __shared__ __align__(16) u64 s_plane[];
+  const RingDev& R = *ring;
+  const InverseOp op = ops[blockIdx.x];
+  if (!op.dst) return;
+  const int j = blockIdx.y, n = R.n;
+  const u64* src = op.src + (long long)j * n;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s_plane[sp(i)] = src[i];
+  __syncthreads();
+  ntt_inverse_fast(s_plane, R, j, 3);
+  u64* dst = op.dst + (long long)j * n;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = s_plane[sp(i)];
+}
+
 // ---- unfused key switch (N = 32768) --------------------------------------------
 // digits[op][prime][d][N] = digit d of op's composed words, mod the prime
 __global__ void k_ks_digits(const SwitchOp* __restrict__ ops, int L, u64* __restrict__ digits,

@@ -229,11 +229,16 @@ struct cuhe_bfv_key {
   cuhe_bfv_ring* ring = nullptr;
   u64* d_key = nullptr;  // [D][2][L][N] NTT domain, then as many Shoup quotients
   u64* d_key_q = nullptr;
+  // the key lifted for NTT-domain rotations (k_lift_key) and its quotients
+  // (residue rings whose planes fit one CTA, two digits or more)
+  u64* d_lift = nullptr;
+  u64* d_lift_q = nullptr;
   size_t bytes = 0;
   ~cuhe_bfv_key() {
-    if (d_key) {
+    if (d_key || d_lift) {
       DeviceGuard g(ring->device);
       cudaFree(d_key);
+      cudaFree(d_lift);
     }
     cuhe_bfv_ring_release(ring);
   }
@@ -552,29 +557,35 @@ size_t small_switch_bytes(const cuhe_bfv_ring* r) {
   return slice(std::max<size_t>(1, kSmallSwitchPairs / L) * unfused_bytes_per_op(r));
 }
 
+int launch_compose(cuhe_bfv_ring* r, Lane& ln, RingDev* d, const ComposeOp* d_cops, size_t count) {
+  const auto& P = r->plan;
+  dim3 grid(blocks_for((long long)(P.n), 256), unsigned(count));
+  const int L = int(P.residue_count);
+  if (r->residue && r->host_dev.words == L) {
+    switch (L) {
+      case 1: k_compose<1><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
+      case 2: k_compose<2><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
+      case 3: k_compose<3><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
+      case 4: k_compose<4><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
+      case 5: k_compose<5><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
+      case 6: k_compose<6><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
+      case 7: k_compose<7><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
+      default: k_compose<8><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
+    }
+  } else {
+    k_compose<0><<<grid, 256, 0, ln.stream>>>(d_cops, d);
+  }
+  BFV_CUDA(cudaGetLastError(), "compose launch");
+  return CUHE_OK;
+}
+
 int run_switch(cuhe_bfv_ring* r, Lane& ln, RingDev* d, const std::vector<ComposeOp>& cops, const std::vector<SwitchOp>& sops,
                ComposeOp* d_cops, SwitchOp* d_sops, Arena* small = nullptr) {
   const auto& P = r->plan;
   if (!cops.empty()) {
     BFV_CUDA(cudaMemcpyAsync(d_cops, cops.data(), cops.size() * sizeof(ComposeOp), cudaMemcpyHostToDevice, ln.stream),
              "compose ops");
-    dim3 grid(blocks_for((long long)(P.n), 256), unsigned(cops.size()));
-    const int L = int(P.residue_count);
-    if (r->residue && r->host_dev.words == L) {
-      switch (L) {
-        case 1: k_compose<1><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
-        case 2: k_compose<2><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
-        case 3: k_compose<3><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
-        case 4: k_compose<4><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
-        case 5: k_compose<5><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
-        case 6: k_compose<6><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
-        case 7: k_compose<7><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
-        default: k_compose<8><<<grid, 256, 0, ln.stream>>>(d_cops, d); break;
-      }
-    } else {
-      k_compose<0><<<grid, 256, 0, ln.stream>>>(d_cops, d);
-    }
-    BFV_CUDA(cudaGetLastError(), "compose launch");
+    if (int rc = launch_compose(r, ln, d, d_cops, cops.size())) return rc;
   }
   if (!sops.empty()) {
     BFV_CUDA(cudaMemcpyAsync(d_sops, sops.data(), sops.size() * sizeof(SwitchOp), cudaMemcpyHostToDevice, ln.stream),
@@ -618,6 +629,96 @@ int run_switch(cuhe_bfv_ring* r, Lane& ln, RingDev* d, const std::vector<Compose
   }
   // op tables are reused by the next call; keep host order
   BFV_CUDA(cudaStreamSynchronize(ln.stream), "switch synchronize");
+  return CUHE_OK;
+}
+
+// Whether this ring's rotations run in the NTT domain (k_rotate_tm).
+bool ntt_rotations(const cuhe_bfv_ring* r) {
+  return r->residue && r->plan.n <= kMaxPlaneN && r->plan.n >= 2 && r->plan.digits >= 2;
+}
+
+// Rotations with their op tables: the host side collects every step of a
+// chain, uploads the tables once and launches step after step without
+// waiting.
+struct RotateStep {
+  size_t first = 0, count = 0;  // ops of the step
+  bool composed = false;        // their words are there already
+};
+
+size_t rotate_table_bytes(size_t ops) {
+  return slice(ops * sizeof(ComposeOp)) + slice(ops * sizeof(RotateOp)) + slice(ops * sizeof(InverseOp));
+}
+
+struct RotateChain {
+  std::vector<ComposeOp> cops;
+  std::vector<RotateOp> rops;
+  std::vector<RotateStep> steps;
+  void add(const ComposeOp& c, const RotateOp& o) {
+    cops.push_back(c);
+    rops.push_back(o);
+  }
+  void close(size_t first, bool composed = false) {
+    if (rops.size() > first) steps.push_back({first, rops.size() - first, composed});
+  }
+};
+
+// Device bytes of the unfused rotation's planes per op.
+size_t rotate_unfused_bytes(const cuhe_bfv_ring* r) {
+  return r->plan.residue_count * (r->plan.digits + 1) * r->plan.n * sizeof(u64);
+}
+
+// Runs the chain on ln's stream with op tables in ar; steps of at most
+// kSmallSwitchPairs (op, prime) pairs run unfused where ar has room for their
+// digit planes.
+int run_chain(cuhe_bfv_ring* r, Lane& ln, RingDev* d, const RotateChain& chain, Arena& ar) {
+  if (chain.rops.empty()) return CUHE_OK;
+  const auto& P = r->plan;
+  const size_t n = P.n, L = P.residue_count, ops = chain.rops.size();
+  ComposeOp* d_cops = ar.take<ComposeOp>(ops);
+  RotateOp* d_rops = ar.take<RotateOp>(ops);
+  InverseOp* d_iops = ar.take<InverseOp>(ops);
+  BFV_ARENA(ar);
+  std::vector<InverseOp> iops(ops);
+  for (size_t k = 0; k < ops; ++k) iops[k] = InverseOp{chain.rops[k].out + L * n, chain.rops[k].coef};
+  BFV_CUDA(cudaMemcpyAsync(d_cops, chain.cops.data(), ops * sizeof(ComposeOp), cudaMemcpyHostToDevice, ln.stream), "ops");
+  BFV_CUDA(cudaMemcpyAsync(d_rops, chain.rops.data(), ops * sizeof(RotateOp), cudaMemcpyHostToDevice, ln.stream), "ops");
+  BFV_CUDA(cudaMemcpyAsync(d_iops, iops.data(), ops * sizeof(InverseOp), cudaMemcpyHostToDevice, ln.stream), "ops");
+  const size_t smem = ntt_smem(r);
+  const size_t room = ar.cap - ar.used;
+  u64* digits = reinterpret_cast<u64*>(ar.base + ar.used);
+  for (const RotateStep& st : chain.steps) {
+    if (!st.composed)
+      if (int rc = launch_compose(r, ln, d, d_cops + st.first, st.count)) return rc;
+    const RotateOp* rop = d_rops + st.first;
+    if (st.count * L <= kSmallSwitchPairs && st.count * rotate_unfused_bytes(r) <= room) {
+      const unsigned bx = blocks_for((long long)n, 256), planes = unsigned(st.count * L * (P.digits - 1));
+      k_rotate_digits<<<dim3(bx, unsigned(st.count * L * P.digits)), 256, 0, ln.stream>>>(rop, int(st.count), int(L),
+                                                                                          digits, d);
+      BFV_CUDA(ntt_planes(n, ln.stream, d, digits, (long long)planes, 0, int(L), int(P.digits - 1), 0), "digit ntt");
+      k_rotate_mac<<<dim3(bx, unsigned(st.count * L)), 256, 0, ln.stream>>>(rop, int(st.count), int(L), digits, d);
+      bool any = false;
+      for (size_t k = 0; k < st.count; ++k) any = any || iops[st.first + k].dst;
+      if (any)
+        k_inverse_ops<<<dim3(unsigned(st.count), unsigned(L)), ntt_default_threads(n), smem, ln.stream>>>(
+            d_iops + st.first, d);
+    } else if (n <= 8192) {
+      k_rotate_tm<3><<<dim3(unsigned(st.count), unsigned(L)), 512, smem, ln.stream>>>(rop, d);
+    } else {
+      k_rotate_tm<3, 32><<<dim3(unsigned(st.count), unsigned(L)), 512, smem, ln.stream>>>(rop, d);
+    }
+    BFV_CUDA(cudaGetLastError(), "rotation launch");
+  }
+  return CUHE_OK;
+}
+
+// Coefficients of NTT-domain polynomials ([L][N] each), in place.
+int inverse_polys(cuhe_bfv_ring* r, Lane& ln, RingDev* d, const std::vector<InverseOp>& ops, Arena& ar) {
+  InverseOp* d_iops = ar.take<InverseOp>(ops.size());
+  BFV_ARENA(ar);
+  BFV_CUDA(cudaMemcpyAsync(d_iops, ops.data(), ops.size() * sizeof(InverseOp), cudaMemcpyHostToDevice, ln.stream), "ops");
+  k_inverse_ops<<<dim3(unsigned(ops.size()), unsigned(r->plan.residue_count)), ntt_default_threads(r->plan.n),
+                  ntt_smem(r), ln.stream>>>(d_iops, d);
+  BFV_CUDA(cudaGetLastError(), "inverse transforms");
   return CUHE_OK;
 }
 
@@ -708,6 +809,114 @@ struct TileArgs {
   std::vector<cuhe_bfv_key*> keys;
   std::vector<const u64*> masks;         // per tile mask NTT [L][N]
 };
+
+// Whether a tile circuit with these rotations leaves its distances in the
+// NTT domain (tile_circuit_ntt).
+bool ntt_circuit(const cuhe_bfv_ring* r, const std::vector<u64>& exps) {
+  if (!ntt_rotations(r) || exps.empty()) return false;
+  for (u64 g : exps)
+    if (g == 1) return false;
+  return true;
+}
+
+size_t tile_ntt_arena_bytes(const cuhe_bfv_ring* r, size_t ct, size_t rotations) {
+  const auto& P = r->plan;
+  const size_t n = P.n, L = P.residue_count, T = P.tensor_count, W = size_t(r->host_dev.words);
+  const size_t unfused = std::min(ct, kSmallSwitchPairs / L) * rotate_unfused_bytes(r);
+  return slice(ct * 2 * T * n * 8) + slice(ct * 3 * T * n * 8) + slice(ct * 3 * L * n * 8) + slice(ct * n * W * 8) +
+         slice(ct * sizeof(ComposeOp)) + rotate_table_bytes(ct) + rotate_table_bytes(ct * rotations) + slice(unfused);
+}
+
+// The tile circuit with its ciphertexts in the NTT domain from the
+// relinearisation on: dist receives [ct][2][L][N] NTT-domain residues, and
+// coef [ct][L][N] the coefficients of component 1 for the tiles with need
+// set (the right operands of the merges that follow).  Nothing waits on the
+// host between the steps.
+int tile_circuit_ntt(cuhe_bfv_ring* r, Lane& ln, RingDev* d, const TileArgs& a, u64* dist, u64* coef, const char* need,
+                     double* ms) {
+  const auto& P = r->plan;
+  const size_t n = P.n, L = P.residue_count, T = P.tensor_count, W = size_t(r->host_dev.words);
+  const size_t ct = a.ct;
+  Arena& ar = ln.arena;
+  u64* diff = ar.take<u64>(ct * 2 * T * n);
+  u64* tens = ar.take<u64>(ct * 3 * T * n);
+  u64* scaled = ar.take<u64>(ct * 3 * L * n);
+  u64* words = ar.take<u64>(ct * n * W);
+  BFV_ARENA(ar);
+  cudaEvent_t ev[4];
+  for (auto& e : ev) cudaEventCreate(&e);
+  cudaEventRecord(ev[0], ln.stream);
+  k_diff_residues<<<blocks_for((long long)(ct * 2 * n), 256), 256, 0, ln.stream>>>(a.q_words, a.t_words, int(ct), int(T),
+                                                                                    diff, d);
+  BFV_CUDA(cudaGetLastError(), "diff residues");
+  BFV_CUDA(launch_ntt(r, ln, d, diff, (long long)(ct * 2 * T), 0, int(T), 1, 0), "tensor ntt");
+  k_tensor_square<<<blocks_for((long long)(ct * T * n), 256), 256, 0, ln.stream>>>(diff, int(ct), int(T), tens, d);
+  BFV_CUDA(cudaGetLastError(), "tensor");
+  BFV_CUDA(launch_ntt(r, ln, d, tens, (long long)(ct * 3 * T), 0, int(T), 1, 1), "tensor intt");
+  k_rns_scale<<<blocks_for((long long)(ct * 3 * n), 128), 128, 0, ln.stream>>>(tens, (long long)(ct * 3), scaled, d);
+  BFV_CUDA(cudaGetLastError(), "rns scale");
+  cudaEventRecord(ev[1], ln.stream);
+  // relinearisation: the switch of p2 (composed from its coefficients, then
+  // all three polynomials transformed), dist = (p0, p1) + KS(p2)
+  {
+    RotateChain chain;
+    std::vector<ComposeOp> cops(ct);
+    ComposeOp* d_cops = ar.take<ComposeOp>(ct);
+    BFV_ARENA(ar);
+    for (size_t t = 0; t < ct; ++t) {
+      u64* st = scaled + t * 3 * L * n;
+      cops[t] = ComposeOp{st + 2 * L * n, words + t * n * W, 1u, 0u};
+      RotateOp o{};
+      o.base = st;
+      o.x1 = st + 2 * L * n;
+      o.words = words + t * n * W;
+      o.key = a.relin->d_lift;
+      o.key_q = a.relin->d_lift_q;
+      o.out = dist + t * 2 * L * n;
+      o.coef = coef + t * L * n;
+      o.g = 1;
+      chain.add(cops[t], o);
+    }
+    chain.close(0, true);
+    BFV_CUDA(cudaMemcpyAsync(d_cops, cops.data(), ct * sizeof(ComposeOp), cudaMemcpyHostToDevice, ln.stream), "ops");
+    if (int rc = launch_compose(r, ln, d, d_cops, ct)) return rc;
+    BFV_CUDA(launch_ntt(r, ln, d, scaled, (long long)(ct * 3 * L), 0, int(L), 1, 0), "scaled ntt");
+    if (int rc = run_chain(r, ln, d, chain, ar)) return rc;
+  }
+  cudaEventRecord(ev[2], ln.stream);
+  // rotations: dist += rotate(dist, g) in place, the last one masked
+  {
+    RotateChain chain;
+    for (size_t k = 0; k < a.exps.size(); ++k) {
+      const bool last = k + 1 == a.exps.size();
+      const size_t first = chain.rops.size();
+      for (size_t t = 0; t < ct; ++t) {
+        RotateOp o{};
+        o.base = o.x0 = o.out = dist + t * 2 * L * n;
+        o.x1 = o.base + L * n;
+        o.words = words + t * n * W;
+        o.key = a.keys[k]->d_lift;
+        o.key_q = a.keys[k]->d_lift_q;
+        o.coef = !last || need[t] ? coef + t * L * n : nullptr;
+        o.mask = last ? a.masks[t] : nullptr;
+        o.g = unsigned(a.exps[k]);
+        chain.add(ComposeOp{coef + t * L * n, words + t * n * W, o.g, 0u}, o);
+      }
+      chain.close(first);
+    }
+    if (int rc = run_chain(r, ln, d, chain, ar)) return rc;
+  }
+  cudaEventRecord(ev[3], ln.stream);
+  BFV_CUDA(cudaStreamSynchronize(ln.stream), "tile circuit");
+  if (ms) {
+    float x;
+    cudaEventElapsedTime(&x, ev[0], ev[1]); ms[0] += x;
+    cudaEventElapsedTime(&x, ev[1], ev[2]); ms[1] += x;
+    cudaEventElapsedTime(&x, ev[2], ev[3]); ms[2] += x;
+  }
+  for (auto& e : ev) cudaEventDestroy(e);
+  return CUHE_OK;
+}
 
 int tile_circuit(cuhe_bfv_ring* r, Lane& ln, RingDev* d, const TileArgs& a, u64* dist, double* ms) {
   const auto& P = r->plan;
@@ -1239,6 +1448,15 @@ int cuhe_bfv_create_ring(uint64_t n, const char* q_hex, uint64_t digit_bits, int
     e = cudaFuncSetAttribute(k_keyswitch_tm<3, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              int(plane_smem_words(16384) * sizeof(u64)));
   if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_rotate_tm<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(plane_smem_words(8192) * sizeof(u64)));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_rotate_tm<3, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(plane_smem_words(16384) * sizeof(u64)));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_inverse_ops, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(plane_smem_words(16384) * sizeof(u64)));
+  if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_ntt_half<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              int(plane_smem_words(16384) * sizeof(u64)));
   if (e == cudaSuccess)
@@ -1334,7 +1552,25 @@ int cuhe_bfv_compile_key(cuhe_bfv_ring* ring, const uint8_t* key_polys, uint64_t
         key->d_key, key->d_key_q, (long long)(2 * digits * L), int(L), d);
     e = cudaGetLastError();
   }
+  u64* d_power = nullptr;
+  if (!rc && e == cudaSuccess && ntt_rotations(ring)) {
+    std::vector<u64> power(size_t(digits) * L);
+    for (size_t dgt = 0; dgt < size_t(digits); ++dgt)
+      for (size_t j = 0; j < L; ++j) power[dgt * L + j] = H::powmod(2, u64(dgt) * P.digit_bits, P.primes[j]);
+    e = cudaMalloc(&d_power, power.size() * 8);
+    if (e == cudaSuccess) e = cudaMalloc(&key->d_lift, key->bytes);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(d_power, power.data(), power.size() * 8, cudaMemcpyHostToDevice, ln.stream);
+    if (e == cudaSuccess) {
+      key->d_lift_q = key->d_lift + size_t(digits) * 2 * L * n;
+      const unsigned blocks = blocks_for((long long)(2 * digits * L * n), 256);
+      k_lift_key<<<blocks, 256, 0, ln.stream>>>(key->d_key, d_power, int(digits), int(L), key->d_lift, d);
+      k_shoup_quotients<<<blocks, 256, 0, ln.stream>>>(key->d_lift, key->d_lift_q, (long long)(2 * digits * L), int(L), d);
+      e = cudaGetLastError();
+    }
+  }
   if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(ln.stream);
+  if (d_power) cudaFree(d_power);
   if (d_words) cudaFree(d_words);
   if (rc || e != cudaSuccess) {
     cuhe_bfv_key_release(key);
@@ -1576,7 +1812,10 @@ int cuhe_bfv_hamming_tile(cuhe_bfv_key* relin, const uint8_t* query, const uint8
       return rc;
     return download_words(r, ln, dist, 2, out);
   }
-  BFV_CUDA(ln.arena.reserve(tile_arena_bytes(r, 1) + slice(2 * n * W * 8) * 2 + slice(n * W * 8) + slice(L * n * 8) * 2 +
+  const std::vector<u64> exps(exponents, exponents + rotations);
+  const bool ntt = ntt_circuit(r, exps);
+  BFV_CUDA(ln.arena.reserve((ntt ? tile_ntt_arena_bytes(r, 1, exps.size()) + slice(2 * sizeof(InverseOp))
+                                 : tile_arena_bytes(r, 1)) + slice(2 * n * W * 8) * 2 + slice(n * W * 8) + slice(L * n * 8) * 2 +
                             slice(2 * L * n * 8) + slice(2 * n * W * 8) + 16384),
            "workspace");
   ln.arena.reset();
@@ -1586,17 +1825,22 @@ int cuhe_bfv_hamming_tile(cuhe_bfv_key* relin, const uint8_t* query, const uint8
   if (int rc = upload_polys(r, ln, d, mask, 1, L, &mw, &mres)) return rc;
   BFV_CUDA(launch_ntt(r, ln, d, mres, (long long)(L), 0, int(L), 1, 0), "mask ntt");
   u64* dist = ln.arena.take<u64>(2 * L * n);
+  u64* coef = ntt ? ln.arena.take<u64>(L * n) : nullptr;
   BFV_ARENA(ln.arena);
   TileArgs a;
   a.q_words = qw;
   a.t_words = tw;
   a.ct = 1;
   a.relin = relin;
-  for (uint64_t k = 0; k < rotations; ++k) {
-    a.exps.push_back(exponents[k]);
-    a.keys.push_back(keys[k]);
-  }
+  a.exps = exps;
+  a.keys.assign(keys, keys + rotations);
   a.masks = {mres};
+  if (ntt) {
+    const char need = 0;
+    if (int rc = tile_circuit_ntt(r, ln, d, a, dist, coef, &need, nullptr)) return rc;
+    if (int rc = inverse_polys(r, ln, d, {{dist, dist}, {dist + L * n, dist + L * n}}, ln.arena)) return rc;
+    return compose_out(r, ln, d, dist, 2, out);
+  }
   if (int rc = tile_circuit(r, ln, d, a, dist, nullptr)) return rc;
   return compose_out(r, ln, d, dist, 2, out);
 }
@@ -1753,7 +1997,11 @@ size_t search_chunk_bytes(const cuhe_bfv_server* s, size_t ct, unsigned out_bits
            slice(2 * n * W * 8) + slice(ct * 2 * n * W * 8) * 2 + slice(gc * 2 * n * W * 8) +
            slice(gc * 2 * out_words * 8) + slice(sizeof(int)) + slice(ct * n * W * 8) +
            slice(ct * sizeof(ComposeOp)) + slice(ct * sizeof(SwitchOp)) + small + 65536;
-  return tile_arena_bytes(r, ct) + slice(2 * in_bytes) + slice(ct * 2 * in_bytes) + slice(2 * n * W * 8) +
+  const bool ntt = ntt_circuit(r, s->left);
+  const size_t tiles = ntt ? tile_ntt_arena_bytes(r, ct, s->left.size()) + slice(ct * L * n * 8) + rotate_table_bytes(ct) +
+                                 slice(2 * gc * sizeof(InverseOp))
+                           : tile_arena_bytes(r, ct);
+  return tiles + slice(2 * in_bytes) + slice(ct * 2 * in_bytes) + slice(2 * n * W * 8) +
          slice(ct * 2 * n * W * 8) + slice(ct * 2 * L * n * 8) + slice(gc * 2 * n * W * 8) +
          slice(gc * 2 * out_words * 8) + slice(sizeof(int)) + slice(ct * n * W * 8) + slice(ct * sizeof(ComposeOp)) +
          slice(ct * sizeof(SwitchOp)) + small + 65536;
@@ -1801,6 +2049,7 @@ int search_impl(cuhe_bfv_server* s, const uint8_t* query, const PolySource* inde
   Lane& ln = acquire_lane(r, lock);
   DeviceGuard guard(r->device);
   RingDev* d = s->d_ring;
+  const bool ntt = r->residue && ntt_circuit(r, s->left);
   double prof[6] = {0, 0, 0, 0, 0, 0};
   // partial mask for the last tile
   const u64* partial = nullptr;
@@ -1833,6 +2082,7 @@ int search_impl(cuhe_bfv_server* s, const uint8_t* query, const PolySource* inde
     u64* qw = ln.arena.take<u64>(2 * n * W);
     u64* tw = resident ? const_cast<u64*>(resident) + first * 2 * n * W : ln.arena.take<u64>(ct * 2 * n * W);
     u64* dist = ln.arena.take<u64>(r->residue ? ct * 2 * L * n : ct * 2 * n * W);
+    u64* coef = ntt ? ln.arena.take<u64>(ct * L * n) : nullptr;  // of component 1, where dist is in the NTT domain
     u64* ow = ln.arena.take<u64>(gc * 2 * n * W);
     u64* packed = ln.arena.take<u64>(gc * 2 * out_words);
     int* d_status = ln.arena.take<int>(1);
@@ -1867,13 +2117,8 @@ int search_impl(cuhe_bfv_server* s, const uint8_t* query, const PolySource* inde
     // the lane's arena.  Writes each group's result slot.
     std::vector<size_t> result_slot(gc, 0);
     std::vector<char> merged(gc, 0);
-    auto merge_groups = [&](Lane& lane, size_t g_lo, size_t g_hi, const NativeScratch& nsc, double* pr) -> int {
-      if (g_lo >= g_hi) return CUHE_OK;
-      cudaEvent_t m0, m1;
-      cudaEventCreate(&m0);
-      cudaEventCreate(&m1);
-      cudaEventRecord(m0, lane.stream);
-      struct Merge { size_t left, right; size_t level; size_t wave; };
+    struct Merge { size_t left, right; size_t level; size_t wave; };
+    auto plan_merges = [&](size_t g_lo, size_t g_hi) {
       std::vector<Merge> merges;
       for (size_t gi = g_lo; gi < g_hi; ++gi) {
         struct Node { size_t slot, ready; };
@@ -1907,6 +2152,28 @@ int search_impl(cuhe_bfv_server* s, const uint8_t* query, const PolySource* inde
         }
         result_slot[gi] = result.slot;
       }
+      return merges;
+    };
+    // which tiles are next read as a right operand, whose component 1 is
+    // composed from coefficients; for a merge, whether its result is
+    auto right_next = [&](const std::vector<Merge>& merges, std::vector<char>& slot_next) {
+      std::vector<char> result(merges.size(), 0);
+      for (size_t k = merges.size(); k-- > 0;) {
+        result[k] = slot_next[merges[k].left];
+        slot_next[merges[k].left] = 0;
+        slot_next[merges[k].right] = 1;
+      }
+      return result;
+    };
+    std::vector<char> need(ct, 0);
+    if (ntt) right_next(plan_merges(0, gc), need);
+    auto merge_groups = [&](Lane& lane, size_t g_lo, size_t g_hi, const NativeScratch& nsc, double* pr) -> int {
+      if (g_lo >= g_hi) return CUHE_OK;
+      cudaEvent_t m0, m1;
+      cudaEventCreate(&m0);
+      cudaEventCreate(&m1);
+      cudaEventRecord(m0, lane.stream);
+      const std::vector<Merge> merges = plan_merges(g_lo, g_hi);
       size_t waves = 0;
       for (const auto& m : merges) waves = std::max(waves, m.wave + 1);
       if (!r->residue) {
@@ -1934,6 +2201,36 @@ int search_impl(cuhe_bfv_server* s, const uint8_t* query, const PolySource* inde
           }
           if (int rc = native_add_ops(r, lane, d, adds, nsc.d_nops)) return rc;
         }
+      } else if (ntt) {
+        const size_t mark = lane.arena.used;
+        u64* mwords = lane.arena.take<u64>(std::max<size_t>(1, merges.size()) * n * W);
+        BFV_ARENA(lane.arena);
+        std::vector<char> slots(ct, 0);
+        const std::vector<char> again = right_next(merges, slots);
+        RotateChain chain;
+        for (size_t w = 0; w < waves; ++w) {
+          const size_t start = chain.rops.size();
+          for (size_t k = 0; k < merges.size(); ++k) {
+            const auto& m = merges[k];
+            if (m.wave != w) continue;
+            const u64 g = s->right.at(m.level);
+            const cuhe_bfv_key* key = s->keys.at(g);
+            u64* words = mwords + chain.rops.size() * n * W;
+            RotateOp o{};
+            o.base = o.out = dist + m.left * 2 * L * n;
+            o.x0 = dist + m.right * 2 * L * n;
+            o.x1 = o.x0 + L * n;
+            o.words = words;
+            o.key = key->d_lift;
+            o.key_q = key->d_lift_q;
+            o.coef = again[k] ? coef + m.left * L * n : nullptr;
+            o.g = unsigned(g);
+            chain.add(ComposeOp{coef + m.right * L * n, words, o.g, 0u}, o);
+          }
+          chain.close(start);
+        }
+        if (int rc = run_chain(r, lane, d, chain, lane.arena)) return rc;
+        lane.arena.used = mark;
       } else {
         const size_t mark = lane.arena.used;
         const size_t most = merges.size();
@@ -1984,6 +2281,8 @@ int search_impl(cuhe_bfv_server* s, const uint8_t* query, const PolySource* inde
         }
         a.masks.assign(tc, s->d_full_mask);
         if (partial && first + t0 + tc == size_t(tiles)) a.masks[tc - 1] = partial;
+        if (ntt)
+          return tile_circuit_ntt(r, lane, d, a, dist + t0 * 2 * L * n, coef + t0 * L * n, need.data() + t0, pr);
         return tile_circuit(r, lane, d, a, dist + t0 * 2 * L * n, pr);
       }
       std::vector<u64> exps(s->left.begin(), s->left.end());
@@ -2021,7 +2320,10 @@ int search_impl(cuhe_bfv_server* s, const uint8_t* query, const PolySource* inde
       size_t offset = mark;
       for (int k = 0; k < K; ++k) {
         part[k].arena.owned = false;
-        const size_t bytes = r->residue ? tile_arena_bytes(r, bound[k + 1] - bound[k]) : small_switch_bytes(r);
+        const size_t tiles_k = bound[k + 1] - bound[k];
+        const size_t bytes = ntt          ? tile_ntt_arena_bytes(r, tiles_k, s->left.size())
+                             : r->residue ? tile_arena_bytes(r, tiles_k)
+                                          : small_switch_bytes(r);
         part[k].arena.base = ln.arena.base + offset;
         part[k].arena.cap = bytes;
         offset += bytes;
@@ -2198,6 +2500,15 @@ int search_impl(cuhe_bfv_server* s, const uint8_t* query, const PolySource* inde
     BFV_ARENA(ln.arena);
     // outputs: compose, optional compaction, packing
     if (r->residue) {
+      if (ntt) {
+        std::vector<InverseOp> polys;
+        for (size_t gi = 0; gi < gc; ++gi)
+          for (size_t comp = 0; comp < 2; ++comp) {
+            u64* poly = dist + (result_slot[gi] * 2 + comp) * L * n;
+            polys.push_back({poly, poly});
+          }
+        if (int rc = inverse_polys(r, ln, d, polys, ln.arena)) return rc;
+      }
       std::vector<ComposeOp> cops;
       for (size_t gi = 0; gi < gc; ++gi)
         for (size_t comp = 0; comp < 2; ++comp)
