@@ -23,6 +23,7 @@ NVCC_FLAGS = [
     "-lineinfo", "-O3", "-std=c++17",
     "-shared", "-Xcompiler", "-fPIC",
     "--expt-relaxed-constexpr",
+    "--split-compile=0",  # one optimiser thread per core
 ]
 
 LIBRARIES = {

@@ -90,6 +90,7 @@ struct cuhe_paillier {
   cuhe::KeyScalars ks{};
   Limbs n, n2;
   Limbs secret_exp;  // empty until set
+  Limbs secret_mult;
   bool have_secret = false;
   int32_t* d_ops_n = nullptr;
   int nops_n = 0;
@@ -109,8 +110,8 @@ struct cuhe_paillier {
   struct SideExponent {
     int32_t* d_ops = nullptr;
     int32_t* d_fall = nullptr;
-    int nops = 0, nfall = 0, scaled = 0;
-    cuhe::PairExponent get() const { return {d_ops, d_fall, nops, nfall, scaled}; }
+    int nops = 0, nfall = 0, halved = 0;
+    cuhe::PairExponent get() const { return {d_ops, d_fall, nops, nfall, halved}; }
   } side_exp[2];
   Limbs factor[2];  // p, q once installed
   cuhe::CrtScalars cs{};
@@ -219,14 +220,25 @@ cudaError_t launch_modexp_crt(cuhe_paillier* ctx, const uint32_t* base, uint32_t
   return cudaGetLastError();
 }
 
-// Batches of at most one CTA of the five-limb kernels to an SM (items5 items a
-// CTA; one warp to a scheduler) run with five limbs per lane: at key_len 1024
-// 2,368 decodes take 1.27 ms against 2.19 with ten, as many decryptions 4.2
-// against 7.3, encryptions 13.3 against 22.7.  With two CTAs to an SM the ten-
-// limb kernel, whose one warp per scheduler then holds the same items, is as
-// fast or faster (decodes 2.15 and 2.19 ms, encryptions 25.5 and 22.7).
-bool pair_small(const cuhe_paillier* ctx, long long count, int items5) {
-  return count <= (long long)ctx->sms * items5;
+// Batches of at most one CTA of the five-limb kernels to an SM (half the ten-
+// limb kernel's items10 a CTA; one warp to a scheduler) run with five limbs
+// per lane: at key_len 1024 2,368 decodes take 1.27 ms against 2.19 with ten,
+// as many decryptions 4.2 against 7.3, encryptions 13.3 against 22.7.  With
+// two CTAs to an SM the ten-limb kernel, whose one warp per scheduler then
+// holds the same items, is as fast or faster (decodes 2.15 and 2.19 ms,
+// encryptions 25.5 and 22.7).
+bool pair_small(const cuhe_paillier* ctx, long long count, int items10) {
+  return count <= (long long)ctx->sms * items10 / 2;
+}
+
+// How many of a batch's items run with ten limbs per lane: none of a small
+// batch, and of a larger one all, or all but a small remainder after whole
+// waves of two CTAs to an SM, which would hold the SMs for as long as a whole
+// one-CTA wave (20,011 decryptions at key_len 512: 4.8 -> 4.3 ms).
+long long pair_waves(const cuhe_paillier* ctx, long long count, int items10) {
+  if (pair_small(ctx, count, items10)) return 0;
+  const long long rest = count % (2ll * ctx->sms * items10);
+  return rest < count && pair_small(ctx, rest, items10) ? count - rest : count;
 }
 
 // The same on pairs of residues mod p and mod q (k_pair_crt).
@@ -247,9 +259,14 @@ cudaError_t launch_pair_crt_l(cuhe_paillier* ctx, const uint32_t* base, uint32_t
 template <int KH>
 cudaError_t launch_pair_crt(cuhe_paillier* ctx, const uint32_t* base, uint32_t* out, long long count, int mode,
                             int pop_words) {
-  if (pair_small(ctx, count, cuhe::PairLayout<5 * KH / 16, 5, 4, 2>::kItems))
-    return launch_pair_crt_l<KH, 5>(ctx, base, out, count, mode, pop_words);
-  return launch_pair_crt_l<KH, 10>(ctx, base, out, count, mode, pop_words);
+  const long long main = pair_waves(ctx, count, cuhe::PairLayout<5 * KH / 16, 10, 4, 2>::kItems);
+  if (main) {
+    if (cudaError_t e = launch_pair_crt_l<KH, 10>(ctx, base, out, main, mode, pop_words)) return e;
+    if (main == count) return cudaSuccess;
+    base += main * 2 * KH;
+    out += mode == cuhe::EXP_DECODE ? main : main * 2 * KH;
+  }
+  return launch_pair_crt_l<KH, 5>(ctx, base, out, count - main, mode, pop_words);
 }
 
 // The exponentiation mod n^2 on pairs of residues mod n (no factors needed).
@@ -270,9 +287,15 @@ cudaError_t launch_pair_modexp_l(cuhe_paillier* ctx, const uint32_t* base, const
 template <int K>
 cudaError_t launch_pair_modexp(cuhe_paillier* ctx, const uint32_t* base, const uint32_t* aux, uint32_t* out,
                                long long count, const int32_t* ops, int nops, int mode, int pop_words) {
-  if (pair_small(ctx, count, cuhe::PairLayout<5 * K / 16, 5, 2, 1>::kItems))
-    return launch_pair_modexp_l<K, 5>(ctx, base, aux, out, count, ops, nops, mode, pop_words);
-  return launch_pair_modexp_l<K, 10>(ctx, base, aux, out, count, ops, nops, mode, pop_words);
+  const long long main = pair_waves(ctx, count, cuhe::PairLayout<5 * K / 16, 10, 2, 1>::kItems);
+  if (main) {
+    if (cudaError_t e = launch_pair_modexp_l<K, 10>(ctx, base, aux, out, main, ops, nops, mode, pop_words)) return e;
+    if (main == count) return cudaSuccess;
+    base += main * K;
+    if (aux) aux += main * K;
+    out += mode == cuhe::EXP_DECODE ? main : main * K;
+  }
+  return launch_pair_modexp_l<K, 5>(ctx, base, aux, out, count - main, ops, nops, mode, pop_words);
 }
 
 // k_pair_modexp for this context's width when the FP64 pipe is selected, else null.
@@ -366,7 +389,7 @@ cudaError_t launch_pair_lookup_l(cuhe_paillier* ctx, const cuhe::LookupDigits& d
 template <int K>
 cudaError_t launch_pair_lookup(cuhe_paillier* ctx, const cuhe::LookupDigits& dg, long long count, const double2* table,
                                const double2* noise, bool pairs, const uint8_t* idx, uint32_t* out) {
-  if (pair_small(ctx, count, cuhe::LookupLayout<K, 5>::kGroups))
+  if (pair_small(ctx, count, cuhe::LookupLayout<K, 10>::kGroups))
     return launch_pair_lookup_l<K, 5>(ctx, dg, count, table, noise, pairs, idx, out);
   return launch_pair_lookup_l<K, 10>(ctx, dg, count, table, noise, pairs, idx, out);
 }
@@ -777,8 +800,8 @@ void balanced52(const Limbs& v, size_t k, double* out, size_t stride) {
 }
 
 // The constants of one modulus m (pair_const_doubles) for pair_power: k limbs
-// per component, `entry` chunks of a value; scale: null, or the cofactor u of
-// an exponent u (m - 1).  m in its natural limb count w; m^2 in 2w limbs.
+// per component, `entry` chunks of a value; scale: null, or the factor of the
+// scale row.  m in its natural limb count w; m^2 in 2w limbs.
 std::vector<double> pair_constants(const Limbs& m_in, size_t k, int entry, const Limbs* scale) {
   Limbs m = m_in;
   while (m.size() > 1 && m.back() == 0) m.pop_back();
@@ -832,25 +855,34 @@ int setup_pair_crt(cuhe_paillier* ctx) {
   std::vector<double> block;
   for (int s = 0; s < 2; ++s) {
     auto& side = ctx->side_exp[s];
-    const Limbs& p = ctx->factor[s];
+    Limbs p = ctx->factor[s], other = ctx->factor[1 - s];
     ctx->cs.ninv52[s] = negative_inverse52(p);
-    side.scaled = 0;
-    Limbs cofactor, main = ctx->secret_exp;
-    if (ctx->have_secret && !cuhe::host::is_zero(ctx->secret_exp)) {
+    side.halved = 0;
+    Limbs cofactor, main = ctx->secret_exp, scale;
+    if (ctx->have_secret) {
+      // (other factor)^-1 multiplier [cofactor] mod p
+      while (p.size() > 1 && p.back() == 0) p.pop_back();
+      const size_t w = p.size();
+      Limbs inv;
+      if (!cuhe::host::mod_inverse_odd(cuhe::host::mod_reduce(other, p), p, &inv))
+        return fail(ctx, CUHE_INVALID_ARGUMENT, "factors are not coprime");
+      scale = cuhe::host::mod_reduce(cuhe::host::mul(inv, cuhe::host::mod_reduce(ctx->secret_mult, p), 2 * w), p);
       Limbs pm1 = p;
       pm1[0] -= 1u;  // p is odd
       while (pm1.size() > 1 && pm1.back() == 0) pm1.pop_back();
-      if (cuhe::host::is_zero(cuhe::host::mod_reduce(ctx->secret_exp, pm1, &cofactor)) &&
+      if (!cuhe::host::is_zero(ctx->secret_exp) &&
+          cuhe::host::is_zero(cuhe::host::mod_reduce(ctx->secret_exp, pm1, &cofactor)) &&
           cuhe::host::bit_length(cofactor) > 1) {
-        side.scaled = 1;
+        side.halved = 1;
         main = pm1;
+        scale = cuhe::host::mod_reduce(cuhe::host::mul(scale, cuhe::host::mod_reduce(cofactor, p), 2 * w), p);
       }
     }
-    const std::vector<double> one = pair_constants(p, k, 4, side.scaled ? &cofactor : nullptr);
+    const std::vector<double> one = pair_constants(p, k, 4, ctx->have_secret ? &scale : nullptr);
     block.insert(block.end(), one.begin(), one.end());
     if (!ctx->have_secret) continue;
     if (int rc = upload_schedule(ctx, main, &side.d_ops, &side.nops, cuhe::kPairWindow)) return rc;
-    if (side.scaled)
+    if (side.halved)
       if (int rc = upload_schedule(ctx, cofactor, &side.d_fall, &side.nfall, cuhe::kPairWindow)) return rc;
   }
   return upload_constants(ctx, block, &ctx->d_crt52);
@@ -1077,6 +1109,7 @@ int cuhe_paillier_set_secret(cuhe_paillier* ctx, const uint32_t* exponent, int e
             "secret upload");
   ctx->ks.mult_is_zero = cuhe::host::is_zero(mult) ? 1u : 0u;
   ctx->secret_exp = e;
+  ctx->secret_mult = mult;
   ctx->have_secret = true;
   if (int rc = upload_schedule(ctx, e, &ctx->d_ops_sec52, &ctx->nops_sec52, cuhe::kPairWindow)) return rc;
   if (int rc = setup_pair_crt(ctx)) return rc;
@@ -1120,6 +1153,16 @@ int cuhe_paillier_set_factors(cuhe_paillier* ctx, const uint32_t* p_in, int p_wo
     put_half(cuhe::CR_R3, s, cuhe::host::shift_mod(rm, 64 * kh, side[s]));
     put_half(cuhe::CR_PR, s, cuhe::host::shift_mod(cuhe::host::resized((s ? q : p).data(), kh, kh), 32 * kh, side[s]));
     ctx->cs.ninv[s] = 0u - cuhe::host::inv32(side[s][0]);
+  }
+  put_half(cuhe::CR_P, 0, cuhe::host::resized(p.data(), kh, kh));
+  {
+    const Limbs ph = cuhe::host::resized(p.data(), kh, kh), nh = cuhe::host::resized(ctx->n.data(), kh, kh);
+    Limbs qp;
+    if (!cuhe::host::mod_inverse_odd(cuhe::host::mod_reduce(q, ph), ph, &qp))
+      return fail(ctx, CUHE_INVALID_ARGUMENT, "factors are not coprime");
+    put_half(cuhe::CR_QI, 0, cuhe::host::shift_mod(qp, 32 * kh, ph));
+    put_half(cuhe::CR_QR, 0, cuhe::host::shift_mod(cuhe::host::resized(q.data(), kh, kh), 32 * kh, nh));
+    ctx->cs.pinv = 0u - cuhe::host::inv32(p[0]);
   }
   put_half(cuhe::CR_H, 0, cuhe::host::shift_mod(qinv, 32 * kh, side[0]));
   Limbs cq = cuhe::host::shift_mod(cuhe::host::resized(side[1].data(), kh, k), 32 * k, ctx->n2);

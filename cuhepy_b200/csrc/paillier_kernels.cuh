@@ -35,11 +35,15 @@ enum CrtRow : int {
   CR_H = 3,    // (q^2)^-1 R_h mod p^2 | 0
   CR_CQ = 4,   // q^2 R mod n^2 (full row)
   CR_PR = 5,   // p R_h mod p^2 | q R_h mod q^2
-  CR_ROWS = 6
+  CR_P = 6,    // p | 0
+  CR_QI = 7,   // q^-1 R_h mod p | 0
+  CR_QR = 8,   // q R_h mod n | 0
+  CR_ROWS = 9
 };
 
 struct CrtScalars {
   uint32_t ninv[2];   // -(p^2)^-1, -(q^2)^-1 mod 2^32
+  uint32_t pinv;      // -p^-1 mod 2^32
   unsigned long long ninv52[2];  // -p^-1, -q^-1 mod 2^52
 };
 
@@ -563,19 +567,18 @@ constexpr int kPairWindow = 3;                       // odd powers x, x^3, x^5, 
 constexpr int kPairTable = 1 << (kPairWindow - 1);
 
 // Constants of one modulus m as doubles: m as K limbs, then rows of K pairs:
-// the entry chunks' R^(j+2) mod m^2, (1, 0), (u R mod m, 0) and R mod m^2.
+// the entry chunks' R^(j+2) mod m^2, (1, 0), (w R mod m, 0) and R mod m^2.
 __host__ __device__ constexpr int pair_const_doubles(int K, int entry) { return K + 2 * K * (entry + 3); }
 
-// An exponent's window schedule, or x^e by way of x^(m-1) (PairExponent::scaled).
+// An exponent's window schedule.  halved: e = u (p - 1) and the schedule is
+// that of p - 1; when x^(p-1) = 1 + p z1 (always, for x prime to a prime p),
+// x^e = 1 + p (z1 u mod p).  Any other value in a CTA sends it through the
+// schedule `fall` of u next, which holds for every x and every p.
 struct PairExponent {
   const int32_t* ops;
   const int32_t* fall;
   int nops, nfall;
-  // e = u (p - 1): the schedule is that of p - 1.  When x^(p-1) = 1 + p z1
-  // (always, for x prime to a prime p), x^e = 1 + p (z1 u mod p); any other
-  // value in a warp sends the warp through the schedule `fall` of u, which
-  // holds for every x and every p.
-  int scaled;
+  int halved;
 };
 
 template <int K, int TPI>
@@ -593,8 +596,11 @@ __device__ __forceinline__ void pair_publish(const cuhe52::Pair52<K, TPI>& f, do
 // memory; s = this group's K pairs, tab = this thread's table column (stride
 // kPairThreads).  aux: null, or the words a of the factor (1, a).  Leaves the
 // canonical limbs (z0, z1), each in [0, m], as pairs of 64-bit integers in s.
-template <int K, int TPI, int kEntry>
-__device__ __forceinline__ void pair_power(const cuhe52::Pair52<K, TPI>& f, const uint32_t* __restrict__ words,
+// kUnits (every thread of the CTA calls it): when z0 is 1 for every value of
+// the CTA, leaves (1, z1 w mod m) instead, w the scale row's factor, and
+// returns true.
+template <int K, int TPI, int kEntry, bool kUnits>
+__device__ __forceinline__ bool pair_power(const cuhe52::Pair52<K, TPI>& f, const uint32_t* __restrict__ words,
                                            int nwords, const double2* rows, const double2* __restrict__ one,
                                            double2* s, double2* tab, const double (&m)[K / TPI], uint64_t ninv,
                                            const PairExponent& ex, const uint32_t* __restrict__ aux) {
@@ -602,13 +608,14 @@ __device__ __forceinline__ void pair_power(const cuhe52::Pair52<K, TPI>& f, cons
   constexpr int kStride = cuhe52::kPairThreads;
   const int32_t* ops = ex.ops;
   int nops = ex.nops;
-  bool scaled = ex.scaled != 0;
+  bool halved = kUnits && ex.halved != 0;
   double z0[L], z1[L], a0[L], a1[L];
   uint64_t A0[L], A1[L];
   const int at = f.gl * L;
   auto bits = [](double d) { return static_cast<uint64_t>(__double_as_longlong(d)); };
   auto raw = [](uint64_t v) { return __longlong_as_double(static_cast<long long>(v)); };
 
+  bool voted = false;
   int j = 0;  // entry chunks, then the square of x; again from there with the schedule ex.fall
   while (true) {
 #pragma unroll 1
@@ -737,15 +744,20 @@ __device__ __forceinline__ void pair_power(const cuhe52::Pair52<K, TPI>& f, cons
       isone = isone && A0[k] == (at + k == 0 ? 1ull : 0ull);
     }
     __syncwarp();
-    if (!scaled) return;
-    if (__all_sync(0xffffffffu, isone)) break;
-    // x^(p-1) is not 1 mod p somewhere: raise it (still in z) to u instead
-    scaled = false;
+    if (!kUnits) return false;
+    // (once per thread: a CTA whose values are not all units stays in the
+    // general form from here on)
+    if (!voted) {
+      if (__syncthreads_and(isone)) break;
+      voted = true;
+    }
+    if (!halved) return false;
+    halved = false;  // raise x^(p-1) (still in z) to u
     ops = ex.fall;
     nops = ex.nfall;
     j = kEntry;
   }
-  // (1, z1) -> (1, z1 u mod p)
+  // (1, z1) -> (1, z1 w mod m)
 #pragma unroll
   for (int k = 0; k < L; ++k) a0[k] = f.to_f64(A1[k]);
   f.template product<false>(A0, A1, a0, a0, rows + (kEntry + 1) * K, m, ninv);
@@ -753,7 +765,7 @@ __device__ __forceinline__ void pair_power(const cuhe52::Pair52<K, TPI>& f, cons
   f.canonical(A0);
 #pragma unroll
   for (int k = 0; k < L; ++k) s[at + k].y = raw(A0[k]);
-  __syncwarp();
+  return true;
 }
 
 // word i (32 bits at 32 i) of component `second` of K pairs of 64-bit limbs
@@ -798,8 +810,10 @@ struct PairLayout {  // K limbs per component (kL per lane), kSides moduli per i
 
 // Decrypt / decode with the factors installed: c^e mod p^2 and mod q^2 in the
 // two halves of the CTA (whole warps per side, so each side follows its own
-// schedule), then Garner's recombination and the epilogue of k_modexp_crt on
-// words, 2 KH / 16 lanes per ciphertext.
+// schedule).  For ciphertexts c^e is 1 mod n and the plaintext comes from the
+// second components alone; a CTA with any other value takes Garner's
+// recombination and the epilogue of k_modexp_crt on words, 2 KH / 16 lanes
+// per ciphertext.
 template <int KH, int kL>
 __global__ void __launch_bounds__(cuhe52::kPairThreads, 2)
 k_pair_crt(const uint32_t* __restrict__ base, uint32_t* __restrict__ out, long long count,
@@ -819,6 +833,7 @@ k_pair_crt(const uint32_t* __restrict__ base, uint32_t* __restrict__ out, long l
   }
   __syncthreads();
   const long long first = (long long)blockIdx.x * IPB;
+  bool units;
   {
     const int side = threadIdx.x / (cuhe52::kPairThreads / 2);
     const int group = threadIdx.x / TPI;  // side * IPB + item
@@ -828,12 +843,81 @@ k_pair_crt(const uint32_t* __restrict__ base, uint32_t* __restrict__ out, long l
     double m[kL];
 #pragma unroll
     for (int k = 0; k < kL; ++k) m[k] = __ldg(cm + f.gl * kL + k);
-    pair_power<KL, TPI, kEntry>(f, base + inst * K, K, s_rows + side * Lay::kRows,
-                                reinterpret_cast<const double2*>(cm + KL) + (kEntry + 2) * KL,
-                                s_vals + group * Lay::kSlot, s_tab + threadIdx.x, m,
-                                f.gl == 0 ? cs.ninv52[side] : 0ull, side ? e1 : e0, nullptr);
+    units = pair_power<KL, TPI, kEntry, true>(f, base + inst * K, K, s_rows + side * Lay::kRows,
+                                              reinterpret_cast<const double2*>(cm + KL) + (kEntry + 2) * KL,
+                                              s_vals + group * Lay::kSlot, s_tab + threadIdx.x, m,
+                                              f.gl == 0 ? cs.ninv52[side] : 0ull, side ? e1 : e0, nullptr);
   }
   __syncthreads();
+  if (units) {
+    // x^e = 1 + n t with t mult = r_p mod p, r_q mod q (the scale rows hold
+    // q^-1 mult and p^-1 mult, times the cofactor): the plaintext
+    // t mult mod n = r_q + q ((r_p - r_q) q^-1 mod p), three products of KH
+    // words an item where the general recombination below takes five of K
+    // words and four of KH (key_len 1024: 0.40 of 3.94 ms a wave of decodes)
+    constexpr int LT = KH / 16, L = 16, PER = cuhe52::kPairThreads / LT;
+    uint32_t* s_qi = reinterpret_cast<uint32_t*>(s_tab);
+    uint32_t* s_qr = s_qi + KH;
+    for (int i = threadIdx.x; i < KH; i += blockDim.x) {
+      s_qi[i] = crt[CR_QI * K + i];
+      s_qr[i] = crt[CR_QR * K + i];
+    }
+    __syncthreads();
+    Group<KH, LT> h;
+#pragma unroll 1
+    for (int item = threadIdx.x / LT; item < IPB; item += PER) {
+      const long long inst = first + item;
+      if (inst >= count) break;
+      uint32_t x[L], y[L], u[L], m[L];
+      {
+        // c < n^2: the upper half decides unless it equals n^2's
+        h.load(x, base + inst * K + KH);
+        h.load_ro(y, consts + C_N2 * K + KH);
+        bool less = h.less_than(x, y);
+        if (!less) {
+          sub_group<KH, LT>(h, x, y);  // zero when they are equal
+          const bool equal = h.is_zero(x);
+          h.load(x, base + inst * K);
+          h.load_ro(y, consts + C_N2 * K);
+          less = equal && h.less_than(x, y);
+        }
+        if (!less) {
+          if (h.gl == 0) atomicOr(status, ST_RANGE);
+          continue;
+        }
+      }
+      const double2* sp = s_vals + item * Lay::kSlot;
+      const double2* sq = s_vals + (IPB + item) * Lay::kSlot;
+      h.load_ro(m, crt + CR_P * K);
+#pragma unroll
+      for (int t = 0; t < L; ++t) {
+        x[t] = word_from_pairs<KL>(sp, true, h.gl * L + t);
+        y[t] = word_from_pairs<KL>(sq, true, h.gl * L + t);
+      }
+      h.mont_mul(u, x, s_qi, m, cs.pinv);  // r_p q^-1 mod p
+      h.mont_mul(x, y, s_qi, m, cs.pinv);  // r_q q^-1 mod p
+      sub_mod<KH, LT>(h, u, x, m);
+      h.load_ro(m, consts + C_N * K);
+      h.mont_mul(x, u, s_qr, m, ks.ninv1);  // q times that, at most n - q
+      (void)add_group<KH, LT>(h, x, y);     // r_q is at most q
+      if (!h.less_than(x, m)) sub_group<KH, LT>(h, x, m);
+      if (mode == EXP_DECRYPT) {
+        h.store(out + inst * K, x);
+#pragma unroll
+        for (int t = 0; t < L; ++t) x[t] = 0u;
+        h.store(out + inst * K + KH, x);
+      } else {
+        int pc = 0;
+#pragma unroll
+        for (int t = 0; t < L; ++t)
+          if (h.gl * L + t < pop_words) pc += __popc(x[t] & 0x55555555u);
+#pragma unroll
+        for (int off = LT / 2; off > 0; off >>= 1) pc += __shfl_xor_sync(h.mask, pc, off, LT);
+        if (h.gl == 0) out[inst] = uint32_t(pc);
+      }
+    }
+    return;
+  }
   // words: ONE, R2N, MULTR (K words each), p R_h, H (two halves), CQ, then
   // per item of a pass x_p and x_q (KH words each), over the powers' table
   constexpr int LT = KH / 16, L = 16;  // lanes per side
@@ -926,7 +1010,7 @@ __device__ __forceinline__ void pair_modexp_unit(const uint32_t* __restrict__ ba
 #pragma unroll
     for (int k = 0; k < kL; ++k) m[k] = __ldg(n52 + f.gl * kL + k);
     const PairExponent ex{ops, nullptr, nops, 0, 0};
-    pair_power<KL, TPI, kEntry>(f, base + inst * K, K, s_rows,
+    (void)pair_power<KL, TPI, kEntry, false>(f, base + inst * K, K, s_rows,
                                 reinterpret_cast<const double2*>(n52 + KL) + (kEntry + 2) * KL,
                                 s_vals + group * Lay::kSlot, s_tab + threadIdx.x, m, f.gl == 0 ? ninv52 : 0ull, ex,
                                 mode == EXP_ENCRYPT ? aux + inst * K : nullptr);

@@ -305,18 +305,19 @@ struct Pair52 {
       carry = t >> 52;
       v[k] = static_cast<uint64_t>(t) & kMask;
     }
-    if constexpr (TPI == 1) return;
-    for (int guard = 0; guard < TPI; ++guard) {
-      int c = __shfl_up_sync(0xffffffffu, static_cast<int>(carry), 1, TPI);
-      if (gl == 0) c = 0;
-      carry = c;
+    if constexpr (TPI > 1) {
+      for (int guard = 0; guard < TPI; ++guard) {
+        int c = __shfl_up_sync(0xffffffffu, static_cast<int>(carry), 1, TPI);
+        if (gl == 0) c = 0;
+        carry = c;
 #pragma unroll
-      for (int k = 0; k < L; ++k) {
-        const int64_t t = static_cast<int64_t>(v[k]) + carry;
-        carry = t >> 52;
-        v[k] = static_cast<uint64_t>(t) & kMask;
+        for (int k = 0; k < L; ++k) {
+          const int64_t t = static_cast<int64_t>(v[k]) + carry;
+          carry = t >> 52;
+          v[k] = static_cast<uint64_t>(t) & kMask;
+        }
+        if (!__any_sync(0xffffffffu, gl != TPI - 1 && carry != 0)) break;
       }
-      if (!__any_sync(0xffffffffu, gl != TPI - 1 && carry != 0)) break;
     }
   }
 };
