@@ -29,7 +29,8 @@ NVCC_FLAGS = [
 LIBRARIES = {
     "libcuhe_b200.so": {
         "sources": ["cuhe_paillier.cu"],
-        "depends": ["bigint52.cuh", "bigint_group.cuh", "host_bigint.h", "pair52.cuh", "paillier_kernels.cuh"],
+        "depends": ["bigint52.cuh", "bigint_group.cuh", "host_bigint.h", "pair52.cuh", "pair52_split.cuh",
+                    "paillier_kernels.cuh", "split_kernels.cuh"],
         "headers": ["cuhe_paillier.h"],
     },
     "libcuhe_bfv_b200.so": {

@@ -13,6 +13,7 @@
 #include "../../include/cuhe_paillier.h"
 #include "host_bigint.h"
 #include "paillier_kernels.cuh"
+#include "split_kernels.cuh"
 
 using cuhe::host::Limbs;
 
@@ -222,13 +223,22 @@ cudaError_t launch_modexp_crt(cuhe_paillier* ctx, const uint32_t* base, uint32_t
 
 // Batches of at most one CTA of the five-limb kernels to an SM (half the ten-
 // limb kernel's items10 a CTA; one warp to a scheduler) run with five limbs
-// per lane: at key_len 1024 2,368 decodes take 1.27 ms against 2.19 with ten,
+// per lane: at key_len 1024 2,368 decodes take 1.21 ms against 2.19 with ten,
 // as many decryptions 4.2 against 7.3, encryptions 13.3 against 22.7.  With
 // two CTAs to an SM the ten-limb kernel, whose one warp per scheduler then
 // holds the same items, is as fast or faster (decodes 2.15 and 2.19 ms,
 // encryptions 25.5 and 22.7).
 bool pair_small(const cuhe_paillier* ctx, long long count, int items10) {
   return count <= (long long)ctx->sms * items10 / 2;
+}
+
+// And batches of at most one CTA of the split kernels to an SM (a quarter of
+// items10, again one warp to a scheduler) run with the components on
+// different lanes: 1,184 decodes at key_len 1024 take 0.90 ms against 1.21
+// with five limbs a lane, 592 encryptions at key_len 2048 37.1 against 52.9.
+// One item more, two CTAs to an SM, 1.49 against 1.21 and 66.4 against 52.9.
+bool pair_tiny(const cuhe_paillier* ctx, long long count, int items10) {
+  return count <= (long long)ctx->sms * items10 / 4;
 }
 
 // How many of a batch's items run with ten limbs per lane: none of a small
@@ -266,6 +276,8 @@ cudaError_t launch_pair_crt(cuhe_paillier* ctx, const uint32_t* base, uint32_t* 
     base += main * 2 * KH;
     out += mode == cuhe::EXP_DECODE ? main : main * 2 * KH;
   }
+  if (pair_tiny(ctx, count - main, cuhe::PairLayout<5 * KH / 16, 10, 4, 2>::kItems))
+    return launch_pair_crt_l<KH, cuhe::kSplit>(ctx, base, out, count - main, mode, pop_words);
   return launch_pair_crt_l<KH, 5>(ctx, base, out, count - main, mode, pop_words);
 }
 
@@ -295,6 +307,8 @@ cudaError_t launch_pair_modexp(cuhe_paillier* ctx, const uint32_t* base, const u
     if (aux) aux += main * K;
     out += mode == cuhe::EXP_DECODE ? main : main * K;
   }
+  if (pair_tiny(ctx, count - main, cuhe::PairLayout<5 * K / 16, 10, 2, 1>::kItems))
+    return launch_pair_modexp_l<K, cuhe::kSplit>(ctx, base, aux, out, count - main, ops, nops, mode, pop_words);
   return launch_pair_modexp_l<K, 5>(ctx, base, aux, out, count - main, ops, nops, mode, pop_words);
 }
 

@@ -609,6 +609,7 @@ __device__ __forceinline__ bool pair_power(const cuhe52::Pair52<K, TPI>& f, cons
   const int32_t* ops = ex.ops;
   int nops = ex.nops;
   bool halved = kUnits && ex.halved != 0;
+  asm volatile("" : "+l"(ninv));  // held, not selected again in every step
   double z0[L], z1[L], a0[L], a1[L];
   uint64_t A0[L], A1[L];
   const int at = f.gl * L;
@@ -797,6 +798,9 @@ __device__ __forceinline__ void pair_words(const Group<K, TPI>& g, uint32_t (&x)
   if (!g.less_than(x, mm)) sub_group<K, TPI>(g, x, mm);
 }
 
+// kL of the split form (pair52_split.cuh), whose layout is a specialisation.
+constexpr int kSplit = -5;
+
 template <int K, int kL, int kEntry, int kSides>
 struct PairLayout {  // K limbs per component (kL per lane), kSides moduli per item
   static constexpr int TPI = K / kL;
@@ -807,6 +811,11 @@ struct PairLayout {  // K limbs per component (kL per lane), kSides moduli per i
   static constexpr size_t kTab = size_t(kPairTable) * kL * cuhe52::kPairThreads;
   static constexpr size_t kBytes = (size_t(kSides) * kRows + size_t(kGroups) * kSlot + kTab) * 16;
 };
+
+template <int KL, int kEntry, int kSides, bool kUnits>
+__device__ __forceinline__ bool split_run(double* smem, const double* __restrict__ cm, int side, int group,
+                                          const uint32_t* __restrict__ words, int nwords, uint64_t ninv52,
+                                          const PairExponent& ex, const uint32_t* __restrict__ aux);
 
 // Decrypt / decode with the factors installed: c^e mod p^2 and mod q^2 in the
 // two halves of the CTA (whole warps per side, so each side follows its own
@@ -827,26 +836,33 @@ k_pair_crt(const uint32_t* __restrict__ base, uint32_t* __restrict__ out, long l
   double2* s_vals = s_rows + 2 * Lay::kRows;
   double2* s_tab = s_vals + Lay::kGroups * Lay::kSlot;
   constexpr int kConst = pair_const_doubles(KL, kEntry);
-  for (int i = threadIdx.x; i < 2 * Lay::kRows; i += blockDim.x) {
-    const int sd = i / Lay::kRows;
-    s_rows[i] = reinterpret_cast<const double2*>(crt52 + sd * kConst + KL)[i - sd * Lay::kRows];
+  if constexpr (kL != kSplit) {
+    for (int i = threadIdx.x; i < 2 * Lay::kRows; i += blockDim.x) {
+      const int sd = i / Lay::kRows;
+      s_rows[i] = reinterpret_cast<const double2*>(crt52 + sd * kConst + KL)[i - sd * Lay::kRows];
+    }
+    __syncthreads();
   }
-  __syncthreads();
   const long long first = (long long)blockIdx.x * IPB;
   bool units;
   {
     const int side = threadIdx.x / (cuhe52::kPairThreads / 2);
     const int group = threadIdx.x / TPI;  // side * IPB + item
     const long long inst = min(first + group - side * IPB, count - 1);  // idle groups repeat the last item
-    cuhe52::Pair52<KL, TPI> f;
-    const double* cm = crt52 + side * kConst;
-    double m[kL];
+    if constexpr (kL == kSplit) {
+      units = split_run<KL, kEntry, 2, true>(reinterpret_cast<double*>(smem), crt52, side, group, base + inst * K, K,
+                                             cs.ninv52[side], side ? e1 : e0, nullptr);
+    } else {
+      cuhe52::Pair52<KL, TPI> f;
+      const double* cm = crt52 + side * kConst;
+      double m[kL];
 #pragma unroll
-    for (int k = 0; k < kL; ++k) m[k] = __ldg(cm + f.gl * kL + k);
-    units = pair_power<KL, TPI, kEntry, true>(f, base + inst * K, K, s_rows + side * Lay::kRows,
-                                              reinterpret_cast<const double2*>(cm + KL) + (kEntry + 2) * KL,
-                                              s_vals + group * Lay::kSlot, s_tab + threadIdx.x, m,
-                                              f.gl == 0 ? cs.ninv52[side] : 0ull, side ? e1 : e0, nullptr);
+      for (int k = 0; k < kL; ++k) m[k] = __ldg(cm + f.gl * kL + k);
+      units = pair_power<KL, TPI, kEntry, true>(f, base + inst * K, K, s_rows + side * Lay::kRows,
+                                                reinterpret_cast<const double2*>(cm + KL) + (kEntry + 2) * KL,
+                                                s_vals + group * Lay::kSlot, s_tab + threadIdx.x, m,
+                                                f.gl == 0 ? cs.ninv52[side] : 0ull, side ? e1 : e0, nullptr);
+    }
   }
   __syncthreads();
   if (units) {
@@ -998,22 +1014,30 @@ __device__ __forceinline__ void pair_modexp_unit(const uint32_t* __restrict__ ba
   double2* s_rows = reinterpret_cast<double2*>(smem);
   double2* s_vals = s_rows + Lay::kRows;
   double2* s_tab = s_vals + Lay::kGroups * Lay::kSlot;
-  for (int i = threadIdx.x; i < Lay::kRows; i += blockDim.x)
-    s_rows[i] = reinterpret_cast<const double2*>(n52 + KL)[i];
-  __syncthreads();
+  if constexpr (kL != kSplit) {
+    for (int i = threadIdx.x; i < Lay::kRows; i += blockDim.x)
+      s_rows[i] = reinterpret_cast<const double2*>(n52 + KL)[i];
+    __syncthreads();
+  }
   const long long first = block * IPB;
   {
     const int group = threadIdx.x / TPI;
     const long long inst = min(first + group, count - 1);  // idle groups repeat the last item
-    cuhe52::Pair52<KL, TPI> f;
-    double m[kL];
-#pragma unroll
-    for (int k = 0; k < kL; ++k) m[k] = __ldg(n52 + f.gl * kL + k);
     const PairExponent ex{ops, nullptr, nops, 0, 0};
-    (void)pair_power<KL, TPI, kEntry, false>(f, base + inst * K, K, s_rows,
-                                reinterpret_cast<const double2*>(n52 + KL) + (kEntry + 2) * KL,
-                                s_vals + group * Lay::kSlot, s_tab + threadIdx.x, m, f.gl == 0 ? ninv52 : 0ull, ex,
-                                mode == EXP_ENCRYPT ? aux + inst * K : nullptr);
+    if constexpr (kL == kSplit) {
+      (void)split_run<KL, kEntry, 1, false>(reinterpret_cast<double*>(smem), n52, 0, group, base + inst * K, K, ninv52,
+                                            ex, mode == EXP_ENCRYPT ? aux + inst * K : nullptr);
+    } else {
+      cuhe52::Pair52<KL, TPI> f;
+      double m[kL];
+#pragma unroll
+      for (int k = 0; k < kL; ++k) m[k] = __ldg(n52 + f.gl * kL + k);
+      (void)pair_power<KL, TPI, kEntry, false>(f, base + inst * K, K, s_rows,
+                                               reinterpret_cast<const double2*>(n52 + KL) + (kEntry + 2) * KL,
+                                               s_vals + group * Lay::kSlot, s_tab + threadIdx.x, m,
+                                               f.gl == 0 ? ninv52 : 0ull, ex,
+                                               mode == EXP_ENCRYPT ? aux + inst * K : nullptr);
+    }
   }
   __syncthreads();
   constexpr int LT = K / 16, L = 16, PER = cuhe52::kPairThreads / LT;

@@ -25,9 +25,10 @@ def _decrypt(c, e, mult, n):
 
 @pytest.mark.parametrize("bits,items", [(512, 32), (1024, 16), (2048, 8)])
 def test_batches_around_the_lanes_rule(bits, items):
-    """Counts of one item, a partial CTA, the last batch of the small rule
-    (items per CTA at five limbs a lane, one CTA on every SM) and the first
-    beyond it, for factors of `bits` bits at the top of their width."""
+    """Counts of one item, a partial CTA, the last batch with the components on
+    different lanes (half the items per CTA, one CTA on every SM) and the first
+    beyond it, the last batch of the small rule (items per CTA at five limbs a
+    lane) and the first beyond it, for factors of `bits` bits at the top of their width."""
     import torch
 
     from cuhepy_b200.paillier.gpu import PaillierDevice
@@ -46,7 +47,7 @@ def test_batches_around_the_lanes_rule(bits, items):
     powers = torch.from_numpy(ctx.limbs([pow(c, e, n * n) for c in base]).view(np.int32)).cuda()
     limbs = torch.from_numpy(ctx.limbs(base).view(np.int32)).cuda()
     edge = SMS * items
-    for count in (1, items + 1, edge, edge + 1):
+    for count in (1, items + 1, edge // 2, edge // 2 + 1, edge, edge + 1):
         rows = torch.arange(count, device="cuda") % len(base)
         c = limbs[rows].contiguous()
         out = torch.full_like(c, -1)
