@@ -60,6 +60,11 @@ BFV_SIGNATURES: dict[str, tuple] = {
                                         _vp]),
     "cuhe_bfv_encrypt_keyed": (ctypes.c_int, [_vp, ctypes.c_char_p, ctypes.c_uint64, _vp, ctypes.c_char_p,
                                               ctypes.c_char_p, ctypes.c_uint, ctypes.c_uint64, _vp]),
+    "cuhe_bfv_encrypt_parts": (ctypes.c_int, [_vp, ctypes.c_char_p, ctypes.c_uint64, _vp, _vp, _vp, ctypes.c_uint64,
+                                              ctypes.POINTER(_vp)]),
+    "cuhe_bfv_encrypt_keyed_parts": (ctypes.c_int, [_vp, ctypes.c_char_p, ctypes.c_uint64, _vp, ctypes.c_char_p,
+                                                    ctypes.c_char_p, ctypes.c_uint, ctypes.c_uint64,
+                                                    ctypes.POINTER(_vp)]),
     "cuhe_bfv_packed_search_parts": (ctypes.c_int, [_vp, ctypes.c_char_p, ctypes.POINTER(ctypes.c_char_p),
                                                     ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int, _vp,
                                                     ctypes.c_uint64, _u64p]),
@@ -441,6 +446,19 @@ def batch_encode(ring: Ring, t: int, slots):
     return out
 
 
+_bytes_new = ctypes.pythonapi.PyBytes_FromStringAndSize
+_bytes_new.restype, _bytes_new.argtypes = ctypes.py_object, [_vp, ctypes.c_ssize_t]
+_bytes_data = ctypes.pythonapi.PyBytes_AsString
+_bytes_data.restype, _bytes_data.argtypes = _vp, [ctypes.py_object]
+
+
+def _new_polys(count: int, size: int) -> tuple[list[bytes], Any]:
+    """`count` bytes objects of `size` (more than one) unset bytes and their
+    buffers' addresses, for a native call to fill before they are handed out."""
+    polys = [_bytes_new(None, size) for _ in range(count)]
+    return polys, (_vp * max(1, count))(*[_bytes_data(p) for p in polys])
+
+
 def encrypt_packed(ring: Ring, public_key: Any, t: int, slots, u, e) -> list[tuple[bytes, bytes]]:
     """Batched client encryption on the device (not in the reference ABI):
     public_key = (b, a) fixed-width polys; slots [count, N] (< t), u
@@ -458,13 +476,10 @@ def encrypt_packed(ring: Ring, public_key: Any, t: int, slots, u, e) -> list[tup
     count = slots.shape[0] if slots.ndim == 2 else -1
     if slots.shape != (count, ring.n) or u.shape != (count, ring.n) or e.shape != (count, 2, ring.n):
         raise ValueError("slots, u and e must be [count, N], [count, N] and [count, 2, N]")
-    size = (ring.n * ring.q_bits + 7) // 8
-    out = np.empty(max(1, count * 2 * size), dtype=np.uint8)  # filled by the call: no zeroing
-    _check(lib().cuhe_bfv_encrypt(ring.ptr, pk, int(t), slots.ctypes.data, u.ctypes.data, e.ctypes.data, count,
-                                  out.ctypes.data))
-    view = memoryview(out)
-    return [(bytes(view[2 * i * size:(2 * i + 1) * size]), bytes(view[(2 * i + 1) * size:(2 * i + 2) * size]))
-            for i in range(count)]
+    polys, parts = _new_polys(2 * count, (ring.n * ring.q_bits + 7) // 8)
+    _check(lib().cuhe_bfv_encrypt_parts(ring.ptr, pk, int(t), slots.ctypes.data, u.ctypes.data, e.ctypes.data, count,
+                                        parts))
+    return list(zip(polys[::2], polys[1::2]))
 
 
 def encrypt_packed_keyed(ring: Ring, public_key: Any, t: int, slots, key: bytes, nonce: bytes,
@@ -485,17 +500,14 @@ def encrypt_packed_keyed(ring: Ring, public_key: Any, t: int, slots, key: bytes,
     count = slots.shape[0] if slots.ndim == 2 else -1
     if slots.shape != (count, ring.n):
         raise ValueError("slots must be [count, N]")
-    size = (ring.n * ring.q_bits + 7) // 8
-    out = np.empty(max(1, count * 2 * size), dtype=np.uint8)
-    rc = lib().cuhe_bfv_encrypt_keyed(ring.ptr, pk, int(t), slots.ctypes.data, bytes(key), bytes(nonce), int(eta),
-                                      count, out.ctypes.data)
+    polys, parts = _new_polys(2 * count, (ring.n * ring.q_bits + 7) // 8)
+    rc = lib().cuhe_bfv_encrypt_keyed_parts(ring.ptr, pk, int(t), slots.ctypes.data, bytes(key), bytes(nonce),
+                                            int(eta), count, parts)
     if rc == CUHE_RANGE:
         message = lib().cuhe_bfv_last_error()
         raise KeystreamRejected(message.decode() if message else "keystream draw rejected")
     _check(rc)
-    view = memoryview(out)
-    return [(bytes(view[2 * i * size:(2 * i + 1) * size]), bytes(view[(2 * i + 1) * size:(2 * i + 2) * size]))
-            for i in range(count)]
+    return list(zip(polys[::2], polys[1::2]))
 
 
 def set_lanes(ring: Ring, lanes: int) -> None:

@@ -168,6 +168,14 @@ int cuhe_bfv_encrypt(cuhe_bfv_ring* ring, const uint8_t* pk, uint64_t t, const u
 int cuhe_bfv_encrypt_keyed(cuhe_bfv_ring* ring, const uint8_t* pk, uint64_t t, const uint32_t* slots,
                            const uint8_t* key, const uint8_t* nonce, unsigned eta, uint64_t count, uint8_t* out);
 
+/* Both with a buffer of its own for each of the count * 2 packed polys:
+ * callers that keep the polys apart save a copy of them. */
+int cuhe_bfv_encrypt_parts(cuhe_bfv_ring* ring, const uint8_t* pk, uint64_t t, const uint32_t* slots, const int8_t* u,
+                           const int8_t* e, uint64_t count, uint8_t* const* out);
+int cuhe_bfv_encrypt_keyed_parts(cuhe_bfv_ring* ring, const uint8_t* pk, uint64_t t, const uint32_t* slots,
+                                 const uint8_t* key, const uint8_t* nonce, unsigned eta, uint64_t count,
+                                 uint8_t* const* out);
+
 /* Execution lanes of a ring (1..8; 1 after create_ring).  Each lane is a
  * CUDA stream with its own device workspace.  packed_search / search_index
  * calls issued concurrently from several host threads take free lanes and
