@@ -756,11 +756,12 @@ int check_status(cuhe_paillier* ctx, bool synchronous) {
   return CUHE_OK;
 }
 
-int upload_schedule(cuhe_paillier* ctx, const Limbs& e, int32_t** dptr, int* nops, int window = 0) {
-  std::vector<int32_t> ops = cuhe::host::window_schedule(e, window ? window : ctx->window);
+int upload_schedule(cuhe_paillier* ctx, const Limbs& e, int32_t** dptr, int* nops, bool pairs = false) {
+  std::vector<int32_t> ops = cuhe::host::window_schedule(e, ctx->window);
+  *nops = int(ops.size());
+  if (pairs) ops = cuhe::host::pair_schedule(e, cuhe::kPairWindow, cuhe::kSplitWindow, nops);
   if (*dptr) cudaFree(*dptr);
   *dptr = nullptr;
-  *nops = int(ops.size());
   if (ops.empty()) return CUHE_OK;
   CUHE_CUDA(ctx, cudaMalloc(dptr, ops.size() * sizeof(int32_t)), "schedule allocation");
   CUHE_CUDA(ctx, cudaMemcpy(*dptr, ops.data(), ops.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
@@ -895,9 +896,9 @@ int setup_pair_crt(cuhe_paillier* ctx) {
     const std::vector<double> one = pair_constants(p, k, 4, ctx->have_secret ? &scale : nullptr);
     block.insert(block.end(), one.begin(), one.end());
     if (!ctx->have_secret) continue;
-    if (int rc = upload_schedule(ctx, main, &side.d_ops, &side.nops, cuhe::kPairWindow)) return rc;
+    if (int rc = upload_schedule(ctx, main, &side.d_ops, &side.nops, true)) return rc;
     if (side.halved)
-      if (int rc = upload_schedule(ctx, cofactor, &side.d_fall, &side.nfall, cuhe::kPairWindow)) return rc;
+      if (int rc = upload_schedule(ctx, cofactor, &side.d_fall, &side.nfall, true)) return rc;
   }
   return upload_constants(ctx, block, &ctx->d_crt52);
 }
@@ -1007,7 +1008,7 @@ int cuhe_paillier_create(const uint32_t* n_in, int n_words, int device, cuhe_pai
   ctx->stream = ctx->own_stream;
   ctx->pair_ninv = negative_inverse52(nk);
   if (upload_schedule(ctx, nk, &ctx->d_ops_n, &ctx->nops_n) != CUHE_OK ||
-      upload_schedule(ctx, nk, &ctx->d_ops_n52, &ctx->nops_n52, cuhe::kPairWindow) != CUHE_OK ||
+      upload_schedule(ctx, nk, &ctx->d_ops_n52, &ctx->nops_n52, true) != CUHE_OK ||
       setup_direct52(ctx) != CUHE_OK ||
       upload_constants(ctx, pair_constants(nk, 5 * k / 16, 2, nullptr), &ctx->d_pair) != CUHE_OK) {
     g_create_error = ctx->error;
@@ -1125,7 +1126,7 @@ int cuhe_paillier_set_secret(cuhe_paillier* ctx, const uint32_t* exponent, int e
   ctx->secret_exp = e;
   ctx->secret_mult = mult;
   ctx->have_secret = true;
-  if (int rc = upload_schedule(ctx, e, &ctx->d_ops_sec52, &ctx->nops_sec52, cuhe::kPairWindow)) return rc;
+  if (int rc = upload_schedule(ctx, e, &ctx->d_ops_sec52, &ctx->nops_sec52, true)) return rc;
   if (int rc = setup_pair_crt(ctx)) return rc;
   return upload_schedule(ctx, e, &ctx->d_ops_sec, &ctx->nops_sec);
 }
@@ -1462,7 +1463,10 @@ int cuhe_paillier_modexp(cuhe_paillier* ctx, const uint32_t* base, const uint32_
   Limbs e(exponent, exponent + exponent_words);
   while (e.size() > 1 && e.back() == 0) e.pop_back();
   const PairModexp f52 = pair_modexp(ctx);
-  std::vector<int32_t> ops = cuhe::host::window_schedule(e, f52 ? cuhe::kPairWindow : ctx->window);
+  int nops = 0;
+  std::vector<int32_t> ops = f52 ? cuhe::host::pair_schedule(e, cuhe::kPairWindow, cuhe::kSplitWindow, &nops)
+                                 : cuhe::host::window_schedule(e, ctx->window);
+  if (!f52) nops = int(ops.size());
   if (!ops.empty()) {
     if (cudaError_t ce = ctx->tmp_ops.reserve(ops.size() * 4)) return cuda_fail(ctx, ce, "schedule allocation");
     CUHE_CUDA(ctx, cudaMemcpyAsync(ctx->tmp_ops.ptr, ops.data(), ops.size() * 4, cudaMemcpyHostToDevice, ctx->stream),
@@ -1475,11 +1479,11 @@ int cuhe_paillier_modexp(cuhe_paillier* ctx, const uint32_t* base, const uint32_
   if (int rc = st.bind()) return rc;
   if (f52) {
     CUHE_CUDA(ctx, f52(ctx, (const uint32_t*)st.dev(0), nullptr, (uint32_t*)st.dev(1), count,
-                       (const int32_t*)ctx->tmp_ops.ptr, int(ops.size()), cuhe::EXP_POW, 0),
+                       (const int32_t*)ctx->tmp_ops.ptr, nops, cuhe::EXP_POW, 0),
               "modexp launch");
   } else {
     CUHE_CUDA(ctx, d.modexp(ctx, (const uint32_t*)st.dev(0), nullptr, (uint32_t*)st.dev(1), count,
-                            (const int32_t*)ctx->tmp_ops.ptr, int(ops.size()), cuhe::EXP_POW, 0),
+                            (const int32_t*)ctx->tmp_ops.ptr, nops, cuhe::EXP_POW, 0),
               "modexp launch");
   }
   if (int rc = st.finish()) return rc;

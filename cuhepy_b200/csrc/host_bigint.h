@@ -199,5 +199,31 @@ inline std::vector<int32_t> window_schedule(const Limbs& e, int window) {
   return ops;
 }
 
+// The schedule of `window` bits for the kernels with a table of that width,
+// and behind it, for those with a table of up to 2^(widest - 1) odd powers,
+// another: its op count, the odd powers it uses (1 to the largest), its ops.
+// That is the width with the fewest products, the table's included.
+inline std::vector<int32_t> pair_schedule(const Limbs& e, int window, int widest, int* nops) {
+  std::vector<int32_t> ops = window_schedule(e, window), best;
+  *nops = int(ops.size());
+  if (ops.empty()) return ops;
+  size_t least = SIZE_MAX;
+  int odd = 0;
+  for (int w = window; w <= widest; ++w) {
+    std::vector<int32_t> wide = window_schedule(e, w);
+    int top = 1;
+    for (int32_t op : wide) top = (op & 0xffff) > top ? (op & 0xffff) : top;
+    if (wide.size() + size_t(top) < least) {
+      least = wide.size() + size_t(top);
+      best = std::move(wide);
+      odd = top;
+    }
+  }
+  ops.push_back(int32_t(best.size()));
+  ops.push_back(odd);
+  ops.insert(ops.end(), best.begin(), best.end());
+  return ops;
+}
+
 }  // namespace host
 }  // namespace cuhe

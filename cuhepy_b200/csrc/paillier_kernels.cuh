@@ -800,6 +800,10 @@ __device__ __forceinline__ void pair_words(const Group<K, TPI>& g, uint32_t (&x)
 
 // kL of the split form (pair52_split.cuh), whose layout is a specialisation.
 constexpr int kSplit = -5;
+// Its table holds up to 16 odd powers (80 KB, one CTA per SM), as many as the
+// exponent's wide schedule uses (host pair_schedule, behind the other's ops):
+// at |e| = 279 four-bit windows, from some 500 bits on five.
+constexpr int kSplitWindow = 5;
 
 template <int K, int kL, int kEntry, int kSides>
 struct PairLayout {  // K limbs per component (kL per lane), kSides moduli per item

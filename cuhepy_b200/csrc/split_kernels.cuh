@@ -16,13 +16,13 @@ struct PairLayout<K, kSplit, kEntry, kSides> {
   static constexpr int kRows = (kEntry + 2) * (K + 4);       // constants per modulus, in pairs of doubles
   static constexpr int kSlot = K + 1;
   // doubles: the powers of one component per thread; the operands, and zeros
-  static constexpr size_t kTab = size_t(kPairTable) * L * cuhe52::kPairThreads;
+  static constexpr size_t kTab = size_t(1 << (kSplitWindow - 1)) * L * cuhe52::kPairThreads;
   static constexpr size_t kWork = size_t(3 * kGroups + 1) * (K + 4);
   static constexpr size_t kBytes = (size_t(kSides) * kRows + size_t(kGroups) * kSlot) * 16 + (kTab + kWork) * 8;
 };
 
 // pair_power with the components on different lanes (pair52_split.cuh): the
-// same schedule and results.  rows: the constants' arrays in shared memory
+// same results, by the exponent's wide schedule.  rows: the constants' arrays in shared memory
 // (split_rows: kEntry entry rows of two components, then (1, 0)'s component 0
 // twice, then the scale row), zeros: kOperand zeros; work: this value's three
 // operand arrays (z0, 2 z0, t0), whose two leading limbs are zero; s: its K
@@ -76,6 +76,10 @@ __device__ __forceinline__ bool split_power(const cuhe52::Split52<K, TPI>& f, co
         z[k] = f.half ? v.y : v.x;
       }
     } else {
+      const int32_t* wide = ops + nops;  // op count, odd powers, ops
+      const int odd = __ldg(wide + 1);
+      nops = __ldg(wide);
+      ops = wide + 2;
       // x to the table and x^2 to z, then x^(2i+1) = x^(2i-1) x^2 in t
 #pragma unroll
       for (int k = 0; k < L; ++k) {
@@ -94,7 +98,7 @@ __device__ __forceinline__ bool split_power(const cuhe52::Split52<K, TPI>& f, co
       publish(zarr, z);
       __syncwarp();
 #pragma unroll 1
-      for (int i = 1; i < kPairTable; ++i) {
+      for (int i = 1; i < odd; ++i) {
         f.template product<true>(A, t, z, f.operand(zarr), f.half ? tarr : zeros, m);
         f.f.template limbs<3>(t, A);
         __syncwarp();
