@@ -338,10 +338,14 @@ def run_gpu(args) -> dict | None:
     imad_peak = ctypes_imad_peak(_native, local)
     k = words
     kh = k // 2
-    k52 = 5 * kh // 8
+    kl = 5 * kh // 16  # 52-bit limbs of a residue mod p
     a_bits = int(sk["a"]).bit_length()
     mm = a_bits + math.ceil(a_bits / 6) + 16
-    fp64_per_decode = 2 * mm * (2 * k52 * k52 + k52) * 3   # three FP64 instructions per 52x52-bit limb product
+    squarings, products = window_products(int(sk["a"]), 3)
+    # beside the windows: four entry chunks, x^2 and the scaling (4 kl^2 limb
+    # products each, as a squaring), three odd powers and the way out (5 kl^2)
+    limb_products = (squarings + 6) * 4 * kl * kl + (products + 4) * 5 * kl * kl
+    fp64_per_decode = 2 * limb_products * 3                # three FP64 instructions per 52x52-bit limb product
     wp_per_decode = 2 * mm * (2 * kh * kh + kh)            # the same products as 32x32-bit word products
     decode_ms = statistics.mean(kernel_ms["decode"])
     decodes = QUERY_BATCH * INDEX_VECTORS
@@ -377,29 +381,29 @@ def run_gpu(args) -> dict | None:
         "decode_direct_ms": statistics.mean(direct_ms),
         "decode_compare": ("the same decode batch outside the timed steps: decode_int_ms on the integer-pipe CRT "
                            "kernel k_modexp_crt<64,8,4>, decode_direct_ms without the factors (c^a mod n^2 itself, "
-                           "k_modexp52 on the FP64 pipe)"),
+                           "k_pair_modexp on the FP64 pipe)"),
         "p50_ms": statistics.median(step_ms),
         "p99_ms": float(np.percentile(step_ms, 99)),
         "plain_value": plain_value,
         "plain": "decode one ciphertext per launch (batch 1), host-synchronised",
         "roofline": {
             "bound": "fp64",
-            "kernel": ("k_modexp_crt52<64,3> decode (c^a mod p^2 and mod q^2 as 40 52-bit limbs, |a|=%d bits, "
-                       "on the FP64 pipe)" % a_bits),
+            "kernel": ("k_pair_crt<64,10> decode (c^a mod p^2 and mod q^2 as pairs of residues mod p and mod q, "
+                       "%d 52-bit limbs each, |a|=%d bits, on the FP64 pipe)" % (kl, a_bits)),
             "achieved": achieved / 1e12, "peak": fp64_peak / 1e12, "unit": "T fp64 instr/s",
             "frac": achieved / fp64_peak, "traffic": traffic,
             "peak_nominal": nominal_fp64 / 1e12, "frac_of_nominal": achieved / nominal_fp64,
             "peak_source": "measured by cuhe_fp64_peak in this run (independent fma.rz.f64 chains)",
             "peak_nominal_source": "SMs x 64 FP64 FMA/clk x median SM clock",
             "traffic_source": "ncu dram bytes of an 8,192-decode launch, scaled by decodes per launch",
-            "work_per_unit": (f"2 sides x MM(e)=e+ceil(e/6)+16={mm} modmuls x (2K52^2+K52)={2 * k52 * k52 + k52} "
-                              f"limb products x 3 FP64 instructions, K52={k52} (recombination and epilogue on the "
-                              f"integer pipe, under 2%, not counted)"),
+            "work_per_unit": (f"2 sides x ({squarings + 6} products of 4K^2 + {products + 4} of 5K^2)={limb_products} "
+                              f"limb products x 3 FP64 instructions, K={kl} (the epilogue on the integer pipe, "
+                              f"about a tenth of the time, not counted)"),
             "as_word_products": {
                 "achieved": achieved_wp / 1e12, "unit": "Twp/s",
                 "imad_peak_measured": imad_peak / 1e12, "frac_of_measured_imad": achieved_wp / imad_peak,
                 "imad_peak_nominal": nominal_imad / 1e12, "frac_of_nominal_imad": achieved_wp / nominal_imad,
-                "note": (f"the same decode counted as 2 x {mm} x (2kh^2+kh)={2 * kh * kh + kh} 32-bit word products, "
+                "note": (f"the same decode counted as full-width products, 2 x {mm} x (2kh^2+kh)={2 * kh * kh + kh} 32-bit word products, "
                          f"kh={kh}, against the integer multiply pipe's measured and nominal rates"),
             },
         },
@@ -559,15 +563,18 @@ def run_bfv(steps: int, warmup: int, cpu: bool, native: bool = False) -> dict:
         m.hamming_tile(relin, qf, qf, rot, mask, BFV_T)
     per_tile = (time.perf_counter() - t0) / plain_tiles
     tiles = len(index)
-    # algorithmic work per query (the counts of bfv_server.h's circuit, which
-    # this implementation follows transform for transform): per tile 200
-    # forward and 87 inverse N-point transforms, per merge 18 and 6.  Native
-    # rings: T tensor, S switch and M mask primes, D digits, R rotations per
-    # tile: forward 2T + (1 + R) D S + 2M, inverse 3T + (1 + R) 2S + 2M;
-    # per merge D S and 2S.
+    # transforms per query.  Residue rings keep ciphertexts in the NTT domain
+    # through the rotations and merges (T tensor primes 7, L residue primes 3,
+    # D digits 6, R rotations 9): per tile 2T and 3T for the tensor, 3L to
+    # bring the relinearisation's input over, and per switch (D - 1) L forward
+    # and L inverse (component 1's coefficients for the next); per merge one
+    # switch; per response 2L inverse.  (The circuit with coefficient-domain
+    # switches, bfv_server.h's, takes 200 and 87 per tile, 18 and 6 per merge.)
+    # Native rings: T tensor, S switch and M mask primes: forward
+    # 2T + (1 + R) D S + 2M, inverse 3T + (1 + R) 2S + 2M; per merge D S and 2S.
     groups = (tiles + layout.padded - 1) // layout.padded
     merges = tiles - groups
-    fwd, inv = 200 * tiles + 18 * merges, 87 * tiles + 6 * merges
+    fwd, inv = 173 * tiles + 15 * merges, 51 * tiles + 3 * merges + 6 * groups
     info = m.ring_info(ring)
     if native:
         T, S, D, R = len(info["primes"]), info["switch_prime_count"], 6, len(layout.left())
@@ -595,7 +602,7 @@ def run_bfv(steps: int, warmup: int, cpu: bool, native: bool = False) -> dict:
     nominal = sms * 64 * (clock.get("sm_mhz") or 1965.0) * 1e6 / 2
     out_roofline = {
         "bound": "imad",
-        "kernel": "whole search (k_keyswitch_tm<3, 16>, the key switch, ~78% of the search kernel time in the ncu launch list)",
+        "kernel": "whole search (k_rotate_tm<3, 16>, the NTT-domain rotations and key switches, ~70% of the search kernel time)",
         "transforms_per_query": fwd + inv, "butterflies_per_query": butterflies,
         "achieved": butterflies * 10 / step_s / 1e12, "peak": imad / 1e12, "unit": "Twp/s",
         "frac": butterflies * 10 / step_s / imad,
@@ -721,11 +728,32 @@ def ctypes_imad_peak(native, device: int) -> float:
     return out.value
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one k_modexp_crt52<64,3>
-# decode launch of 8,192 ciphertexts (ncu, key_len 1024): 4,491,776 + 0
+# dram__bytes_read.sum + dram__bytes_write.sum of one k_pair_crt<64,10>
+# decode launch of 8,192 ciphertexts (ncu, key_len 1024): 4,556,032 + 0
 # bytes.  Each ciphertext is read once, so the traffic of a larger launch
 # scales with the number of decodes.
-DECODE_TRAFFIC_BYTES, DECODE_TRAFFIC_ITEMS = 4_491_776, 8192
+DECODE_TRAFFIC_BYTES, DECODE_TRAFFIC_ITEMS = 4_556_032, 8192
+
+
+def window_products(e: int, width: int) -> tuple[int, int]:
+    """Squarings and products of e's sliding windows of up to `width` bits,
+    from the top, each ending in a one."""
+    squarings = products = 0
+    top = e.bit_length() - 1
+    i = top
+    while i >= 0:
+        if not e >> i & 1:
+            squarings += 1
+            i -= 1
+            continue
+        low = max(0, i - width + 1)
+        while not e >> low & 1:
+            low += 1
+        if i != top:
+            squarings += i - low + 1
+            products += 1
+        i = low - 1
+    return squarings, products
 
 
 def ncu_traffic(items: int) -> float:
@@ -1313,7 +1341,7 @@ def profile_case(which: str) -> None:
     if which in ("paillier", "paillier_int"):
         from cuhepy_b200.paillier.gpu import PaillierDevice
 
-        keys = seeded_lookup_keys(0)  # k_modexp_crt52 (k_modexp_crt: paillier_int) serves only the decodes
+        keys = seeded_lookup_keys(0)  # k_pair_crt (k_modexp_crt: paillier_int) serves only the decodes
         pk, sk = keys["pk"], keys["sk"]
         ctx = PaillierDevice(pk["n"])
         ctx.set_secret(sk["a"], sk["g_a_inv"])

@@ -14,11 +14,11 @@ stream, the NTT batches forked onto a second stream so that the two kinds
 overlap, joined back before the graph ends.  ``replay()`` is then a single
 launch from the host.
 
-A width whose contexts select the FP64 pipe (n^2 of 4096 or 8192 bits by
-default, ``PaillierDevice.set_fp64``) runs the persistent kernel of 52-bit-limb
-products on that pipe, as those contexts' own calls do.  The autotuner picks,
+A width whose contexts select the FP64 pipe (n^2 of 2048, 4096 or 8192
+bits by default, ``PaillierDevice.set_fp64``) runs the persistent kernel of
+limb pairs on that pipe, as those contexts' own calls do.  The autotuner picks,
 per Paillier width, the (threads per instance, window) variant of the integer
-kernel or, for those widths, the FP64 kernel, whichever finishes that width's
+kernel or the FP64 kernel, whichever finishes that width's
 own batches fastest (and sets the contexts' pipe accordingly), and per ring
 the (threads per CTA, radix) of its NTT batches, by timing the candidates on
 the batch's own data with CUDA events.
@@ -265,16 +265,14 @@ class MixedBatch:
                     e.ctx.set_fp64(0)
                 for tpi, w in PaillierDevice.VARIANTS[words]:
                     timings[(tpi, w)] = timed({words: (tpi, w)})
-                if words >= 128:  # the FP64-pipe kernel's widths
-                    for e in entries:
-                        e.ctx.set_fp64(1)
-                    timings["fp64"] = timed({})
+                for e in entries:
+                    e.ctx.set_fp64(1)
+                timings["fp64"] = timed({})
             finally:
                 for e, f in zip(entries, saved):
                     e.ctx.set_fp64(f)
             best = min(timings, key=timings.get)
-            if words >= 128:
-                self.paillier_fp64[words] = best == "fp64"
+            self.paillier_fp64[words] = best == "fp64"
             if best == "fp64":
                 self.paillier_tuning.pop(words, None)
             else:

@@ -1,4 +1,6 @@
-// Warp-cooperative Montgomery arithmetic on the FP64 pipe, for sm_100a.
+// Warp-cooperative Montgomery arithmetic on the FP64 pipe, for sm_100a: single
+// products of unrelated values mod n^2 (the server's outer products), where
+// entering and leaving the pairs of pair52.cuh would cost more than they save.
 //
 // The integer multiply pipe (fmaheavy) is the bound of the 32-bit-limb CIOS
 // in bigint_group.cuh: every 32x32 word product costs a mad.lo and a mad.hi.

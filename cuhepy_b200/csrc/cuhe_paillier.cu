@@ -236,7 +236,8 @@ bool pair_small(const cuhe_paillier* ctx, long long count, int items10) {
 // items10, again one warp to a scheduler) run with the components on
 // different lanes: 1,184 decodes at key_len 1024 take 0.90 ms against 1.21
 // with five limbs a lane, 592 encryptions at key_len 2048 37.1 against 52.9.
-// One item more, two CTAs to an SM, 1.49 against 1.21 and 66.4 against 52.9.
+// One item more, two CTAs to an SM, 1.49 against 1.21 and 66.4 against 52.9
+// (all with three-bit windows; the split kernels' own take another 5 and 6%).
 bool pair_tiny(const cuhe_paillier* ctx, long long count, int items10) {
   return count <= (long long)ctx->sms * items10 / 4;
 }

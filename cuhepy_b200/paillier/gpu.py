@@ -104,9 +104,10 @@ class PaillierDevice:
         return bool(self._lib.cuhe_paillier_has_factors(self._ctx))
 
     def set_fp64(self, enable: int) -> None:
-        """CRT exponentiations as 52-bit-limb products on the FP64 pipe for n^2
-        of 4096 bits or more (1, the default; 2: also for 2048 bits) or as
-        32-bit word products on the integer pipe (0); identical results."""
+        """Exponentiations and lookup encryptions on pairs of residues on the
+        FP64 pipe (1, the default; 2: also the server's products of n^2 of 2048
+        bits, which else take it from 4096) or everything as 32-bit word
+        products on the integer pipe (0); identical results."""
         self._check(self._lib.cuhe_paillier_set_fp64(self._ctx, int(enable)))
 
     @property

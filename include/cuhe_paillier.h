@@ -81,17 +81,16 @@ int cuhe_paillier_set_factors(cuhe_paillier* ctx, const uint32_t* p, int p_words
 int cuhe_paillier_has_factors(const cuhe_paillier* ctx);
 
 /* Pipe of the exponentiations.  With enable = 1 (the default), keys with n^2
- * of 4096 or 8192 bits run them as Montgomery products of 52-bit limbs on the
- * FP64 pipe (three exact FP64 instructions per 52x52-bit product, sums in
- * 64-bit integers, ten limbs per lane, a 3-bit window): decrypt / decode by
- * the CRT when the factors are installed (both half-width exponentiations),
- * and otherwise mod n^2 itself, as do encryption (r^n), cuhe_paillier_modexp
- * and mixed batches (cuhe_mix_plan, per width whose contexts all select it).
- * Entry and exit go through 32-bit Montgomery products and the same
- * recombination and epilogues, so results are identical to the integer-pipe
- * kernels.  n^2 of 2048 bits stays on the integer pipe (measured faster
- * there) unless enable = 2; enable = 0 keeps every product on the integer
- * pipe.  get returns the setting.  No reference counterpart (the reference's
+ * of 2048, 4096 or 8192 bits run them on the FP64 pipe, a value mod m^2 held
+ * as a pair of residues mod m in 52-bit limbs (three exact FP64 instructions
+ * per 52x52-bit product, sums in 64-bit integers): decrypt / decode by the
+ * CRT when the factors are installed (pairs mod p and mod q), and otherwise
+ * pairs mod n, as do encryption (r^n), the lookup encryption's table
+ * products, cuhe_paillier_modexp and mixed batches (cuhe_mix_plan, per width
+ * whose contexts all select it).  Results are identical to the integer-pipe
+ * kernels.  The server's products (cuhe_paillier_mulmod_outer) take that pipe
+ * from n^2 of 4096 bits, and at 2048 bits with enable = 2; enable = 0 keeps
+ * every product on the integer pipe.  get returns the setting.  No reference counterpart (the reference's
  * CGBN kernels multiply 32-bit words on the integer pipe). */
 int cuhe_paillier_set_fp64(cuhe_paillier* ctx, int enable);
 int cuhe_paillier_get_fp64(const cuhe_paillier* ctx);
@@ -212,21 +211,24 @@ int cuhe_lookup_encrypt_bits(cuhe_paillier* ctx, const uint8_t* bits, int64_t ve
  * looked up as one entry W[j][D] = G[2j][D mod 256] * G[2j+1][D / 256] (mod
  * n^2, Montgomery form), so each ciphertext takes half the table products and
  * the ciphertexts are the same.  The table holds (message_chunks + 1) / 2 *
- * 65,536 entries, K words each (4 GiB at key_len 1024), or 5K/8 doubles each
- * when the FP64 pipe is selected (cuhe_paillier_set_fp64; 5 GiB at key_len
- * 1024, with the noise table converted likewise, and the products then run
- * on that pipe), and costs one or two products per entry to build, which
- * about 150,000 encryptions repay.  mode 1 (the
+ * 65,536 entries of K words (4 GiB at key_len 1024) and costs a product per
+ * entry to build, which about 150,000 encryptions repay.  When the FP64 pipe
+ * is selected (cuhe_paillier_set_fp64) the entries are limb pairs of 5K/8
+ * doubles; embeddings in chunks of an even length are then looked up by 8 or
+ * 16 bits of the embedding itself (two plaintext bits each), a quarter as
+ * many rows, and only the rows that the calls' embeddings reach are built
+ * (1.25 GiB for 512-bit embeddings at key_len 1024); words and odd chunk
+ * lengths use the pairs of plaintext digits.  A call of 8,192 ciphertexts or
+ * more also builds the products of all pairs of noise entries.  mode 1 (the
  * default) builds it during an encryption call of at least 65,536
  * ciphertexts, when it takes at most 8 GiB and a quarter of the free device
  * memory; mode 2 builds it at the next encryption call of any size
  * (CUHE_OUT_OF_MEMORY without the memory); mode 0 frees it and keeps the
  * 8-bit table.  Installing new tables drops it.  The table is built for the
- * pipe selected at that time.  If cuhe_paillier_set_fp64 later selects the
- * other pipe, the table is kept; FP64-form limbs are then left unused and the
- * 8-bit table serves, while a word table still serves the FP64 selection on
- * the integer pipe.  Call mode 0, then mode 2, to rebuild it for the new
- * pipe.  ready returns 1 once it is built.  No reference counterpart (the
+ * pipe selected at that time and is kept, unused, while the other pipe is
+ * selected, which builds its own by the same rule.  Without memory for the
+ * limb pairs a call runs on the integer pipe; inside a stream capture nothing
+ * is built and the tables that are there serve.  ready returns 1 once it is built.  No reference counterpart (the
  * reference multiplies one entry per 8-bit digit, lookup.py:213-252). */
 int cuhe_lookup_set_wide_table(cuhe_paillier* ctx, int mode);
 int cuhe_lookup_wide_table_ready(const cuhe_paillier* ctx);
