@@ -130,22 +130,29 @@ struct cuhe_paillier {
     double2* noise = nullptr;   // [noise_entries]
     double2* noise2 = nullptr;  // [noise_entries][noise_entries]: products of two
     double2* wide_digits = nullptr;  // [ceil(message_chunks / 2)][65536]: 16-bit digits
-    double2* wide_embed = nullptr;   // [wide_rows][65536]: 16 embedding bits
+    // Rows of 65,536 entries by 16 embedding bits, as far as calls reached.
+    // Rows are added and never moved, nor is the device array of their
+    // addresses: calls captured in a graph read both at every replay.
+    std::vector<double2*> wide_blocks;      // each growth's allocation
+    const double2** embed_rows = nullptr;   // [ceil(message_chunks / 4)], wide_rows of them set
     int wide_rows = 0;
     void release() {
-      for (double2** p : {&digits, &embed, &noise, &noise2, &wide_digits, &wide_embed}) {
+      for (double2** p : {&digits, &embed, &noise, &noise2}) {
         cudaFree(*p);
         *p = nullptr;
       }
-      wide_rows = 0;
+      release_wide();
     }
     void release_wide() {
       cudaFree(wide_digits);
-      cudaFree(wide_embed);
-      wide_digits = wide_embed = nullptr;
+      wide_digits = nullptr;
+      for (double2* block : wide_blocks) cudaFree(block);
+      wide_blocks.clear();
+      cudaFree(embed_rows);
+      embed_rows = nullptr;
       wide_rows = 0;
     }
-    bool wide() const { return wide_digits || wide_embed; }
+    bool wide() const { return wide_digits || wide_rows; }
   } pt;
   double2* d_entry = nullptr;  // k_pair_rows' constants
   int wide_mode = 1;           // 0 never, 1 for large batches when it fits, 2 always
@@ -1881,6 +1888,36 @@ int ensure_wide_table(cuhe_paillier* ctx, const Dispatch& d, long long items) {
 // saved by a ciphertext) from this many ciphertexts in one call.
 constexpr long long kNoisePairItems = 8192;
 
+// Rows [wide_rows, need) of the 16-bit embedding table (of the 8-bit table's
+// rows8), in an allocation of their own.  Without memory for them the table
+// stays as it is (CUHE_OUT_OF_MEMORY in mode 2).
+int grow_embed_rows(cuhe_paillier* ctx, const PairLookup& pl, int rows8, int need) {
+  auto& pt = ctx->pt;
+  const int before = pt.wide_rows, added = need - before;
+  const size_t entries = size_t(5 * ctx->K / 16) * 65536;  // pairs of a row
+  double2* block = nullptr;
+  cudaError_t e = pt.embed_rows ? cudaSuccess : cudaMalloc(&pt.embed_rows, size_t((rows8 + 1) / 2) * sizeof(double2*));
+  if (e == cudaSuccess) e = cudaMalloc(&block, size_t(added) * entries * sizeof(double2));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return ctx->wide_mode == 2 ? fail(ctx, CUHE_OUT_OF_MEMORY, "wide table allocation") : CUHE_OK;
+  }
+  std::vector<const double2*> rows;
+  for (int r = 0; r < added; ++r) rows.push_back(block + size_t(r) * entries);
+  e = pl.products(ctx, pt.embed, rows8, cuhe::kWide, (long long)before * 65536, (long long)added * 65536, block);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(pt.embed_rows + before, rows.data(), rows.size() * sizeof(double2*), cudaMemcpyHostToDevice,
+                        ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) {
+    cudaFree(block);
+    return cuda_fail(ctx, e, "wide table build");
+  }
+  pt.wide_blocks.push_back(block);
+  pt.wide_rows = need;
+  return CUHE_OK;
+}
+
 // Encryption from the limb-pair tables, building those the call needs; *done
 // is false (nothing launched) when they do not fit in device memory.
 int pair_lookup_encrypt(cuhe_paillier* ctx, const PairLookup& pl, cuhe::LookupDigits dg, long long count,
@@ -1908,34 +1945,14 @@ int pair_lookup_encrypt(cuhe_paillier* ctx, const PairLookup& pl, cuhe::LookupDi
     const int need8 = std::min(rows8, (reach + 15) / 16), need = (need8 + 1) / 2;
     if (pt.wide_rows < need && !capturing(ctx)) {
       if (int rc = wide_allowed(ctx, count, size_t(need) * 65536 * row_bytes, &allowed)) return rc;
-      if (allowed) {
-        double2* wide = nullptr;
-        const int before = pt.wide_rows;
-        if (cudaMalloc(&wide, size_t(need) * 65536 * row_bytes) != cudaSuccess) {
-          cudaGetLastError();
-          if (ctx->wide_mode == 2) return fail(ctx, CUHE_OUT_OF_MEMORY, "wide table allocation");
-        } else {
-          cudaError_t e = before ? cudaMemcpyAsync(wide, pt.wide_embed, size_t(before) * 65536 * row_bytes,
-                                                   cudaMemcpyDeviceToDevice, ctx->stream)
-                                 : cudaSuccess;
-          if (e == cudaSuccess)
-            e = pl.products(ctx, pt.embed, rows8, cuhe::kWide, (long long)before * 65536,
-                            (long long)(need - before) * 65536, wide);
-          if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-          if (e != cudaSuccess) {
-            cudaFree(wide);
-            return cuda_fail(ctx, e, "wide table build");
-          }
-          cudaFree(pt.wide_embed);
-          pt.wide_embed = wide;
-          pt.wide_rows = need;
-        }
-      }
+      if (allowed)
+        if (int rc = grow_embed_rows(ctx, pl, rows8, need)) return rc;
     }
-    const bool wide = pt.wide_rows >= need && pt.wide_embed;
+    const bool wide = pt.wide_rows >= need && pt.wide_rows;
     dg.embed_bits = wide ? 16 : 8;
     dg.rows = wide ? need : need8;
-    table = wide ? pt.wide_embed : pt.embed;
+    dg.embed_rows = wide ? pt.embed_rows : nullptr;
+    table = pt.embed;
   } else {
     const int rows = (chunks + 1) / 2;
     if (!pt.wide_digits && !capturing(ctx)) {

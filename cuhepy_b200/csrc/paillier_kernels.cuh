@@ -1750,7 +1750,8 @@ k_pair_rows(const uint32_t* __restrict__ in, long long count, double2* __restric
 //           8-bit table at the bits of b spread to the even places
 //   kWide   row j = i / 65536 of 16 bits D: rows 2j and 2j + 1 at D's bytes
 //   kNoise  i = a entries + b: noise entries a and b
-// A factor past the source's last row is one.
+// A factor past the source's last row is one.  Entries [first, first + count)
+// of the whole table, from the start of out.
 enum PairProducts : int { kEmbed = 0, kWide = 1, kNoise = 2 };
 
 __device__ __forceinline__ int spread4(int b) { return (b & 1) | (b & 2) << 1 | (b & 4) << 2 | (b & 8) << 3; }
@@ -1797,7 +1798,7 @@ k_pair_products(const double2* __restrict__ src, int rows, int kind, long long f
   f.template limbs<3>(a1, A1);
   if (item >= first + count) return;
 #pragma unroll
-  for (int k = 0; k < L; ++k) out[item * KL + pair_row_slot<KL, L>(f.gl, k)] = make_double2(a0[k], a1[k]);
+  for (int k = 0; k < L; ++k) out[(item - first) * KL + pair_row_slot<KL, L>(f.gl, k)] = make_double2(a0[k], a1[k]);
 }
 
 // How a ciphertext's rows are found.
@@ -1809,6 +1810,7 @@ struct LookupDigits {
   int wide;               // 16-bit digits
   int rows;               // rows of the table
   int message_chunks;     // 8-bit plaintext digits the tables cover
+  const double2* const* embed_rows;  // 16 embedding bits: each row's 65,536 entries, in place of one table
 };
 
 __device__ __forceinline__ int lookup_digit(const LookupDigits& d, long long inst, int r) {
@@ -1896,7 +1898,10 @@ k_pair_lookup(LookupDigits dg, long long count, const double2* __restrict__ tabl
       return t;
     };
     auto row = [&](int t) -> const double2* {
-      if (t < dg.rows) return table + ((static_cast<long long>(t) << digit_bits) + digits[t]) * KL;
+      if (t < dg.rows) {
+        if (dg.embed_rows) return dg.embed_rows[t] + static_cast<long long>(digits[t]) * KL;
+        return table + ((static_cast<long long>(t) << digit_bits) + digits[t]) * KL;
+      }
       const int k = t - dg.rows;
       if (!valid) return noise;
       if (noise_pairs) return noise + (static_cast<long long>(idx[2 * k]) * noise_entries + idx[2 * k + 1]) * KL;

@@ -228,8 +228,11 @@ int cuhe_lookup_encrypt_bits(cuhe_paillier* ctx, const uint8_t* bits, int64_t ve
  * pipe selected at that time and is kept, unused, while the other pipe is
  * selected, which builds its own by the same rule.  Without memory for the
  * limb pairs a call runs on the integer pipe; inside a stream capture nothing
- * is built and the tables that are there serve.  ready returns 1 once it is built.  No reference counterpart (the
- * reference multiplies one entry per 8-bit digit, lookup.py:213-252). */
+ * is built and the tables that are there serve.  Rows are added and never
+ * moved: an encryption captured in a graph can be replayed until mode 0, new
+ * tables or the end of the context free what it reads.  ready returns 1 once
+ * it is built.  No reference counterpart (the reference multiplies one entry
+ * per 8-bit digit, lookup.py:213-252). */
 int cuhe_lookup_set_wide_table(cuhe_paillier* ctx, int mode);
 int cuhe_lookup_wide_table_ready(const cuhe_paillier* ctx);
 
