@@ -374,11 +374,12 @@ Outer52 outer52(const cuhe_paillier* ctx) {
 // Rows of limb pairs for the lookup encryption (k_pair_rows, k_pair_products)
 // and encryption from them (k_pair_lookup).
 template <int K>
-cudaError_t launch_pair_rows(cuhe_paillier* ctx, const uint32_t* in, long long count, double2* out) {
+cudaError_t launch_pair_rows(cuhe_paillier* ctx, const uint32_t* in, long long count, bool digits, double2* out) {
   constexpr int KL = 5 * K / 16, IPB = cuhe52::kPairThreads / (KL / 10);
   const size_t smem = size_t(2 * KL + 1) * 16;
   cuhe::k_pair_rows<K><<<dim3(unsigned((count + IPB - 1) / IPB)), cuhe52::kPairThreads, smem, ctx->stream>>>(
-      in, count, out, ctx->d_entry, ctx->d_pair, ctx->pair_ninv);
+      in, count, digits ? ctx->d_consts + size_t(cuhe::C_RM) * K : nullptr, out, ctx->d_entry, ctx->d_pair,
+      ctx->pair_ninv);
   return cudaGetLastError();
 }
 
@@ -417,7 +418,7 @@ cudaError_t launch_pair_lookup(cuhe_paillier* ctx, const cuhe::LookupDigits& dg,
 }
 
 struct PairLookup {
-  cudaError_t (*rows)(cuhe_paillier*, const uint32_t*, long long, double2*);
+  cudaError_t (*rows)(cuhe_paillier*, const uint32_t*, long long, bool, double2*);
   cudaError_t (*products)(cuhe_paillier*, const double2*, int, int, long long, long long, double2*);
   cudaError_t (*launch)(cuhe_paillier*, const cuhe::LookupDigits&, long long, const double2*, const double2*, bool,
                         const uint8_t*, uint32_t*);
@@ -525,7 +526,8 @@ cudaError_t launch_lookup(cuhe_paillier* ctx, const uint8_t* bits, int embed_len
   return cudaGetLastError();
 }
 
-// W[j][D] = G[2j][D mod 256] * G[2j+1][D / 256] for every 16-bit D.
+// W[j][D] = G[2j][D mod 256] * G[2j+1][D / 256] for every 16-bit D, entries of
+// the digit zero taken as one.
 template <int K, int TPI>
 cudaError_t launch_wide_table(cuhe_paillier* ctx, uint32_t* wide) {
   constexpr int IPB = cuhe::kBlockThreads / TPI;
@@ -1715,10 +1717,11 @@ int pair_tables(cuhe_paillier* ctx, const PairLookup& pl) {
     if (int rc = upload_constants(ctx, block, reinterpret_cast<double**>(&ctx->d_entry))) return rc;
   }
   if (int rc = pair_table(ctx, &pt.digits, (long long)chunks * 256, [&](double2* t) {
-        return pl.rows(ctx, ctx->d_gtab, (long long)chunks * 256, t);
+        return pl.rows(ctx, ctx->d_gtab, (long long)chunks * 256, true, t);
       }))
     return rc;
-  if (int rc = pair_table(ctx, &pt.noise, entries, [&](double2* t) { return pl.rows(ctx, ctx->d_noise, entries, t); }))
+  if (int rc = pair_table(ctx, &pt.noise, entries,
+                          [&](double2* t) { return pl.rows(ctx, ctx->d_noise, entries, false, t); }))
     return rc;
   if (!pt.digits) return CUHE_OK;
   return pair_table(ctx, &pt.embed, (long long)rows8 * 256, [&](double2* t) {

@@ -1655,8 +1655,8 @@ k_lookup_encrypt(const uint8_t* __restrict__ bits, int embed_len, int chunk_len,
 }
 
 // The 16-bit-digit table: W[j][D] = G[2j][D mod 256] * G[2j+1][D / 256]
-// (Montgomery form in and out; for an odd message_chunks the last row's high
-// factor is 1).  One group per entry.
+// (Montgomery form in and out; the digit zero's factor, and for an odd
+// message_chunks the last row's high factor, is 1).  One group per entry.
 template <int K, int TPI>
 __global__ void __launch_bounds__(kBlockThreads)
 k_wide_table(const uint32_t* __restrict__ gtab, int message_chunks, uint32_t* __restrict__ wide,
@@ -1674,8 +1674,9 @@ k_wide_table(const uint32_t* __restrict__ gtab, int message_chunks, uint32_t* __
   uint32_t* s_b = smem + slot * STRIDE;
   uint32_t n2[L], lo[L], hi[L], r[L];
   g.load_ro(n2, consts + C_N2 * K);
-  g.load_ro(lo, gtab + ((long long)(2 * j) * 256 + (D & 255)) * K);
-  if (2 * j + 1 < message_chunks) g.load_ro(hi, gtab + ((long long)(2 * j + 1) * 256 + (D >> 8)) * K);
+  if (D & 255) g.load_ro(lo, gtab + ((long long)(2 * j) * 256 + (D & 255)) * K);
+  else g.load_ro(lo, consts + C_RM * K);
+  if (2 * j + 1 < message_chunks && D >> 8) g.load_ro(hi, gtab + ((long long)(2 * j + 1) * 256 + (D >> 8)) * K);
   else g.load_ro(hi, consts + C_RM * K);
   g.publish(s_b, hi);
   g.mont_mul(r, lo, s_b, n2, ks.ninv2);
@@ -1707,10 +1708,14 @@ __device__ __forceinline__ int pair_row_slot(int gl, int k) {
 }
 
 // out[i] = in[i] as a row: in = K words in the 32-bit Montgomery form x 2^(32K)
-// mod n^2, entry = R^(j+2) 2^(-32K) mod n^2 as pairs for the two chunks.
+// mod n^2, entry = R^(j+2) 2^(-32K) mod n^2 as pairs for the two chunks.  one:
+// null, or that form of 1, which takes the place of every 256th row from the
+// first: the digit zero, which the 8-bit kernel never looks up, is looked up
+// here where another group of the warp has a digit.
 template <int K>
 __global__ void __launch_bounds__(cuhe52::kPairThreads, 2)
-k_pair_rows(const uint32_t* __restrict__ in, long long count, double2* __restrict__ out,
+k_pair_rows(const uint32_t* __restrict__ in, long long count, const uint32_t* __restrict__ one,
+            double2* __restrict__ out,
             const double2* __restrict__ entry, const double* __restrict__ n52, unsigned long long ninv52) {
   constexpr int KL = 5 * K / 16, TPI = KL / 10, L = 10;
   extern __shared__ __align__(16) uint32_t smem[];
@@ -1720,6 +1725,7 @@ k_pair_rows(const uint32_t* __restrict__ in, long long count, double2* __restric
   cuhe52::Pair52<KL, TPI> f;
   const long long item = (long long)blockIdx.x * (cuhe52::kPairThreads / TPI) + threadIdx.x / TPI;
   const long long inst = min(item, count - 1);
+  const uint32_t* x = one && inst % 256 == 0 ? one : in + inst * K;
   const uint64_t ninv = f.gl == 0 ? ninv52 : 0ull;
   double m[L], a[L], r[L];
   uint64_t A0[L], A1[L], S0[L], S1[L];
@@ -1728,7 +1734,7 @@ k_pair_rows(const uint32_t* __restrict__ in, long long count, double2* __restric
 #pragma unroll 1
   for (int j = 0; j < 2; ++j) {
 #pragma unroll
-    for (int k = 0; k < L; ++k) a[k] = f.to_f64(limb52_from_words(in + inst * K, K, j * KL + f.gl * L + k));
+    for (int k = 0; k < L; ++k) a[k] = f.to_f64(limb52_from_words(x, K, j * KL + f.gl * L + k));
     f.template product<false>(A0, A1, a, a, s_rows + j * KL, m, ninv);
     f.template columns<2>(A0);
     f.template columns<2>(A1);

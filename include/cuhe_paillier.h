@@ -184,7 +184,9 @@ int cuhe_paillier_mulmod_outer(cuhe_paillier* ctx, const uint32_t* query, int64_
                                const uint32_t* index, int64_t nx, uint32_t* out);
 
 /* Install the fixed-base tables of Paillier-Lookup in normal (non-Montgomery)
- * form: g_table[(i*256 + j)*K ...] = g_table[i][j] and noise[k*K ...].
+ * form: g_table[(i*256 + j)*K ...] = g_table[i][j] and noise[k*K ...].  A
+ * digit 0 multiplies by nothing: g_table[i][0] is taken as 1, whatever stands
+ * there (cuhe_lookup_get_g_table gives it back as it was installed).
  * Replaces load_config(tables) / ensure_device_tables_
  * (paillier_GPU_lookup_client.cu:1771-1836, 2625-2652). */
 int cuhe_lookup_set_tables(cuhe_paillier* ctx, const uint32_t* g_table, int message_chunks,

@@ -99,3 +99,53 @@ def test_wide_rows_grow_behind_a_captured_call():
     # a later capture reads all rows
     late = _capture(ctx, calls[3])
     assert torch.equal(_replay(late, calls[3]), want[3])
+
+
+@pytest.mark.parametrize("message_chunks", [4, 5])
+def test_entry_of_the_digit_zero_is_taken_as_one(message_chunks):
+    """A table whose entries of the digit zero are not one: every kind of row
+    leaves them out, as the integer kernel does, whatever the neighbours of a
+    warp look up."""
+    from cuhepy_b200.paillier.gpu import PaillierDevice
+
+    rng = random.Random(message_chunks)
+    n = _odd(rng, 1000)
+    n2 = n * n
+    table = [[rng.randrange(2, n2) for _ in range(256)] for _ in range(message_chunks)]
+    noise = [rng.randrange(n2) for _ in range(5)]
+    ctx = PaillierDevice(n)
+    ctx.set_tables(table, noise)
+    plain = [0, 1, 256, 255 << 8, 7 << 16, 9 << 24] + [rng.getrandbits(8 * message_chunks) for _ in range(30)]
+    plain += [m & ~(255 << 8 * (k % message_chunks)) for k, m in enumerate(plain)]
+    idx = np.array([[rng.randrange(5) for _ in range(14)] for _ in plain], dtype=np.uint8)
+    want = []
+    for m, row in zip(plain, idx):
+        x = 1
+        for i in range(message_chunks):
+            d = m >> 8 * i & 255
+            x = x * table[i][d] % n2 if d else x
+        for k in row:
+            x = x * noise[int(k)] % n2
+        want.append(x)
+    # embeddings: plaintext bit 2 i is embedding bit last - i; odd chunk lengths take plain digits
+    embed = 4 * message_chunks
+    bits = np.array([[rng.randrange(2) if k % 3 else 0 for _ in range(embed)] for k in range(40)], dtype=np.uint8)
+    bits[5, : embed // 2] = 0
+    bits[6, embed // 2:] = 0
+    bnoise = np.zeros((40, 14), dtype=np.uint8)
+    bwant = []
+    for row in bits:
+        m = sum(int(b) << 2 * (embed - 1 - i) for i, b in enumerate(row))
+        x = pow(noise[0], 14, n2)
+        for i in range(message_chunks):
+            d = m >> 8 * i & 255
+            x = x * table[i][d] % n2 if d else x
+        bwant.append([x])
+    for fp64 in (1, 0):
+        ctx.set_fp64(fp64)
+        for wide in (0, 2):
+            ctx.set_wide_table(wide)
+            assert ctx.lookup_encrypt_ints(plain, idx) == want, (fp64, wide)
+            for chunk_len in (8 * message_chunks, 8 * message_chunks + 1):
+                assert ctx.lookup_encrypt_bits(bits, chunk_len, 1, bnoise) == bwant, (fp64, wide, chunk_len)
+    assert ctx.g_table() == table
