@@ -1867,8 +1867,10 @@ int wide_allowed(cuhe_paillier* ctx, long long items, size_t bytes, bool* allowe
   return CUHE_OK;
 }
 
+// The integer kernel's 16-bit-digit table; under stream capture, where nothing
+// may be allocated, the 8-bit table serves.
 int ensure_wide_table(cuhe_paillier* ctx, const Dispatch& d, long long items) {
-  if (ctx->d_wide || !ctx->d_gtab) return CUHE_OK;
+  if (ctx->d_wide || !ctx->d_gtab || capturing(ctx)) return CUHE_OK;
   const size_t bytes = size_t((ctx->message_chunks + 1) / 2) * 65536 * size_t(ctx->K) * 4;
   bool allowed = false;
   if (int rc = wide_allowed(ctx, items, bytes, &allowed)) return rc;

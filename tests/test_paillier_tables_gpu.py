@@ -16,15 +16,16 @@ def _odd(rng, bits):
     return rng.getrandbits(bits) | 1 | (1 << (bits - 1))
 
 
-def _pair(seed, message_chunks, entries):
-    """A context and one with the same tables that keeps to the integer kernel's 8-bit digits."""
+def _pair(seed, message_chunks, entries, pipe=1):
+    """A context with its tables installed for `pipe`, and one with the same
+    tables that keeps to the integer kernel's 8-bit digits."""
     from cuhepy_b200.paillier.gpu import PaillierDevice
 
     rng = random.Random(seed)
     n = _odd(rng, 1000)
     g, noise = rng.randrange(2, n * n), [rng.randrange(n * n) for _ in range(entries)]
     contexts = []
-    for fp64 in (1, 0):
+    for fp64 in (pipe, 0):
         ctx = PaillierDevice(n)
         ctx.set_fp64(fp64)
         ctx.set_wide_table(0)
@@ -149,3 +150,22 @@ def test_entry_of_the_digit_zero_is_taken_as_one(message_chunks):
             for chunk_len in (8 * message_chunks, 8 * message_chunks + 1):
                 assert ctx.lookup_encrypt_bits(bits, chunk_len, 1, bnoise) == bwant, (fp64, wide, chunk_len)
     assert ctx.g_table() == table
+
+
+@pytest.mark.parametrize("fp64", [1, 0])
+def test_a_capture_without_tables_of_its_pipe_builds_nothing(fp64):
+    """Tables installed for the integer pipe, the limb pairs and the wide table
+    first wanted inside a capture: the 8-bit words serve."""
+    import torch
+
+    ctx, plain = _pair(2, 16, 16, pipe=0)
+    call = _Call(ctx, 2, 50, 60, 16)
+    want = call.result(plain)
+    ctx.set_fp64(fp64)
+    ctx.set_wide_table(2)
+    graph = _capture(ctx, call)
+    assert torch.equal(_replay(graph, call), want)
+    assert not ctx.wide_table_ready()
+    assert torch.equal(call.result(ctx), want)
+    assert ctx.wide_table_ready()
+    assert torch.equal(_replay(graph, call), want)
