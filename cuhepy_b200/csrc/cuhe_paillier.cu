@@ -137,15 +137,16 @@ struct cuhe_paillier {
     const double2** embed_rows = nullptr;   // [ceil(message_chunks / 4)], wide_rows of them set
     int wide_rows = 0;
     void release() {
-      for (double2** p : {&digits, &embed, &noise, &noise2}) {
+      for (double2** p : {&digits, &embed, &noise}) {
         cudaFree(*p);
         *p = nullptr;
       }
       release_wide();
     }
     void release_wide() {
+      cudaFree(noise2);
       cudaFree(wide_digits);
-      wide_digits = nullptr;
+      noise2 = wide_digits = nullptr;
       for (double2* block : wide_blocks) cudaFree(block);
       wide_blocks.clear();
       cudaFree(embed_rows);
@@ -740,14 +741,15 @@ cudaError_t stream_after(cudaStream_t waiter, cudaStream_t from) {
   return e;
 }
 
-// The 16-bit-digit encryption table (W[j][D] = G[2j][D mod 256] *
-// G[2j+1][D / 256], 65,536 rows per pair of 8-bit digits): half the table
-// products per ciphertext, for (message_chunks + 1) / 2 * 65,536 * 4K bytes
-// (4 GiB at key_len 1024) and one product per entry to build, which about
-// 150,000 encryptions repay.  Mode 1 builds it for a call of at least
-// kWideMinItems ciphertexts when it takes at most kWideMaxBytes and a quarter
-// of the free device memory (else the 8-bit table serves); mode 2 builds it
-// for any call and fails without memory; mode 0 never.
+// The wide tables, rows of 65,536 entries that halve the table products per
+// ciphertext: 16 embedding bits a row (32 plaintext bits, built as far as the
+// calls reach, 42 MB a row at key_len 1024), 16-bit plaintext digits (128 rows
+// there), and on the integer pipe 16-bit digits in words (32 MB a row); one
+// product per entry to build.  Mode 1 builds what a call of at least
+// kWideMinItems ciphertexts wants when all of them together take at most
+// kWideMaxBytes and a quarter of the device memory they find free (else the
+// 8-bit tables serve); mode 2 builds it for any call and fails without memory;
+// mode 0 never.
 constexpr long long kWideMinItems = 1 << 16;
 constexpr size_t kWideMaxBytes = size_t(8) << 30;
 
@@ -1857,13 +1859,23 @@ int cuhe_lookup_get_g_table(cuhe_paillier* ctx, uint32_t* out) {
 
 namespace {
 
-// The wide table's share of device memory under the default policy.
+// Device bytes of one 65,536-entry row of the wide tables: words, limb pairs.
+size_t wide_word_row(const cuhe_paillier* ctx) { return size_t(65536) * size_t(ctx->K) * 4; }
+size_t wide_pair_row(const cuhe_paillier* ctx) { return size_t(65536) * size_t(5 * ctx->K / 16) * 16; }
+
+// Whether a wide table may take `bytes` more.  Under the default policy all of
+// them together (the words', the digits' and the embeddings') stay within
+// kWideMaxBytes and a quarter of the memory that would be free without them.
 int wide_allowed(cuhe_paillier* ctx, long long items, size_t bytes, bool* allowed) {
   *allowed = ctx->wide_mode == 2;
-  if (ctx->wide_mode != 1 || items < kWideMinItems || bytes > kWideMaxBytes) return CUHE_OK;
+  if (ctx->wide_mode != 1 || items < kWideMinItems) return CUHE_OK;
+  const size_t digit_rows = size_t(ctx->message_chunks + 1) / 2;
+  const size_t held = (ctx->d_wide ? digit_rows * wide_word_row(ctx) : 0) +
+                      ((ctx->pt.wide_digits ? digit_rows : 0) + size_t(ctx->pt.wide_rows)) * wide_pair_row(ctx);
+  if (held + bytes > kWideMaxBytes) return CUHE_OK;
   size_t free_bytes = 0, total_bytes = 0;
   CUHE_CUDA(ctx, cudaMemGetInfo(&free_bytes, &total_bytes), "free memory");
-  *allowed = bytes <= free_bytes / 4;
+  *allowed = held + bytes <= (free_bytes + held) / 4;
   return CUHE_OK;
 }
 
@@ -1871,7 +1883,7 @@ int wide_allowed(cuhe_paillier* ctx, long long items, size_t bytes, bool* allowe
 // may be allocated, the 8-bit table serves.
 int ensure_wide_table(cuhe_paillier* ctx, const Dispatch& d, long long items) {
   if (ctx->d_wide || !ctx->d_gtab || capturing(ctx)) return CUHE_OK;
-  const size_t bytes = size_t((ctx->message_chunks + 1) / 2) * 65536 * size_t(ctx->K) * 4;
+  const size_t bytes = size_t((ctx->message_chunks + 1) / 2) * wide_word_row(ctx);
   bool allowed = false;
   if (int rc = wide_allowed(ctx, items, bytes, &allowed)) return rc;
   if (!allowed) return CUHE_OK;
@@ -1890,7 +1902,8 @@ int ensure_wide_table(cuhe_paillier* ctx, const Dispatch& d, long long items) {
 }
 
 // Noise products of two repay their table (noise_entries^2 products, seven
-// saved by a ciphertext) from this many ciphertexts in one call.
+// saved by a ciphertext) from this many ciphertexts in one call; mode 0, which
+// asks for the small tables alone, does without.
 constexpr long long kNoisePairItems = 8192;
 
 // Rows [wide_rows, need) of the 16-bit embedding table (of the 8-bit table's
@@ -1899,7 +1912,7 @@ constexpr long long kNoisePairItems = 8192;
 int grow_embed_rows(cuhe_paillier* ctx, const PairLookup& pl, int rows8, int need) {
   auto& pt = ctx->pt;
   const int before = pt.wide_rows, added = need - before;
-  const size_t entries = size_t(5 * ctx->K / 16) * 65536;  // pairs of a row
+  const size_t entries = wide_pair_row(ctx) / sizeof(double2);  // pairs of a row
   double2* block = nullptr;
   cudaError_t e = pt.embed_rows ? cudaSuccess : cudaMalloc(&pt.embed_rows, size_t((rows8 + 1) / 2) * sizeof(double2*));
   if (e == cudaSuccess) e = cudaMalloc(&block, size_t(added) * entries * sizeof(double2));
@@ -1932,7 +1945,7 @@ int pair_lookup_encrypt(cuhe_paillier* ctx, const PairLookup& pl, cuhe::LookupDi
   const int chunks = ctx->message_chunks, entries = ctx->noise_entries;
   if (int rc = pair_tables(ctx, pl)) return rc;
   if (!pt.digits || !pt.noise) return CUHE_OK;
-  if (count >= kNoisePairItems)
+  if (count >= kNoisePairItems && ctx->wide_mode != 0)
     if (int rc = pair_table(ctx, &pt.noise2, (long long)entries * entries, [&](double2* t) {
           return pl.products(ctx, pt.noise, entries, cuhe::kNoise, 0, (long long)entries * entries, t);
         }))
@@ -1941,7 +1954,6 @@ int pair_lookup_encrypt(cuhe_paillier* ctx, const PairLookup& pl, cuhe::LookupDi
   dg.message_chunks = chunks;
   dg.rows = chunks;
   dg.wide = dg.embed_bits = 0;
-  const size_t row_bytes = size_t(5 * ctx->K / 16) * 16;
   bool allowed = false;
   if (dg.bits && dg.chunk_len % 2 == 0 && pt.embed) {
     const int rows8 = (chunks + 1) / 2;
@@ -1949,7 +1961,7 @@ int pair_lookup_encrypt(cuhe_paillier* ctx, const PairLookup& pl, cuhe::LookupDi
     const int reach = std::min(2 * dg.embed_len, dg.chunk_len);
     const int need8 = std::min(rows8, (reach + 15) / 16), need = (need8 + 1) / 2;
     if (pt.wide_rows < need && !capturing(ctx)) {
-      if (int rc = wide_allowed(ctx, count, size_t(need) * 65536 * row_bytes, &allowed)) return rc;
+      if (int rc = wide_allowed(ctx, count, size_t(need - pt.wide_rows) * wide_pair_row(ctx), &allowed)) return rc;
       if (allowed)
         if (int rc = grow_embed_rows(ctx, pl, rows8, need)) return rc;
     }
@@ -1961,7 +1973,7 @@ int pair_lookup_encrypt(cuhe_paillier* ctx, const PairLookup& pl, cuhe::LookupDi
   } else {
     const int rows = (chunks + 1) / 2;
     if (!pt.wide_digits && !capturing(ctx)) {
-      if (int rc = wide_allowed(ctx, count, size_t(rows) * 65536 * row_bytes, &allowed)) return rc;
+      if (int rc = wide_allowed(ctx, count, size_t(rows) * wide_pair_row(ctx), &allowed)) return rc;
       if (allowed) {
         if (int rc = pair_table(ctx, &pt.wide_digits, (long long)rows * 65536, [&](double2* t) {
               return pl.products(ctx, pt.digits, chunks, cuhe::kWide, 0, (long long)rows * 65536, t);
@@ -1994,7 +2006,7 @@ int cuhe_lookup_set_wide_table(cuhe_paillier* ctx, int mode) {
   DeviceGuard guard(ctx->device);
   std::lock_guard<std::mutex> lock(ctx->mu);
   ctx->wide_mode = mode;
-  if (mode == 0 && (ctx->d_wide || ctx->pt.wide())) {
+  if (mode == 0 && (ctx->d_wide || ctx->pt.wide() || ctx->pt.noise2)) {
     CUHE_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "wide table release");
     cudaFree(ctx->d_wide);
     ctx->d_wide = nullptr;

@@ -221,14 +221,16 @@ int cuhe_lookup_encrypt_bits(cuhe_paillier* ctx, const uint8_t* bits, int64_t ve
  * many rows, and only the rows that the calls' embeddings reach are built
  * (1.25 GiB for 512-bit embeddings at key_len 1024); words and odd chunk
  * lengths use the pairs of plaintext digits.  A call of 8,192 ciphertexts or
- * more also builds the products of all pairs of noise entries.  mode 1 (the
- * default) builds it during an encryption call of at least 65,536
- * ciphertexts, when it takes at most 8 GiB and a quarter of the free device
- * memory; mode 2 builds it at the next encryption call of any size
- * (CUHE_OUT_OF_MEMORY without the memory); mode 0 frees it and keeps the
- * 8-bit table.  Installing new tables drops it.  The table is built for the
- * pipe selected at that time and is kept, unused, while the other pipe is
- * selected, which builds its own by the same rule.  Without memory for the
+ * more also builds the products of all pairs of noise entries (42 MB at
+ * key_len 1024).  mode 1 (the default) builds a wide table during an
+ * encryption call of at least 65,536 ciphertexts, while all that the context
+ * holds of them takes at most 8 GiB and a quarter of the device memory that is
+ * free without them; mode 2 builds it at the next encryption call of any size
+ * (CUHE_OUT_OF_MEMORY without the memory); mode 0 frees them and the products
+ * of noise entries, and keeps the 8-bit tables alone.  Installing new tables
+ * drops them.  A table is built for the pipe selected at that time and is
+ * kept, unused, while the other pipe is selected, which builds its own by the
+ * same rule.  Without memory for the
  * limb pairs a call runs on the integer pipe; inside a stream capture nothing
  * is built and the tables that are there serve.  Rows are added and never
  * moved: an encryption captured in a graph can be replayed until mode 0, new

@@ -37,18 +37,18 @@ def _pair(seed, message_chunks, entries, pipe=1):
 class _Call:
     """`count` embeddings of `embed` bits with their noise, and a place for the result."""
 
-    def __init__(self, ctx, seed, count, embed, entries):
+    def __init__(self, ctx, seed, count, embed, entries, chunk_len=CHUNK_LEN):
         import torch
 
         gen = np.random.default_rng([seed, embed])
-        self.count, self.embed = count, embed
+        self.count, self.embed, self.chunk_len = count, embed, chunk_len
         self.bits = torch.from_numpy(gen.integers(0, 2, size=(count, embed), dtype=np.uint8)).cuda()
         self.noise = torch.from_numpy(gen.integers(0, entries, size=(count, 14), dtype=np.uint8)).cuda()
         self.out = torch.zeros((count, ctx.words), dtype=torch.int32, device="cuda")
         torch.cuda.synchronize()
 
     def enqueue(self, ctx):
-        ctx.lookup_encrypt_bits_array(self.bits, self.count, self.embed, CHUNK_LEN, 1, self.noise, self.out)
+        ctx.lookup_encrypt_bits_array(self.bits, self.count, self.embed, self.chunk_len, 1, self.noise, self.out)
 
     def result(self, ctx):
         import torch
@@ -169,3 +169,64 @@ def test_a_capture_without_tables_of_its_pipe_builds_nothing(fp64):
     assert torch.equal(call.result(ctx), want)
     assert ctx.wide_table_ready()
     assert torch.equal(_replay(graph, call), want)
+
+
+def _key_1024(message_chunks, entries):
+    from cuhepy_b200.paillier.gpu import PaillierDevice
+
+    rng = random.Random(7)
+    n = _odd(rng, 2047)
+    ctx = PaillierDevice(n)
+    ctx.set_wide_table(0)
+    ctx.build_tables(n + 2, message_chunks, [rng.randrange(n * n) for _ in range(entries)])
+    return ctx
+
+
+def _held(before):
+    import torch
+
+    torch.cuda.synchronize()
+    return before - torch.cuda.mem_get_info()[0]
+
+
+def test_mode_0_holds_no_noise_products():
+    """256^2 products of noise entries (42 MB) come with a large call, and go with mode 0."""
+    import torch
+
+    ctx = _key_1024(16, 256)
+    call, small = _Call(ctx, 1, 8192, 60, 256), _Call(ctx, 2, 40, 60, 256)
+    small.result(ctx)
+    call.out.clone()
+    before = torch.cuda.mem_get_info()[0]
+    want = call.result(ctx)
+    assert _held(before) < 1 << 24
+    ctx.set_wide_table(1)
+    assert torch.equal(call.result(ctx), want)
+    assert _held(before) >= 256 * 256 * 640
+    ctx.set_wide_table(0)
+    assert _held(before) < 1 << 24
+    assert torch.equal(call.result(ctx), want)
+
+
+def test_wide_tables_share_one_bound():
+    """Tables for embeddings (2.5 GiB), digits (5 GiB) and words (4 GiB): a
+    context of the default mode holds at most 8 GiB of them."""
+    import torch
+
+    ctx = _key_1024(256, 16)
+    count = 1 << 16
+    call = _Call(ctx, 1, count, 1024, 16, 2048)
+    words, out = torch.zeros_like(call.out), torch.zeros_like(call.out)
+    torch.cuda.synchronize()
+    want = call.result(ctx)
+    call.out.clone()
+    before = torch.cuda.mem_get_info()[0]
+    ctx.set_wide_table(1)
+    for fp64, least in ((1, 7 << 30), (0, 7 << 30), (1, 7 << 30)):
+        ctx.set_fp64(fp64)
+        assert torch.equal(call.result(ctx), want)
+        ctx.lookup_encrypt_ints_array(words, count, call.noise, out)
+        ctx.synchronize()
+        assert least < _held(before) < (8 << 30) + (64 << 20), fp64
+    ctx.set_wide_table(0)
+    assert _held(before) < 1 << 24
