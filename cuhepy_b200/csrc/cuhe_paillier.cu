@@ -81,6 +81,7 @@ bool is_device_pointer(const void* p) {
 struct cuhe_paillier {
   int device = 0;
   int sms = 1;  // multiprocessors of the device
+  int smem_limit = 48 << 10;  // dynamic shared memory a block may ask for beside 1 KB of static
   int K = 0;
   int n_words = 0;
   int tpi = 0, window = 0;
@@ -400,8 +401,10 @@ cudaError_t launch_pair_lookup_l(cuhe_paillier* ctx, const cuhe::LookupDigits& d
                                  uint32_t* out) {
   using Lay = cuhe::LookupLayout<K, kL>;
   const size_t smem = Lay::bytes(dg.rows);
+  // the device's limit, not this call's size: a kernel has one setting, and
+  // other contexts set it between this line and the launch
   cudaError_t e = cudaFuncSetAttribute(cuhe::k_pair_lookup<K, kL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(smem));
+                                       ctx->smem_limit);
   if (e != cudaSuccess) return e;
   const long long blocks = (count + Lay::kGroups - 1) / Lay::kGroups;
   cuhe::k_pair_lookup<K, kL><<<dim3(unsigned(blocks)), cuhe52::kPairThreads, smem, ctx->stream>>>(
@@ -518,7 +521,8 @@ cudaError_t launch_lookup(cuhe_paillier* ctx, const uint8_t* bits, int embed_len
   const size_t smem = size_t(K + IPB * cuhe::inst_stride_words<K>(1)) * 4 + ((rows_bytes + 15) & ~size_t(15));
   const bool wide = ctx->d_wide != nullptr;
   auto kernel = wide ? cuhe::k_lookup_encrypt<K, TPI, true> : cuhe::k_lookup_encrypt<K, TPI, false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  // (the device's limit: as for k_pair_lookup)
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_limit);
   if (e != cudaSuccess) return e;
   const long long blocks = (count + IPB - 1) / IPB;
   kernel<<<dim3(unsigned(blocks)), cuhe::kBlockThreads, smem, ctx->stream>>>(
@@ -970,6 +974,8 @@ int cuhe_paillier_create(const uint32_t* n_in, int n_words, int device, cuhe_pai
   if (!ctx) return fail(nullptr, CUHE_OUT_OF_MEMORY, "context allocation");
   ctx->device = device;
   if (cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) ctx->sms = 148;
+  cudaDeviceGetAttribute(&ctx->smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  ctx->smem_limit -= 1 << 10;
   ctx->K = K;
   ctx->n_words = K / 2;
   default_tuning(K, &ctx->tpi, &ctx->window);

@@ -230,3 +230,40 @@ def test_wide_tables_share_one_bound():
         assert least < _held(before) < (8 << 30) + (64 << 20), fp64
     ctx.set_wide_table(0)
     assert _held(before) < 1 << 24
+
+
+@pytest.mark.parametrize("fp64", [1, 0])
+def test_contexts_with_tables_of_other_sizes_on_two_threads(fp64):
+    """Calls whose blocks ask for much and for little shared memory, each on
+    its own context and thread: neither one's launch meets the other's limit."""
+    import threading
+
+    import torch
+
+    jobs = []
+    for seed, chunks, embed in ((4, 128, 500), (5, 2, 8)):
+        ctx, plain = _pair(seed, chunks, 4)
+        call = _Call(ctx, seed, 3, embed, 4)
+        want = call.result(plain)
+        ctx.set_fp64(fp64)
+        jobs.append((ctx, call, want))
+    errors = []
+
+    def work(ctx, call):
+        try:
+            for _ in range(5000):
+                if errors:
+                    break
+                call.enqueue(ctx)
+            ctx.synchronize()
+        except Exception as error:  # reported by the main thread
+            errors.append(error)
+
+    threads = [threading.Thread(target=work, args=job[:2]) for job in jobs]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert not errors
+    for ctx, call, want in jobs:
+        assert torch.equal(call.out, want)
