@@ -113,6 +113,7 @@ struct cuhe_paillier {
     int32_t* d_ops = nullptr;
     int32_t* d_fall = nullptr;
     int nops = 0, nfall = 0, halved = 0;
+    size_t room = 0;  // ops that each array holds
     cuhe::PairExponent get() const { return {d_ops, d_fall, nops, nfall, halved}; }
   } side_exp[2];
   Limbs factor[2];  // p, q once installed
@@ -785,6 +786,15 @@ int upload_schedule(cuhe_paillier* ctx, const Limbs& e, int32_t** dptr, int* nop
   return CUHE_OK;
 }
 
+// One of a side's schedules into its array of side.room ops, which stays where
+// it is: calls captured in a graph read it at every replay.
+int upload_side_schedule(cuhe_paillier* ctx, const Limbs& e, int32_t* d_ops, int* nops) {
+  const std::vector<int32_t> ops = cuhe::host::pair_schedule(e, cuhe::kPairWindow, cuhe::kSplitWindow, nops);
+  CUHE_CUDA(ctx, cudaMemcpy(d_ops, ops.data(), ops.size() * sizeof(int32_t), cudaMemcpyHostToDevice),
+            "schedule upload");
+  return CUHE_OK;
+}
+
 // The 52-bit constants mod n^2: n^2 and R52 mod n^2 as K52 = 5K/8 limbs of 52 bits
 // (doubles), then R52 R mod n^2 as K words; R52 = 2^(52 K52), R = 2^(32K).
 int setup_direct52(cuhe_paillier* ctx) {
@@ -912,9 +922,22 @@ int setup_pair_crt(cuhe_paillier* ctx) {
     const std::vector<double> one = pair_constants(p, k, 4, ctx->have_secret ? &scale : nullptr);
     block.insert(block.end(), one.begin(), one.end());
     if (!ctx->have_secret) continue;
-    if (int rc = upload_schedule(ctx, main, &side.d_ops, &side.nops, true)) return rc;
+    // both schedules are of divisors of the secret exponent: a context's
+    // arrays are made anew for a longer secret only
+    const size_t room = cuhe::host::pair_schedule_room(cuhe::host::bit_length(ctx->secret_exp), cuhe::kPairWindow);
+    if (room > side.room) {
+      for (int32_t** ops : {&side.d_ops, &side.d_fall}) {
+        cudaFree(*ops);
+        *ops = nullptr;
+      }
+      side.room = 0;
+      for (int32_t** ops : {&side.d_ops, &side.d_fall})
+        CUHE_CUDA(ctx, cudaMalloc(ops, room * sizeof(int32_t)), "schedule allocation");
+      side.room = room;
+    }
+    if (int rc = upload_side_schedule(ctx, main, side.d_ops, &side.nops)) return rc;
     if (side.halved)
-      if (int rc = upload_schedule(ctx, cofactor, &side.d_fall, &side.nfall, true)) return rc;
+      if (int rc = upload_side_schedule(ctx, cofactor, side.d_fall, &side.nfall)) return rc;
   }
   return upload_constants(ctx, block, &ctx->d_crt52);
 }
@@ -1144,9 +1167,11 @@ int cuhe_paillier_set_secret(cuhe_paillier* ctx, const uint32_t* exponent, int e
   ctx->secret_exp = e;
   ctx->secret_mult = mult;
   ctx->have_secret = true;
-  if (int rc = upload_schedule(ctx, e, &ctx->d_ops_sec52, &ctx->nops_sec52, true)) return rc;
-  if (int rc = setup_pair_crt(ctx)) return rc;
-  return upload_schedule(ctx, e, &ctx->d_ops_sec, &ctx->nops_sec);
+  int rc = upload_schedule(ctx, e, &ctx->d_ops_sec52, &ctx->nops_sec52, true);
+  if (!rc) rc = setup_pair_crt(ctx);
+  if (!rc) rc = upload_schedule(ctx, e, &ctx->d_ops_sec, &ctx->nops_sec);
+  if (rc) ctx->have_secret = false;  // nothing reads what is half installed
+  return rc;
 }
 
 int cuhe_paillier_set_factors(cuhe_paillier* ctx, const uint32_t* p_in, int p_words, const uint32_t* q_in,
@@ -1207,7 +1232,9 @@ int cuhe_paillier_set_factors(cuhe_paillier* ctx, const uint32_t* p_in, int p_wo
   ctx->factor[0] = p;
   ctx->factor[1] = q;
   ctx->have_factors = true;
-  return setup_pair_crt(ctx);
+  const int rc = setup_pair_crt(ctx);
+  if (rc) ctx->have_factors = false;  // decryption goes without what is half installed
+  return rc;
 }
 
 int cuhe_paillier_has_factors(const cuhe_paillier* ctx) { return ctx && ctx->have_factors ? 1 : 0; }

@@ -225,5 +225,10 @@ inline std::vector<int32_t> pair_schedule(const Limbs& e, int window, int widest
   return ops;
 }
 
+// The most ops that pair_schedule makes of an exponent of `bits` bits, the wide
+// schedule's two head words included: an op's window starts at least `window`
+// bits below the one before, and zeros at the end may take one more.
+inline size_t pair_schedule_room(size_t bits, int window) { return 2 * (bits / size_t(window) + 2) + 2; }
+
 }  // namespace host
 }  // namespace cuhe
