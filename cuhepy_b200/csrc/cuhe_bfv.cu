@@ -236,8 +236,9 @@ struct cuhe_bfv_key {
   cuhe_bfv_ring* ring = nullptr;
   u64* d_key = nullptr;  // [D][2][L][N] NTT domain, then as many Shoup quotients
   u64* d_key_q = nullptr;
-  // the key lifted for NTT-domain rotations (k_lift_key) and its quotients
-  // (residue rings whose planes fit one CTA, two digits or more)
+  // the key lifted for NTT-domain rotations (k_lift_key) and its quotients:
+  // as many bytes again, made when a server or a tile circuit first uses the
+  // key (lift_key), under lane 0's lock
   u64* d_lift = nullptr;
   u64* d_lift_q = nullptr;
   size_t bytes = 0;
@@ -257,6 +258,7 @@ struct cuhe_bfv_server {
   cuhe_bfv_key* relin = nullptr;
   std::map<u64, cuhe_bfv_key*> keys;
   size_t padded = 0, lanes = 0, capacity = 0;
+  bool ntt = false;  // searches keep their ciphertexts in the NTT domain (every key is lifted)
   u64 t = 0;
   H::Big target;
   unsigned target_bits = 0;
@@ -644,6 +646,45 @@ bool ntt_rotations(const cuhe_bfv_ring* r) {
   return r->residue && r->plan.n <= kMaxPlaneN && r->plan.n >= 2 && r->plan.digits >= 2;
 }
 
+// The lifted form of a key for this ring's NTT-domain rotations.  Without
+// memory for it the key stays as it is (CUHE_OK): the caller's circuit then
+// switches in the coefficient domain.  ln: lane 0, locked.
+int lift_key(cuhe_bfv_key* key, Lane& ln, RingDev* d) {
+  cuhe_bfv_ring* r = key->ring;
+  if (key->d_lift || !ntt_rotations(r)) return CUHE_OK;
+  const auto& P = r->plan;
+  const size_t L = P.residue_count, D = P.digits, planes = 2 * D * L;
+  std::vector<u64> power(D * L);
+  for (size_t k = 0; k < D; ++k)
+    for (size_t j = 0; j < L; ++j) power[k * L + j] = H::powmod(2, u64(k) * P.digit_bits, P.primes[j]);
+  u64 *lift = nullptr, *d_power = nullptr;
+  cudaError_t e = cudaMalloc(&lift, key->bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&d_power, power.size() * 8);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(d_power, power.data(), power.size() * 8, cudaMemcpyHostToDevice, ln.stream);
+  if (e == cudaSuccess) {
+    u64* quotients = lift + planes * P.n;
+    const unsigned blocks = blocks_for((long long)(planes * P.n), 256);
+    k_lift_key<<<blocks, 256, 0, ln.stream>>>(key->d_key, d_power, int(D), int(L), lift, d);
+    k_shoup_quotients<<<blocks, 256, 0, ln.stream>>>(lift, quotients, (long long)(planes), int(L), d);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ln.stream);
+    if (e == cudaSuccess) {
+      key->d_lift = lift;
+      key->d_lift_q = quotients;
+    }
+  }
+  cudaFree(d_power);
+  if (e == cudaSuccess) return CUHE_OK;
+  cudaFree(lift);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return CUHE_OK;
+  }
+  BFV_CUDA(e, "key lifting");
+  return CUHE_OK;
+}
+
 // Rotations with their op tables: the host side collects every step of a
 // chain, uploads the tables once and launches step after step without
 // waiting.
@@ -818,7 +859,7 @@ struct TileArgs {
 };
 
 // Whether a tile circuit with these rotations leaves its distances in the
-// NTT domain (tile_circuit_ntt).
+// NTT domain (tile_circuit_ntt), given lifted keys.
 bool ntt_circuit(const cuhe_bfv_ring* r, const std::vector<u64>& exps) {
   if (!ntt_rotations(r) || exps.empty()) return false;
   for (u64 g : exps)
@@ -1559,25 +1600,7 @@ int cuhe_bfv_compile_key(cuhe_bfv_ring* ring, const uint8_t* key_polys, uint64_t
         key->d_key, key->d_key_q, (long long)(2 * digits * L), int(L), d);
     e = cudaGetLastError();
   }
-  u64* d_power = nullptr;
-  if (!rc && e == cudaSuccess && ntt_rotations(ring)) {
-    std::vector<u64> power(size_t(digits) * L);
-    for (size_t dgt = 0; dgt < size_t(digits); ++dgt)
-      for (size_t j = 0; j < L; ++j) power[dgt * L + j] = H::powmod(2, u64(dgt) * P.digit_bits, P.primes[j]);
-    e = cudaMalloc(&d_power, power.size() * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&key->d_lift, key->bytes);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(d_power, power.data(), power.size() * 8, cudaMemcpyHostToDevice, ln.stream);
-    if (e == cudaSuccess) {
-      key->d_lift_q = key->d_lift + size_t(digits) * 2 * L * n;
-      const unsigned blocks = blocks_for((long long)(2 * digits * L * n), 256);
-      k_lift_key<<<blocks, 256, 0, ln.stream>>>(key->d_key, d_power, int(digits), int(L), key->d_lift, d);
-      k_shoup_quotients<<<blocks, 256, 0, ln.stream>>>(key->d_lift, key->d_lift_q, (long long)(2 * digits * L), int(L), d);
-      e = cudaGetLastError();
-    }
-  }
   if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(ln.stream);
-  if (d_power) cudaFree(d_power);
   if (d_words) cudaFree(d_words);
   if (rc || e != cudaSuccess) {
     cuhe_bfv_key_release(key);
@@ -1820,7 +1843,15 @@ int cuhe_bfv_hamming_tile(cuhe_bfv_key* relin, const uint8_t* query, const uint8
     return download_words(r, ln, dist, 2, out);
   }
   const std::vector<u64> exps(exponents, exponents + rotations);
-  const bool ntt = ntt_circuit(r, exps);
+  bool ntt = ntt_circuit(r, exps);
+  if (ntt) {
+    if (int rc = lift_key(relin, ln, d)) return rc;
+    ntt = relin->d_lift;
+    for (uint64_t k = 0; k < rotations && ntt; ++k) {
+      if (int rc = lift_key(keys[k], ln, d)) return rc;
+      ntt = keys[k]->d_lift;
+    }
+  }
   BFV_CUDA(ln.arena.reserve((ntt ? tile_ntt_arena_bytes(r, 1, exps.size()) + slice(2 * sizeof(InverseOp))
                                  : tile_arena_bytes(r, 1)) + slice(2 * n * W * 8) * 2 + slice(n * W * 8) + slice(L * n * 8) * 2 +
                             slice(2 * L * n * 8) + slice(2 * n * W * 8) + 16384),
@@ -1921,6 +1952,15 @@ int cuhe_bfv_create_server(cuhe_bfv_key* relin, const uint64_t* exponents, cuhe_
   int rc = upload_plain_ntt(r, ln, d, small_to_words(hamming_mask(n, t, lanes, s->capacity), W), &s->d_full_mask,
                             s->mask_primes);
   cudaError_t e = cudaSuccess;
+  // the keys of the search's own switches, in the form its circuit takes
+  s->ntt = ntt_circuit(r, left);
+  std::vector<cuhe_bfv_key*> used{relin};
+  for (const auto* exps : {&left, &right})
+    for (u64 g : *exps) used.push_back(keymap.at(g));
+  for (size_t k = 0; k < used.size() && !rc && s->ntt; ++k) {
+    rc = lift_key(used[k], ln, d);
+    s->ntt = used[k]->d_lift;
+  }
   if (!rc) e = cudaMalloc(&s->d_target, 8 * std::max<size_t>(1, target.w.size()));
   if (!rc && e == cudaSuccess)
     e = cudaMemcpy(s->d_target, target.w.data(), 8 * target.w.size(), cudaMemcpyHostToDevice);
@@ -2004,8 +2044,7 @@ size_t search_chunk_bytes(const cuhe_bfv_server* s, size_t ct, unsigned out_bits
            slice(2 * n * W * 8) + slice(ct * 2 * n * W * 8) * 2 + slice(gc * 2 * n * W * 8) +
            slice(gc * 2 * out_words * 8) + slice(sizeof(int)) + slice(ct * n * W * 8) +
            slice(ct * sizeof(ComposeOp)) + slice(ct * sizeof(SwitchOp)) + small + 65536;
-  const bool ntt = ntt_circuit(r, s->left);
-  const size_t tiles = ntt ? tile_ntt_arena_bytes(r, ct, s->left.size()) + slice(ct * L * n * 8) + rotate_table_bytes(ct) +
+  const size_t tiles = s->ntt ? tile_ntt_arena_bytes(r, ct, s->left.size()) + slice(ct * L * n * 8) + rotate_table_bytes(ct) +
                                  slice(2 * gc * sizeof(InverseOp))
                            : tile_arena_bytes(r, ct);
   return tiles + slice(2 * in_bytes) + slice(ct * 2 * in_bytes) + slice(2 * n * W * 8) +
@@ -2056,7 +2095,7 @@ int search_impl(cuhe_bfv_server* s, const uint8_t* query, const PolySource* inde
   Lane& ln = acquire_lane(r, lock);
   DeviceGuard guard(r->device);
   RingDev* d = s->d_ring;
-  const bool ntt = r->residue && ntt_circuit(r, s->left);
+  const bool ntt = s->ntt;
   double prof[6] = {0, 0, 0, 0, 0, 0};
   // partial mask for the last tile
   const u64* partial = nullptr;

@@ -45,7 +45,11 @@ int cuhe_bfv_ring_info(const cuhe_bfv_ring* ring, uint64_t* primes, int capacity
                        uint64_t* coefficient_bytes, int* kernel_level, int* fast);
 
 /* compile_key(ring, ((b, a),) * digits) (bindings.cpp:194-208): the key as
- * digits*2 consecutive polys b_0, a_0, b_1, a_1, ... */
+ * digits*2 consecutive polys b_0, a_0, b_1, a_1, ...  key_bytes gives its
+ * device bytes.  On residue rings of N <= 16384 with two or more digits, a key
+ * that create_server takes for its searches, or hamming_tile uses, holds as
+ * many again from then on, in the form that NTT-domain rotations read; where
+ * the device has no memory for that, those run in the coefficient domain. */
 int cuhe_bfv_compile_key(cuhe_bfv_ring* ring, const uint8_t* key_polys, uint64_t digits, cuhe_bfv_key** out);
 void cuhe_bfv_key_release(cuhe_bfv_key* key);
 uint64_t cuhe_bfv_key_bytes(const cuhe_bfv_key* key);
