@@ -117,8 +117,10 @@ class MixedBatch:
 
     def _select_pipe(self, entries: list[_Modexp]) -> None:
         for e in entries:
-            if e.ctx.words in self.paillier_fp64:
-                e.ctx.set_fp64(1 if self.paillier_fp64[e.ctx.words] else 0)
+            use = self.paillier_fp64.get(e.ctx.words)
+            # a context on the FP64 pipe keeps its own setting (1, or 2)
+            if use is not None and use != bool(e.ctx.fp64):
+                e.ctx.set_fp64(int(use))
 
     def _build_mix(self, entries: list[_Modexp], tuning: dict[int, tuple[int, int]]):
         self._select_pipe(entries)
