@@ -563,18 +563,11 @@ def run_bfv(steps: int, warmup: int, cpu: bool, native: bool = False) -> dict:
         m.hamming_tile(relin, qf, qf, rot, mask, BFV_T)
     per_tile = (time.perf_counter() - t0) / plain_tiles
     tiles = len(index)
-    # transforms per query.  Residue rings keep ciphertexts in the NTT domain
-    # through the rotations and merges (T tensor primes 7, L residue primes 3,
-    # D digits 6, R rotations 9): per tile 2T and 3T for the tensor, 3L to
-    # bring the relinearisation's input over, and per switch (D - 1) L forward
-    # and L inverse (component 1's coefficients for the next); per merge one
-    # switch; per response 2L inverse.  (The circuit with coefficient-domain
-    # switches, bfv_server.h's, takes 200 and 87 per tile, 18 and 6 per merge.)
-    # Native rings: T tensor, S switch and M mask primes: forward
-    # 2T + (1 + R) D S + 2M, inverse 3T + (1 + R) 2S + 2M; per merge D S and 2S.
-    groups = (tiles + layout.padded - 1) // layout.padded
-    merges = tiles - groups
-    fwd, inv = 173 * tiles + 15 * merges, 51 * tiles + 3 * merges + 6 * groups
+    # transforms per query (residue_transforms).  Native rings: T tensor, S
+    # switch and M mask primes: forward 2T + (1 + R) D S + 2M, inverse
+    # 3T + (1 + R) 2S + 2M; per merge D S and 2S.
+    merges = tiles - (tiles + layout.padded - 1) // layout.padded
+    fwd, inv = residue_transforms(tiles, layout.padded, T=7, L=3, D=6, R=len(layout.left()))
     info = m.ring_info(ring)
     if native:
         T, S, D, R = len(info["primes"]), info["switch_prime_count"], 6, len(layout.left())
@@ -638,6 +631,24 @@ def run_bfv(steps: int, warmup: int, cpu: bool, native: bool = False) -> dict:
     if cpu:
         out["_setup"] = (q, layout, exps, keys, query, index, target, native)
     return out
+
+
+def residue_transforms(tiles: int, padded: int, T: int, L: int, D: int, R: int) -> tuple[int, int]:
+    """Forward and inverse transforms of one search on a residue ring (T tensor
+    primes, L residue primes, D digits, R rotations per tile), whose ciphertexts
+    stay in the NTT domain through the rotations and merges.  Per tile: 2T and
+    3T for the tensor, 3L to bring the relinearisation's input over; per switch
+    (relinearisation, rotation, merge) (D - 1) L forward.  A switch transforms
+    component 1 back, L inverse, where another switch takes it from there: the
+    relinearisation and all rotations but a tile's last, and one last rotation
+    or merge for every merge, that of its right operand.  Per response 2L
+    inverse.  (The circuit with coefficient-domain switches, bfv_server.h's,
+    takes 200 and 87 per tile and 18 and 6 per merge at T 7, L 3, D 6, R 9.)"""
+    responses = (tiles + padded - 1) // padded
+    merges = tiles - responses
+    forward = (2 * T + 3 * L) * tiles + ((1 + R) * tiles + merges) * (D - 1) * L
+    inverse = (3 * T + R * L) * tiles + merges * L + 2 * L * responses
+    return forward, inverse
 
 
 def native_mask_primes(primes, q: int, n: int, t: int) -> int:
