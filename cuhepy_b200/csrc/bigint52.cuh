@@ -71,12 +71,6 @@ __device__ __forceinline__ uint64_t shfl_up64(uint32_t mask, uint64_t v, int del
   const uint32_t hi = __shfl_up_sync(mask, static_cast<uint32_t>(v >> 32), delta, width);
   return (static_cast<uint64_t>(hi) << 32) | lo;
 }
-__device__ __forceinline__ double shfl_f64(uint32_t mask, double v, int src, int width) {
-  const long long b = __double_as_longlong(v);
-  const uint32_t lo = __shfl_sync(mask, static_cast<uint32_t>(b), src, width);
-  const uint32_t hi = __shfl_sync(mask, static_cast<uint32_t>(static_cast<unsigned long long>(b) >> 32), src, width);
-  return __longlong_as_double(static_cast<long long>((static_cast<uint64_t>(hi) << 32) | lo));
-}
 
 template <int K, int TPI>
 struct Group52 {
@@ -236,24 +230,6 @@ struct Group52 {
     for (int k = 0; k < L; ++k) acc[k] = 0;
     cios(acc, a, b, n, ninv);
     finalize(r, acc, n);
-  }
-
-  // r = (init + a * b) * 2^(-52K) mod M, init < 2^(52K) in canonical limbs.
-  __device__ __forceinline__ void mont_mul_acc(double (&r)[L], const double (&init)[L], const double (&a)[L],
-                                               const double* __restrict__ b, const double (&n)[L],
-                                               uint64_t ninv) const {
-    uint64_t acc[L];
-#pragma unroll
-    for (int k = 0; k < L; ++k) acc[k] = to_u64(init[k]);
-    cios(acc, a, b, n, ninv);
-    finalize(r, acc, n);
-  }
-
-  __device__ __forceinline__ void publish(double* buf, const double (&x)[L]) const {
-    __syncwarp(mask);
-#pragma unroll
-    for (int k = 0; k < L; ++k) buf[gl * L + k] = x[k];
-    __syncwarp(mask);
   }
 };
 

@@ -104,7 +104,7 @@ struct cuhe_paillier {
   double* d_crt52 = nullptr;  // per side: the constants mod p, q of k_pair_crt (pair_const_doubles)
   double* d_pair = nullptr;   // the constants mod n of k_pair_modexp
   unsigned long long pair_ninv = 0;  // -n^-1 mod 2^52
-  double* d_n52 = nullptr;    // n^2 and R52 mod n^2 as 52-bit limbs, then R52 R mod n^2 in words
+  double* d_n52 = nullptr;    // n^2 as 52-bit limbs, then R52 R mod n^2 in words
   unsigned long long ninv52 = 0;  // -(n^2)^-1 mod 2^52
   int32_t* d_ops_n52 = nullptr;   // the schedule of n for k_pair_modexp's window
   int nops_n52 = 0;
@@ -348,7 +348,7 @@ cudaError_t launch_outer52(cuhe_paillier* ctx, const uint32_t* query, long long 
   constexpr int TPI = K / 16, K52 = 5 * K / 8, IPB = cuhe::kBlockThreads / TPI;
   const size_t csmem = size_t(K + IPB * K) * 4;
   cuhe::k_to_mont52<K><<<dim3(unsigned((nq + IPB - 1) / IPB)), cuhe::kBlockThreads, csmem, ctx->stream>>>(
-      query, nq, q52, ctx->d_consts, ctx->ks, reinterpret_cast<const uint32_t*>(ctx->d_n52 + 2 * K52),
+      query, nq, q52, ctx->d_consts, ctx->ks, reinterpret_cast<const uint32_t*>(ctx->d_n52 + K52),
       ctx->d_status);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -795,27 +795,23 @@ int upload_side_schedule(cuhe_paillier* ctx, const Limbs& e, int32_t* d_ops, int
   return CUHE_OK;
 }
 
-// The 52-bit constants mod n^2: n^2 and R52 mod n^2 as K52 = 5K/8 limbs of 52 bits
-// (doubles), then R52 R mod n^2 as K words; R52 = 2^(52 K52), R = 2^(32K).
+// The 52-bit constants mod n^2: n^2 as K52 = 5K/8 limbs of 52 bits (doubles),
+// then R52 R mod n^2 as K words; R52 = 2^(52 K52), R = 2^(32K).
 int setup_direct52(cuhe_paillier* ctx) {
   const size_t k = size_t(ctx->K), k52 = 5 * k / 8;
   Limbs one(k, 0u);
   one[0] = 1u;
-  std::vector<double> block(2 * k52 + k / 2, 0.0);
-  auto put52 = [&](size_t row, const Limbs& v) {
-    for (size_t i = 0; i < k52; ++i) {
-      uint64_t limb = 0;
-      for (int b = 0; b < 52; ++b) {
-        const size_t bit = 52 * i + size_t(b);
-        if (bit / 32 < v.size() && ((v[bit / 32] >> (bit % 32)) & 1u)) limb |= 1ull << b;
-      }
-      block[row * k52 + i] = double(limb);
+  std::vector<double> block(k52 + k / 2, 0.0);
+  for (size_t i = 0; i < k52; ++i) {
+    uint64_t limb = 0;
+    for (int b = 0; b < 52; ++b) {
+      const size_t bit = 52 * i + size_t(b);
+      if (bit / 32 < ctx->n2.size() && ((ctx->n2[bit / 32] >> (bit % 32)) & 1u)) limb |= 1ull << b;
     }
-  };
-  put52(0, ctx->n2);
-  put52(1, cuhe::host::shift_mod(one, 52 * k52, ctx->n2));
+    block[i] = double(limb);
+  }
   const Limbs r52r = cuhe::host::shift_mod(one, 52 * k52 + 32 * k, ctx->n2);
-  std::memcpy(block.data() + 2 * k52, r52r.data(), 4 * k);
+  std::memcpy(block.data() + k52, r52r.data(), 4 * k);
   const uint64_t m0 = (uint64_t(ctx->n2[1]) << 32) | ctx->n2[0];
   uint64_t inv = m0;
   for (int it = 0; it < 6; ++it) inv *= 2 - m0 * inv;
