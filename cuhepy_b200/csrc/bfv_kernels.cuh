@@ -1205,8 +1205,9 @@ k_rotate_tm(const RotateOp* __restrict__ ops, const RingDev* __restrict__ ring) 
   const ulonglong2* w2 = R.fwd2[j];
   const int half_n = n >> 1;
   const long long plane = (long long)j * n, comp = (long long)L * n;
-  // a sum starts below 2p and each digit adds less than 2p: up to seven
-  // digits are summed unreduced (below 16p)
+  // a sum starts below 4p (digit 0's product below 2p, base and x0 below p)
+  // and each further digit adds less than 2p: up to seven digits are summed
+  // unreduced (below 16p)
   const bool lazy_sum = R.digits <= 7;
   // digit 0: sigma(x1) itself, with the addends
 #pragma unroll 1

@@ -550,12 +550,12 @@ __device__ __forceinline__ uint32_t word_from_limbs52(const uint64_t* l, int nli
 // the kernel mod n^2 (m = n) for encryption's r^n, public powers and
 // decryption without the factors.  K limbs of 52 bits a component on TPI
 // lanes, 128 threads.  kL = 10 limbs per lane with two CTAs per SM (about 250
-// registers a thread, which let the compiler interleave the accumulations;
-// 168 registers and three CTAs: 1,530 against 2,045 M squarings a second at
-// 2,048-bit m^2) is the best rate; kL = 5 spreads a value over twice the lanes
-// for batches that leave SMs idle: 1,960 M a second when the GPU is full, but
-// 2.7 us a squaring against 4.7 for a warp alone (the host's rule:
-// pair_small).
+// registers a thread, which let the compiler interleave the accumulations; a
+// quarter fewer squarings a second with 168 registers and three CTAs) is the
+// best rate, 2,210 M squarings a second at 2,048-bit m^2; kL = 5 spreads a
+// value over twice the lanes for batches that leave SMs idle: 1,930 M a second
+// when the GPU is full, but 2.6 us a squaring against 4.4 for a warp alone
+// (the host's rule: pair_small).
 //
 // A value of 32-bit words enters as kEntry chunks u_j of 52 K bits,
 // x R = sum_j u_j (R^(j+2) R^-1), one product with a constant pair each, and
@@ -595,10 +595,10 @@ __device__ __forceinline__ void pair_publish(const cuhe52::Pair52<K, TPI>& f, do
 // (kEntry entry rows, (1, 0), the scale row); one = R mod m^2 in global
 // memory; s = this group's K pairs, tab = this thread's table column (stride
 // kPairThreads).  aux: null, or the words a of the factor (1, a).  Leaves the
-// canonical limbs (z0, z1), each in [0, m], as pairs of 64-bit integers in s.
-// kUnits (every thread of the CTA calls it): when z0 is 1 for every value of
-// the CTA, leaves (1, z1 w mod m) instead, w the scale row's factor, and
-// returns true.
+// canonical limbs (z0, z1), in [0, m] (z1 with aux up to m + 2 m^2 / R), as
+// pairs of 64-bit integers in s.  kUnits (every thread of the CTA calls it):
+// when z0 is 1 for every value of the CTA, leaves (1, y) instead, y = z1 w
+// mod m in [0, m + m^2 / R] with w the scale row's factor, and returns true.
 template <int K, int TPI, int kEntry, bool kUnits>
 __device__ __forceinline__ bool pair_power(const cuhe52::Pair52<K, TPI>& f, const uint32_t* __restrict__ words,
                                            int nwords, const double2* rows, const double2* __restrict__ one,
@@ -791,7 +791,7 @@ __device__ __forceinline__ void pair_words(const Group<K, TPI>& g, uint32_t (&x)
   uint32_t z[L];
 #pragma unroll
   for (int j = 0; j < L; ++j) z[j] = word_from_pairs<KL>(s, true, g.gl * L + j);
-  g.mont_mul(x, z, mr, mm, ninv);  // z1 m, at most m^2 - m
+  g.mont_mul(x, z, mr, mm, ninv);  // z1 m mod m^2, a multiple of m
 #pragma unroll
   for (int j = 0; j < L; ++j) z[j] = word_from_pairs<KL>(s, false, g.gl * L + j);
   (void)add_group<K, TPI>(g, x, z);  // at most m^2
@@ -919,7 +919,7 @@ k_pair_crt(const uint32_t* __restrict__ base, uint32_t* __restrict__ out, long l
       sub_mod<KH, LT>(h, u, x, m);
       h.load_ro(m, consts + C_N * K);
       h.mont_mul(x, u, s_qr, m, ks.ninv1);  // q times that, at most n - q
-      (void)add_group<KH, LT>(h, x, y);     // r_q is at most q
+      (void)add_group<KH, LT>(h, x, y);     // r_q is at most q + q^2 / R: the sum is below 2 n
       if (!h.less_than(x, m)) sub_group<KH, LT>(h, x, m);
       if (mode == EXP_DECRYPT) {
         h.store(out + inst * K, x);

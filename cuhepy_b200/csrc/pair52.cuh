@@ -10,8 +10,10 @@
 // limb products and a squaring (x0 y1 + x1 y0 = x0 (2 x1)) four, where the
 // Montgomery product of 2K-limb values mod m^2 costs eight: the quotient of
 // the first reduction is what the second component needs, and nothing wider
-// than m is ever multiplied.  R is at least 2^8 m and both
-// components stay below 2 m, so no product ends with a subtraction.
+// than m is ever multiplied.  R is at least 2^8 m.  Operands with components
+// below 8 m (sums of up to four entry products, each below 2 m) give
+// z0 < m + 64 m^2 / R and z1 < m + 128 m^2 / R, below 2 m again, so no product
+// ends with a subtraction.
 //
 // Limbs are 52 bits and balanced (in [-2^51, 2^51] up to a carry of 2^10),
 // held exactly as doubles.  The
@@ -32,9 +34,10 @@
 // and integer adds.  A limb product with its accumulation takes 10.2-11.4
 // cycles per warp in isolation in every form tried (high halves chained
 // through the FMA addend, low halves by integer multiplies, 46- and 49-bit
-// limbs with FP64 accumulators) and 10.9 in the whole squaring, so the gain
-// over the 2K-limb product is the number of limb products: 2,045 M squarings
-// mod a 2,048-bit m^2 a second against 980 M.
+// limbs with FP64 accumulators) and 10.5 in a loop of whole squarings, so the
+// gain over the 2K-limb product is the number of limb products: 2,210 M
+// squarings mod a 2,048-bit m^2 a second, ten limbs a lane and two CTAs on
+// every SM, against 980 M.
 #pragma once
 #include <cstdint>
 
@@ -52,8 +55,8 @@ constexpr int kPairThreads = 128;
 // K limbs per component over TPI consecutive lanes, lane g owning limbs
 // [gL, gL + L).  Every lane of a warp takes part in every call (shuffles use
 // the full mask), so groups of a warp follow one schedule.  U: steps per
-// unrolled block; 2 keeps the product small in the instruction cache (U = 10:
-// 1,892 M squarings a second, 2 and 5: 2,045 M).
+// unrolled block; 2 keeps the product small in the instruction cache (2 and 5
+// are 8% faster than 10).
 template <int K, int TPI, int U = 2>
 struct Pair52 {
   static_assert(K % TPI == 0 && K % U == 0, "limbs divide over lanes and blocks");
@@ -167,8 +170,8 @@ struct Pair52 {
   // component.  Column 0 of both is formed first, from limb products made
   // during the step before, so both quotients travel while the other columns'
   // products run; and squarings and products are separate loops, with no
-  // branch inside a step (one loop with the quotients in turn: 1,805 against
-  // 2,168 M squarings a second, one warp alone 7.5 against 4.7 us).
+  // branch inside a step (one loop with the quotients in turn runs 17% fewer
+  // squarings a second, and one warp alone takes 1.6 times as long).
   template <bool kBoth>
   __device__ __forceinline__ void steps(uint64_t (&A0)[L], uint64_t (&A1)[L], const double (&a0)[L],
                                         const double (&a1)[L], const double2* b, const double (&m)[L],
