@@ -31,10 +31,6 @@ LIBRARIES = {
         "depends": ["bigint52.cuh", "bigint_group.cuh", "host_bigint.h", "pair52.cuh", "pair52_split.cuh",
                     "paillier_kernels.cuh", "split_kernels.cuh"],
         "headers": ["cuhe_paillier.h"],
-        # One optimiser thread per core, for its many kernel variants.  Not for
-        # the BFV library, whose searches run 1.3-2% slower when its kernels are
-        # optimised in parts.
-        "flags": ["--split-compile=0"],
     },
     "libcuhe_bfv_b200.so": {
         "sources": ["cuhe_bfv.cu"],
@@ -66,7 +62,7 @@ def build_library(name: str, force: bool = False, verbose: bool = False) -> Path
     if not force and not _stale(out, inputs):
         return out
     tmp = out.with_suffix(".so.tmp")
-    cmd = [nvcc(), *NVCC_FLAGS, *spec.get("flags", []), "-I", str(INCLUDE), "-o", str(tmp),
+    cmd = [nvcc(), *NVCC_FLAGS, "-I", str(INCLUDE), "-o", str(tmp),
            *[str(CSRC / s) for s in spec["sources"]]]
     if verbose:
         cmd.insert(1, "-Xptxas=-v")
