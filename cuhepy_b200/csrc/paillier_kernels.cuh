@@ -609,7 +609,6 @@ __device__ __forceinline__ bool pair_power(const cuhe52::Pair52<K, TPI>& f, cons
   const int32_t* ops = ex.ops;
   int nops = ex.nops;
   bool halved = kUnits && ex.halved != 0;
-  asm volatile("" : "+l"(ninv));  // held, not selected again in every step
   double z0[L], z1[L], a0[L], a1[L];
   uint64_t A0[L], A1[L];
   const int at = f.gl * L;

@@ -55,8 +55,9 @@ constexpr int kPairThreads = 128;
 // K limbs per component over TPI consecutive lanes, lane g owning limbs
 // [gL, gL + L).  Every lane of a warp takes part in every call (shuffles use
 // the full mask), so groups of a warp follow one schedule.  U: steps per
-// unrolled block; 2 keeps the product small in the instruction cache (2 and 5
-// are 8% faster than 10).
+// unrolled block; 2 keeps the product small in the instruction cache (65,536
+// decodes at key_len 1024 with U = 1, 2, 4, 5, 10: 26.8, 25.7, 28.4, 28.4 and
+// 31.2 ms).
 template <int K, int TPI, int U = 2>
 struct Pair52 {
   static_assert(K % TPI == 0 && K % U == 0, "limbs divide over lanes and blocks");
@@ -71,7 +72,6 @@ struct Pair52 {
   __device__ __forceinline__ Pair52() {
     gl = int(threadIdx.x & 31) & (TPI - 1);
     csh = gl == 0 ? 20u : 32u;
-    asm volatile("" : "+r"(csh));  // held: selecting it again in every step costs 2.7%
   }
 
   __device__ __forceinline__ static void mul52(double x, double y, uint64_t& hi, uint64_t& lo) {

@@ -21,7 +21,7 @@
 // the five-limb kernels, one limb of both components, takes 256 for the same
 // 20 limb products per lane, so a value of 20 limbs needs 11 x 345 cycles a
 // squaring against 20 x 256: one decode at key_len 1024 0.83 against 1.19 ms,
-// 0.79 with the wider windows that its table has room for.
+// 0.80 with the wider windows that its table has room for.
 #pragma once
 #include "pair52.cuh"
 
@@ -51,7 +51,6 @@ struct Split52 {
     const u128 inv = u128(0) - ninv, twice = u128(0) - inv * (2 - low * inv);
     n0 = f.gl == 0 ? ninv : 0ull;
     n1 = f.gl == 0 ? static_cast<uint64_t>(twice >> 52) & kMask : 0ull;
-    asm volatile("" : "+l"(n0), "+l"(n1));  // held, not selected again in every step
   }
 
   // Limbs 2i, 2i + 1 for half 0 and 2i - 2, 2i - 1 for half 1 of an operand
