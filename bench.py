@@ -740,10 +740,10 @@ def ctypes_imad_peak(native, device: int) -> float:
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one k_pair_crt<64,10>
-# decode launch of 8,192 ciphertexts (ncu, key_len 1024): 4,556,032 + 0
+# decode launch of 8,192 ciphertexts (ncu, key_len 1024): 4,396,288 + 0
 # bytes.  Each ciphertext is read once, so the traffic of a larger launch
 # scales with the number of decodes.
-DECODE_TRAFFIC_BYTES, DECODE_TRAFFIC_ITEMS = 4_556_032, 8192
+DECODE_TRAFFIC_BYTES, DECODE_TRAFFIC_ITEMS = 4_396_288, 8192
 
 
 def window_products(e: int, width: int) -> tuple[int, int]:
