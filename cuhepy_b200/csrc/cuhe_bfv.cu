@@ -560,6 +560,12 @@ size_t unfused_bytes_per_op(const cuhe_bfv_ring* r) {
 // when the caller lends scratch.
 constexpr size_t kSmallSwitchPairs = 148;
 
+// Whether a wave of so many pairs may: one CTA row of its first kernel per pair
+// and digit, and a launch has at most 65,535 rows (148 pairs: 442 digits).
+bool small_wave(const cuhe_bfv_ring* r, size_t pairs) {
+  return pairs <= kSmallSwitchPairs && pairs * r->plan.digits <= 65535;
+}
+
 // Scratch bytes of the largest such wave.
 size_t small_switch_bytes(const cuhe_bfv_ring* r) {
   const size_t L = r->residue ? r->plan.residue_count : r->switch_prime_count;
@@ -603,7 +609,7 @@ int run_switch(cuhe_bfv_ring* r, Lane& ln, RingDev* d, const std::vector<Compose
     dim3 grid(unsigned(sops.size()), unsigned(r->residue ? P.residue_count : r->switch_prime_count));
     const size_t pairs = size_t(grid.x) * grid.y;
     const size_t small_need = slice(sops.size() * unfused_bytes_per_op(r));
-    if (small && P.n <= kMaxPlaneN && pairs <= kSmallSwitchPairs && small->used + small_need <= small->cap) {
+    if (small && P.n <= kMaxPlaneN && small_wave(r, pairs) && small->used + small_need <= small->cap) {
       // few ops: six times as many CTAs per op in the digit transforms
       u64* scratch = reinterpret_cast<u64*>(small->base + small->used);
       if (int rc = switch_unfused(r, ln, d, d_sops, sops.size(), scratch, sops.size())) return rc;
@@ -738,7 +744,7 @@ int run_chain(cuhe_bfv_ring* r, Lane& ln, RingDev* d, const RotateChain& chain, 
     if (!st.composed)
       if (int rc = launch_compose(r, ln, d, d_cops + st.first, st.count)) return rc;
     const RotateOp* rop = d_rops + st.first;
-    if (st.count * L <= kSmallSwitchPairs && st.count * rotate_unfused_bytes(r) <= room) {
+    if (small_wave(r, st.count * L) && st.count * rotate_unfused_bytes(r) <= room) {
       const unsigned bx = blocks_for((long long)n, 256), planes = unsigned(st.count * L * (P.digits - 1));
       k_rotate_digits<<<dim3(bx, unsigned(st.count * L * P.digits)), 256, 0, ln.stream>>>(rop, int(st.count), int(L),
                                                                                           digits, d);
